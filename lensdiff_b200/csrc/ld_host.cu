@@ -1387,8 +1387,13 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
         staged(c, LD_STAGE_PSF_ROWS, s, [&] { launch_psf_rows(a, s); });
         staged(c, LD_STAGE_PSF_COLS, s, [&] { launch_psf_cols(a, s); });
     }
-    const bool pairs = std::all_of(infos.begin(), infos.end(), [](const WavelengthInfo& w) { return w.taps == 0; });
-    staged(c, LD_STAGE_RESAMPLE, s, [&] { launch_resample(a, pairs, s); });
+    bool filtered = false;
+    float inv_max = 0.0f;
+    for (const WavelengthInfo& w : infos) {
+        if (w.taps != 0) filtered = true;
+        else inv_max = std::max(inv_max, w.inv_scale);
+    }
+    staged(c, LD_STAGE_RESAMPLE, s, [&] { launch_resample(a, filtered, inv_max, s); });
     const bool fused = fused_shaping(a);
     if (!fused) staged(c, LD_STAGE_SHAPE_STATS, s, [&] { launch_shape_stats(a, s); });
     staged(c, LD_STAGE_SUPPORT, s, [&] { launch_support(a, s); });

@@ -17,6 +17,7 @@
 // overwritten stage by stage: resampled value -> shaped value (shape_stats) ->
 // shaped * taper inside the crop box, 0 outside (crop_sum); the final,
 // normalised kernel is that value / (s3 * s4).
+#include <algorithm>
 #include <climits>
 
 #include "ld_internal.h"
@@ -55,35 +56,44 @@ __device__ double block_sum(double v) {
     return r;
 }
 
-// Adds each lane's v to ring[slot] (and, with PEAK, maxes it into
-// peak[slot] as float bits) where the lanes' slots form runs of equal values
-// in consecutive lanes (slot < 0: nothing to add), v >= 0.  A warp is 32
-// pixels of a canvas row, along which the ring index is monotonic on each
-// side of the centre, so equal slots are contiguous.  One inclusive
-// segmented scan over the warp (five shuffles) gives each run's sum (and
-// maximum) in its last lane, which adds it with one shared-memory atomic:
-// a fixed cost per warp whatever the number of runs.
+// Inclusive segmented scan over the runs of equal slots in consecutive lanes:
+// leaves each run's sum (and maximum) in v (and m) of its last lane, for
+// which it returns true.  `far`: lanes whose `o` lanes before them belong to
+// their run, i.e. the step of distance o has work; off the canvas's axes a
+// run is one to three pixels long, so most rows need one or two steps.
 template <bool PEAK>
-__device__ __forceinline__ void warp_runs_accumulate(int slot, float v, float* ring, unsigned int* peak) {
+__device__ __forceinline__ bool warp_runs_scan(int slot, float& v, float& m) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int prev = __shfl_up_sync(full, slot, 1);
     const unsigned heads = __ballot_sync(full, lane == 0 || prev != slot);
-    const int head = 31 - __clz(heads & (full >> (31 - lane)));  // first lane of this lane's run
-    float sum = v, m = v;
+    unsigned far = ~heads;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(full, sum, o);
+        if (far == 0u) break;  // uniform
+        const float t = __shfl_up_sync(full, v, o);
         const float u = PEAK ? __shfl_up_sync(full, m, o) : 0.0f;
-        if (lane - o >= head) {
-            sum += t;
+        if ((far >> lane) & 1u) {
+            v += t;
             if (PEAK) m = fmaxf(m, u);
         }
+        far &= far << o;
     }
-    const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u) != 0u;
-    if (tail && slot >= 0) {
-        if (sum != 0.0f) atomicAdd(&ring[slot], sum);
-        if (PEAK && m != 0.0f) atomicMax(&peak[slot], __float_as_uint(m));
+    return lane == 31 || ((heads >> (lane + 1)) & 1u) != 0u;
+}
+
+// Adds each lane's v to ring[slot] (and, with PEAK, maxes its top into
+// peak[slot] as float bits) where the lanes' slots form runs of equal values
+// in consecutive lanes (slot < 0: nothing to add), v >= 0.  A warp is 32
+// pixels of a canvas row, along which the ring index is monotonic on each
+// side of the centre, so equal slots are contiguous.  One inclusive
+// segmented scan over the warp (warp_runs_scan) gives each run's sum (and
+// maximum) in its last lane, which adds it with one shared-memory atomic.
+template <bool PEAK>
+__device__ __forceinline__ void warp_runs_accumulate(int slot, float v, float top, float* ring, unsigned int* peak) {
+    if (warp_runs_scan<PEAK>(slot, v, top) && slot >= 0) {
+        if (v != 0.0f) atomicAdd(&ring[slot], v);
+        if (PEAK && top != 0.0f) atomicMax(&peak[slot], __float_as_uint(top));
     }
 }
 
@@ -187,59 +197,21 @@ struct Window {
     int stride, x0, n, S;
 };
 
-// sampleSquareBilinear (LensDiffCpuReference.cpp:316-336) reading the |F|^2
-// window; the window covers every pixel the kernel touches.
-__device__ __forceinline__ float sample_bilinear(const Window& w, float x, float y) {
-    const float lim = static_cast<float>(w.S - 1);
-    if (x < 0.0f || y < 0.0f || x > lim || y > lim) return 0.0f;
-    const int x0 = static_cast<int>(floorf(x));
-    const int y0 = static_cast<int>(floorf(y));
-    const int x1 = min(x0 + 1, w.S - 1);
-    const int y1 = min(y0 + 1, w.S - 1);
-    const float tx = x - static_cast<float>(x0);
-    const float ty = y - static_cast<float>(y0);
-    const int hi = w.n - 1;
-    const int ax0 = min(max(x0 - w.x0, 0), hi), ax1 = min(max(x1 - w.x0, 0), hi);
-    const int ay0 = min(max(y0 - w.x0, 0), hi), ay1 = min(max(y1 - w.x0, 0), hi);
-    const float v00 = w.p[static_cast<size_t>(ay0) * w.stride + ax0];
-    const float v10 = w.p[static_cast<size_t>(ay0) * w.stride + ax1];
-    const float v01 = w.p[static_cast<size_t>(ay1) * w.stride + ax0];
-    const float v11 = w.p[static_cast<size_t>(ay1) * w.stride + ax1];
-    const float vx0 = v00 + (v10 - v00) * tx;
-    const float vx1 = v01 + (v11 - v01) * tx;
-    return vx0 + (vx1 - vx0) * ty;
-}
-
-// sampleSquareFiltered (LensDiffCpuReference.cpp:338-353)
-__device__ __forceinline__ float sample_filtered(const Window& w, float x, float y, float footprint, int taps,
-                                                 float step) {
-    if (taps == 0) return sample_bilinear(w, x, y);
-    float sum = 0.0f;
-    for (int ty = 0; ty < taps; ++ty) {
-        const float oy = (static_cast<float>(ty) + 0.5f) * step - footprint * 0.5f;
-        for (int tx = 0; tx < taps; ++tx) {
-            const float ox = (static_cast<float>(tx) + 0.5f) * step - footprint * 0.5f;
-            sum += sample_bilinear(w, x + ox, y + oy);
-        }
-    }
-    return sum / static_cast<float>(taps * taps);
-}
-
-// First ring index a 32 x TH tile can touch, for a centre at (c, c) and ring
+// First ring index a 32 x th tile can touch, for a centre at (c, c) and ring
 // indices clamped to `cap`: every pixel of the tile has a ring index in
 // [base, base + span) with span <= the tile's diagonal + 3 (kRingSpan for
 // 32 x 32 tiles, kRingSpanTall for the 32 x 128 tiles of the ring-statistics
 // passes).
-template <int TH = kTile>
-__device__ __forceinline__ int tile_ring_base(int tx0, int ty0, int c, int cap) {
+__device__ __forceinline__ int tile_ring_base(int tx0, int ty0, int c, int cap, int th = kTile) {
     const int dx = tx0 > c ? tx0 - c : (tx0 + kTile - 1 < c ? c - (tx0 + kTile - 1) : 0);
-    const int dy = ty0 > c ? ty0 - c : (ty0 + TH - 1 < c ? c - (ty0 + TH - 1) : 0);
+    const int dy = ty0 > c ? ty0 - c : (ty0 + th - 1 < c ? c - (ty0 + th - 1) : 0);
     const float r = sqrtf(static_cast<float>(dx * dx + dy * dy));
     return min(cap, max(0, static_cast<int>(r) - 1));
 }
 
 // The column half of a bilinear sample of the |F|^2 window at x
-// (sampleSquareBilinear's x terms): the same for every row a thread samples.
+// (sampleSquareBilinear, LensDiffCpuReference.cpp:316-336; the window covers
+// every pixel the kernel touches): the same for every row a thread samples.
 struct ColTap {
     bool in;       // x inside [0, S - 1]
     int ax0, ax1;  // window columns of x0 and x1
@@ -256,57 +228,25 @@ __device__ __forceinline__ ColTap col_tap(const Window& w, float x) {
     c.ax1 = min(max(x1 - w.x0, 0), hi);
     return c;
 }
-// sample_bilinear with the column half precomputed (identical arithmetic).
-__device__ __forceinline__ float sample_row(const Window& w, const ColTap& c, float y) {
-    if (!c.in || y < 0.0f || y > static_cast<float>(w.S - 1)) return 0.0f;
-    const int y0 = static_cast<int>(floorf(y));
-    const int y1 = min(y0 + 1, w.S - 1);
-    const float ty = y - static_cast<float>(y0);
-    const int hi = w.n - 1;
-    const float* r0 = w.p + min(max(y0 - w.x0, 0), hi) * w.stride;
-    const float* r1 = w.p + min(max(y1 - w.x0, 0), hi) * w.stride;
-    const float v00 = __ldg(r0 + c.ax0), v10 = __ldg(r0 + c.ax1);
-    const float v01 = __ldg(r1 + c.ax0), v11 = __ldg(r1 + c.ax1);
-    const float vx0 = v00 + (v10 - v00) * c.tx;
-    const float vx1 = v01 + (v11 - v01) * c.tx;
-    return vx0 + (vx1 - vx0) * ty;
-}
-
-// grid (ceil(K/32), ceil(K/128), B), block (32, 8).
 // FUSED (anisotropy gain 1): reshapeAnisotropy (LensDiffCpuReference.cpp:1122-1134)
 // then gives mean + (base - mean) * 1, the base kernel itself up to one
-// rounding, so the canvas keeps the resampled values unnormalised and this
-// pass takes the shaped kernel's statistics that shape_stats_kernel takes
+// rounding, so the canvas keeps the resampled values unnormalised and the
+// rescale takes the shaped kernel's statistics that shape_stats_kernel takes
 // otherwise (s3 = s1, the ceil(r) ring energies and peaks, the peak) in
 // place of the round(r) ring sums, which only the Split look's ring means
 // need (ring_sums_kernel, run when a Split render first uses the bank).
-// The bilinear path (no box filter: the canvas samples the |F|^2 window at
-// most one window pixel apart, scaleFactor >= 1) stages the window pixels a
-// 32 x 128 tile reads in shared memory first: at most 33 x 129 of them, with
-// one more on each side so that the span holds whatever the rounding of the
-// sample positions.
-constexpr int kStageW = kTile + 4, kStageH = kTallH + 4;
 
-// Rows / columns of the window that canvas coordinates c0 .. c1 sample
-// (sample_bilinear's x0 .. x1 of the first and last sample, clamped to the
-// window as it clamps them): [lo, hi] in window indices.
-__device__ __forceinline__ void stage_span(const Window& w, float rc, float kc, float inv, int c0, int c1, int* lo,
-                                           int* hi) {
-    const float p0 = rc + (static_cast<float>(c0) - kc) * inv;
-    const float p1 = rc + (static_cast<float>(c1) - kc) * inv;
-    const int whi = w.n - 1;
-    const int a0 = static_cast<int>(floorf(fmaxf(p0, 0.0f)));
-    const int a1 = min(static_cast<int>(floorf(fminf(fmaxf(p1, 0.0f), static_cast<float>(w.S - 1)))) + 1, w.S - 1);
-    *lo = min(max(a0 - 1 - w.x0, 0), whi);
-    *hi = min(max(a1 + 1 - w.x0, 0), whi);
-}
-
-// Shared memory of one λ-rescale tile.
+// Ring statistics of one λ-rescale tile, and its staged window pixels.
 template <bool FUSED>
-struct ResampleSmem {
+struct RingSmem {
     float ring[kRingSpanTall];  // FUSED: the ceil(r) ring energies, else the round(r) sums
     unsigned int ring_p[FUSED ? kRingSpanTall : 1];
-    float stage[kStageH][kStageW];
+    __device__ void clear(int tid) {
+        for (int i = tid; i < kRingSpanTall; i += 256) {
+            ring[i] = 0.0f;
+            if constexpr (FUSED) ring_p[i] = 0u;
+        }
+    }
 };
 
 // Ring slot of canvas pixel (x, y) relative to the tile's first ring `rbase`
@@ -318,54 +258,24 @@ __device__ __forceinline__ int ring_slot(bool in, float dx, float dy, int R, int
     return min(R, static_cast<int>(FUSED ? ceilf(rr) : roundf(rr))) - rbase;
 }
 
-// The window pixels (rows cy0.., columns cx0..) a staged tile samples.
-struct StageBox {
-    int cx0, cy0, sw, sh;
-};
-
-// The staged box of wavelength `w`'s window for the tile at (tx0, ty0);
-// ok = false when the samples are box-filtered or the span is too wide.
-__device__ __forceinline__ bool stage_box(const Window& w, float rc, float kc, float inv, int taps, int tx0, int ty0,
-                                          int K, StageBox* b) {
-    if (taps != 0) return false;
-    int cx1 = -1, cy1 = -1;
-    stage_span(w, rc, kc, inv, tx0, min(tx0 + kTile, K) - 1, &b->cx0, &cx1);
-    stage_span(w, rc, kc, inv, ty0, min(ty0 + kTallH, K) - 1, &b->cy0, &cy1);
-    b->sw = cx1 - b->cx0 + 1;
-    b->sh = cy1 - b->cy0 + 1;
-    return b->sw <= kStageW && b->sh <= kStageH;
-}
-
-__device__ __forceinline__ void stage_load(const Window& w, const StageBox& b, float (*stage)[kStageW], int tid) {
-    for (int i = tid; i < b.sw * b.sh; i += 256) {
-        const int r = i / b.sw, c = i - r * b.sw;
-        stage[r][c] = __ldg(w.p + static_cast<size_t>(b.cy0 + r) * w.stride + b.cx0 + c);
+// The peak and the sum of a tile's pixels go to the wavelength's statistics.
+template <bool FUSED>
+__device__ __forceinline__ void resample_totals(const PsfBankArgs& a, int b, float lsum, unsigned int lpeak, int tid) {
+    if constexpr (FUSED) {
+        for (int o = 16; o > 0; o >>= 1) lpeak = max(lpeak, __shfl_xor_sync(0xffffffffu, lpeak, o));
+        if ((tid & 31) == 0 && lpeak != 0u) atomicMax(&a.scalars[b].peak, lpeak);
     }
-}
-
-// sample_row's arithmetic on staged pixels: the bilinear sample at window
-// row coordinate yy of the column tap ct (sx0, sx1: its columns in the box).
-__device__ __forceinline__ float staged_sample(const Window& w, const ColTap& ct, int sx0, int sx1, int cy0,
-                                              const float (*stage)[kStageW], bool in, float yy) {
-    const float lim = static_cast<float>(w.S - 1);
-    if (!(in && ct.in && !(yy < 0.0f || yy > lim))) return 0.0f;
-    const int hi = w.n - 1;
-    const int y0 = static_cast<int>(floorf(yy));
-    const int y1 = min(y0 + 1, w.S - 1);
-    const float ty = yy - static_cast<float>(y0);
-    const int sy0 = min(max(y0 - w.x0, 0), hi) - cy0;
-    const int sy1 = min(max(y1 - w.x0, 0), hi) - cy0;
-    const float v00 = stage[sy0][sx0], v10 = stage[sy0][sx1];
-    const float v01 = stage[sy1][sx0], v11 = stage[sy1][sx1];
-    const float vx0 = v00 + (v10 - v00) * ct.tx;
-    const float vx1 = v01 + (v11 - v01) * ct.tx;
-    return vx0 + (vx1 - vx0) * ty;
+    const double tot = block_sum(static_cast<double>(lsum));
+    if (tid == 0) {
+        atomicAdd(&a.scalars[b].s1, tot);
+        if constexpr (FUSED) atomicAdd(&a.scalars[b].s3, tot);
+    }
 }
 
 // The end of one wavelength's tile: the CTA's ring sums and peaks, the peak
 // and the canvas sum go to the wavelength's global statistics.
 template <bool FUSED>
-__device__ __forceinline__ void resample_flush(const PsfBankArgs& a, int b, int rbase, ResampleSmem<FUSED>& sm,
+__device__ __forceinline__ void resample_flush(const PsfBankArgs& a, int b, int rbase, RingSmem<FUSED>& sm,
                                                float lsum, unsigned int lpeak, int tid) {
     __syncthreads();
     const int R = a.R;
@@ -378,39 +288,251 @@ __device__ __forceinline__ void resample_flush(const PsfBankArgs& a, int b, int 
             if (sm.ring_p[i] != 0u) atomicMax(&a.ring_peak[ro + rbase + i], sm.ring_p[i]);
         }
     }
-    if constexpr (FUSED) {
-        for (int o = 16; o > 0; o >>= 1) lpeak = max(lpeak, __shfl_xor_sync(0xffffffffu, lpeak, o));
-        if ((tid & 31) == 0 && lpeak != 0u) atomicMax(&a.scalars[b].peak, lpeak);
-    }
-    const double tot = block_sum(static_cast<double>(lsum));
-    if (tid == 0) {
-        atomicAdd(&a.scalars[b].s1, tot);
-        if constexpr (FUSED) atomicAdd(&a.scalars[b].s3, tot);
-    }
+    resample_totals<FUSED>(a, b, lsum, lpeak, tid);
 }
 
-// One wavelength's 32 x 128 canvas tile (grid (ceil(K/32), ceil(K/128), .),
-// block (32, 8); 16 rows per thread).
-// FUSED (anisotropy gain 1): reshapeAnisotropy (LensDiffCpuReference.cpp:1122-1134)
-// then gives mean + (base - mean) * 1, the base kernel itself up to one
-// rounding, so the canvas keeps the resampled values unnormalised and this
-// pass takes the shaped kernel's statistics that shape_stats_kernel takes
-// otherwise (s3 = s1, the ceil(r) ring energies and peaks, the peak) in
-// place of the round(r) ring sums, which only the Split look's ring means
-// need (ring_sums_kernel, run when a Split render first uses the bank).
-// The bilinear path (no box filter: the canvas samples the |F|^2 window at
-// most one window pixel apart, scaleFactor >= 1) stages the window pixels the
-// tile reads in shared memory first (stage_box); box-filtered samples, and
-// any span too wide to stage, read the window directly.
+// ---- lambda-rescale without a box filter ----------------------------------------
+// The canvas samples the |F|^2 window at most one window pixel apart
+// (scaleFactor >= 1).  A CTA takes a 32 x th tile of the canvas's quadrant
+// dx, dy >= 0 together with its three mirror images: the four pixels
+// (+-dx, +-dy) lie on one ring, so the ring slot and the segmented scan of the
+// ring statistics run once for the four.  The window pixels under the four
+// images are staged in shared memory.  A warp walks th / 8 consecutive canvas
+// rows; the rows' sample positions are uniform in the warp, so the two
+// horizontally interpolated window rows a sample blends are kept in registers
+// until the position moves to the next window row (every 1 / inv_scale
+// canvas rows).  Bound by instruction issue (84 M warp instructions, 76 % of
+// the issue slots): 112 us for 31 wavelengths at K = 1025 (168 us for tiles
+// without the mirror images, two wavelengths at a time, every sample from
+// four shared-memory reads).
+constexpr int kQuadH = 128;
+
+// Window indices [lo, hi] that canvas offsets d0 .. d1 (d0 <= d1) from the
+// centre sample, one more on each side so that the span holds whatever the
+// rounding of the sample positions.
+__device__ __forceinline__ void quad_span(const Window& w, float rc, float inv, float d0, float d1, int* lo, int* hi) {
+    const float p0 = rc + d0 * inv, p1 = rc + d1 * inv;
+    const int whi = w.n - 1;
+    const int a0 = static_cast<int>(floorf(fmaxf(p0, 0.0f)));
+    const int a1 = min(static_cast<int>(floorf(fminf(fmaxf(p1, 0.0f), static_cast<float>(w.S - 1)))) + 1, w.S - 1);
+    *lo = min(max(a0 - 1 - w.x0, 0), whi);
+    *hi = min(max(a1 + 1 - w.x0, 0), whi);
+}
+
+// Staged pixels per box side for `n` canvas pixels sampled `inv` apart
+// (quad_span's count, with one for rounding).
+__host__ __device__ constexpr int quad_stage(int n, float inv) { return static_cast<int>((n - 1) * inv) + 7; }
+
+// Tile (tx, ty) of wavelength b; block (32, 8).  Shared memory: the warps' ring
+// statistics, then the staged boxes [row image][column image][sh][sw].
+// Along a quadrant's row the ring index only grows, so a row's runs have
+// distinct slots: each warp adds them to ring statistics of its own with
+// plain loads and stores.
+constexpr int kRingSpanQuad = 136;  // >= sqrt(31^2 + 127^2) + 3
+constexpr size_t kQuadRingBytes = 8 * kRingSpanQuad * sizeof(float2);
+
 template <bool FUSED>
-__device__ void resample_tile(const PsfBankArgs& a, int b, int rbase, ResampleSmem<FUSED>& sm, int tid) {
-    for (int i = tid; i < kRingSpanTall; i += 256) {
-        sm.ring[i] = 0.0f;
-        if constexpr (FUSED) sm.ring_p[i] = 0u;
-    }
+__device__ __forceinline__ void resample_quad(const PsfBankArgs& a, int tx, int ty, int b, int th, int sw, int sh,
+                                              float2* smem) {
+    float2(*ring)[kRingSpanQuad] = reinterpret_cast<float2(*)[kRingSpanQuad]>(smem);  // per warp: sums and peaks
+    float* stage = reinterpret_cast<float*>(smem + 8 * kRingSpanQuad);
     const WavelengthInfo* wi = a.wl + b;
+    const int lane = threadIdx.x;
+    const int tid = lane + threadIdx.y * 32;
     const int K = a.K, R = a.R;
-    const int tx0 = blockIdx.x * kTile, ty0 = blockIdx.y * kTallH;
+    const int tx0 = tx * kTile, ty0 = ty * th;  // offsets from the centre
+    const int rbase = tile_ring_base(tx0, ty0, 0, R, th);
+    float2* wring = ring[threadIdx.y];
+    for (int i = lane; i < kRingSpanQuad; i += 32) wring[i] = make_float2(0.0f, 0.0f);
+    const Window w{a.win + static_cast<size_t>(b) * a.win_stride * a.win_stride, a.win_stride, wi->win_x0,
+                   wi->win_n, a.S};
+    const float inv = wi->inv_scale;
+    const float rc = a.raw_center;
+    // [0]: the images at +dx / +dy, [1]: at -dx / -dy
+    int cx[2], cy[2], hx[2], hy[2];
+    const float fx0 = static_cast<float>(tx0), fx1 = static_cast<float>(min(tx0 + kTile - 1, R));
+    const float fy0 = static_cast<float>(ty0), fy1 = static_cast<float>(min(ty0 + th - 1, R));
+    quad_span(w, rc, inv, fx0, fx1, &cx[0], &hx[0]);
+    quad_span(w, rc, inv, -fx1, -fx0, &cx[1], &hx[1]);
+    quad_span(w, rc, inv, fy0, fy1, &cy[0], &hy[0]);
+    quad_span(w, rc, inv, -fy1, -fy0, &cy[1], &hy[1]);
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        const int bh = min(hy[v] - cy[v] + 1, sh);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int bw = min(hx[h] - cx[h] + 1, sw);
+            float* st = stage + (v * 2 + h) * sh * sw;
+            const float* src = w.p + static_cast<size_t>(cy[v]) * w.stride + cx[h];
+            for (int r = threadIdx.y; r < bh; r += 8)
+                for (int c = lane; c < bw; c += 32) st[r * sw + c] = __ldg(src + r * w.stride + c);
+        }
+    }
+    __syncthreads();
+    const int ix = tx0 + lane;
+    const bool in = ix <= R;
+    const bool mirror = in && ix > 0;  // column 0 has no mirror image
+    const float dx = static_cast<float>(ix);
+    const ColTap ct[2] = {col_tap(w, rc + dx * inv), col_tap(w, rc - dx * inv)};
+    int s0[2], s1[2];  // the taps' columns in the staged boxes
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        s0[h] = min(max(ct[h].ax0 - cx[h], 0), sw - 1) + h * sh * sw;
+        s1[h] = min(max(ct[h].ax1 - cx[h], 0), sw - 1) + h * sh * sw;
+    }
+    const bool use[2] = {in && ct[0].in, mirror && ct[1].in};
+    // the two window rows under a canvas row, interpolated at the thread's two
+    // columns (h0, h1 [row image][column image]), and the window row (as a
+    // float) they belong to
+    float h0[2][2] = {}, h1[2][2] = {}, at[2] = {-1.0f, -1.0f};
+    const float lim = static_cast<float>(w.S - 1);
+    const int rows = th / 8;
+    const int iy0 = ty0 + threadIdx.y * rows;
+    float* const canvas = a.canvas + static_cast<size_t>(b) * K * K + static_cast<size_t>(R) * K + R;
+    float* up = canvas + static_cast<ptrdiff_t>(iy0) * K;   // row +dy, at the centre column
+    float* down = canvas - static_cast<ptrdiff_t>(iy0) * K; // row -dy
+    // ceil(sqrtf(n)) of integers n < 2^24 is exact, so the slot follows n by
+    // comparison with the squares; else (and for round(r)) by the square root
+    const bool exact = FUSED && R < 2048;
+    int n = ix * ix + iy0 * iy0;
+    int ring_i = exact ? static_cast<int>(ceilf(sqrtf(static_cast<float>(n)))) : 0;
+    float lsum = 0.0f;  // this thread's pixels; one double add per thread at the flush
+    float lpeak = 0.0f;
+    for (int i = 0; i < rows; ++i) {
+        const int iy = iy0 + i;
+        if (iy > R) break;  // uniform: a warp walks canvas rows
+        const float dy = static_cast<float>(iy);
+        float sum = 0.0f, m = 0.0f;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            if (v == 1 && iy == 0) break;  // row 0 has no mirror image
+            const float yy = v == 0 ? rc + dy * inv : rc - dy * inv;
+            const bool ok = !(yy < 0.0f || yy > lim);
+            const float fl = floorf(yy);
+            const float f = yy - fl;
+            if (ok && fl != at[v]) {  // uniform
+                const int y0 = static_cast<int>(fl);
+                const int hi = w.n - 1;
+                const int o = v * 2 * sh;
+                const int r0 = (min(min(max(y0 - w.x0, 0), hi) - cy[v], sh - 1) + o) * sw;
+                const int r1 = (min(min(max(min(y0 + 1, w.S - 1) - w.x0, 0), hi) - cy[v], sh - 1) + o) * sw;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float v00 = stage[r0 + s0[h]], v10 = stage[r0 + s1[h]];
+                    const float v01 = stage[r1 + s0[h]], v11 = stage[r1 + s1[h]];
+                    h0[v][h] = v00 + (v10 - v00) * ct[h].tx;
+                    h1[v][h] = v01 + (v11 - v01) * ct[h].tx;
+                }
+                at[v] = fl;
+            }
+            float* row = v == 0 ? up : down;
+            const float v0 = ok && use[0] ? h0[v][0] + (h1[v][0] - h0[v][0]) * f : 0.0f;
+            const float v1 = ok && use[1] ? h0[v][1] + (h1[v][1] - h0[v][1]) * f : 0.0f;
+            if (in) row[ix] = v0;
+            if (mirror) row[-ix] = v1;
+            sum += v0 + v1;
+            m = fmaxf(m, fmaxf(v0, v1));
+        }
+        up += K;
+        down -= K;
+        lsum += sum;
+        lpeak = fmaxf(lpeak, m);
+        int slot = -1;
+        if (exact) {
+            if (in) slot = min(R, ring_i) - rbase;
+            n += 2 * iy + 1;  // the next row's
+            ring_i += n > ring_i * ring_i ? 1 : 0;
+        } else {
+            slot = ring_slot<FUSED>(in, dx, dy, R, rbase);
+        }
+        if (warp_runs_scan<FUSED>(slot, sum, m) && slot >= 0) {
+            float2 e = wring[slot];
+            e.x += sum;
+            if constexpr (FUSED) e.y = fmaxf(e.y, m);
+            wring[slot] = e;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    const size_t ro = static_cast<size_t>(b) * (R + 1);
+    for (int i = tid; i < kRingSpanQuad; i += 256) {
+        if (rbase + i > R) continue;
+        float e = 0.0f, p = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            e += ring[k][i].x;
+            p = fmaxf(p, ring[k][i].y);
+        }
+        if (e != 0.0f) atomicAdd(&(FUSED ? a.ring_ceil : a.ring_round)[ro + rbase + i], static_cast<double>(e));
+        if (FUSED && p != 0.0f) atomicMax(&a.ring_peak[ro + rbase + i], __float_as_uint(p));
+    }
+    resample_totals<FUSED>(a, b, lsum, __float_as_uint(lpeak), tid);
+}
+
+// ---- box-filtered lambda-rescale ------------------------------------------------
+// Samples more than one window pixel apart (scaleFactor < 1) are the mean of
+// taps x taps bilinear samples (sampleSquareFiltered,
+// LensDiffCpuReference.cpp:338-353).  The mean is separable: along each axis
+// the taps' bilinear weights add up to weights on a run of at most
+// kFilterSpan window pixels (taps <= 6, footprint <= 20: five steps of at
+// most 20 / 6 and the two pixels of a tap).  A CTA forms the column weights
+// of its 32 canvas columns and the row weights of its th canvas rows once;
+// each warp then takes a canvas row at a time: the run of window rows into
+// one weighted row (coalesced: lanes are window columns), from which its 32
+// lanes take their weighted runs.  Per canvas pixel about footprint x run
+// multiply-adds instead of taps^2 bilinear samples of ~40 instructions.
+// Bound by the latency of the window reads: 71 us for 16 wavelengths at
+// K = 513 with footprints 3.3-5.7 and PSF size 1024 (186 us sampling tap by
+// tap), 20 us for 3 at K = 257 with footprints 5.2-9.1 (77 us).
+constexpr int kFilterSpan = 20;
+constexpr int kFilterRow = 672;  // >= 31 * 20 + 17 + 3 window columns under 32 canvas columns
+
+struct FilterSmem {
+    float row[8][kFilterRow];          // per warp: the window rows of one canvas row, weighted
+    float cw[kFilterSpan][kTile];      // column weights [run][canvas column]
+    float rw[kTallH][kFilterSpan];     // row weights [canvas row][run]
+    int r0[kTallH], rn[kTallH];        // first window row of a canvas row's run, and its length
+    int cx0, span;                     // window columns the tile reads
+    float ring[2 * kRingSpanTall];     // RingSmem
+};
+
+// Weights of the taps around coordinate p on a run of window pixels from
+// *first on (w[j * stride], j < the returned length; 0: no tap inside
+// [0, S - 1], where sampleSquareBilinear is zero).
+__device__ __forceinline__ int tap_weights(const Window& win, float p, float footprint, int taps, float step, float* w,
+                                           int stride, int* first) {
+    for (int j = 0; j < kFilterSpan; ++j) w[j * stride] = 0.0f;
+    const float lim = static_cast<float>(win.S - 1);
+    const int hi = win.n - 1;
+    int lo = 0, n = 0;
+    for (int t = 0; t < taps; ++t) {
+        const float q = p + ((static_cast<float>(t) + 0.5f) * step - footprint * 0.5f);
+        if (q < 0.0f || q > lim) continue;
+        const int i0 = static_cast<int>(floorf(q));
+        const float f = q - static_cast<float>(i0);
+        const int a0 = min(max(i0 - win.x0, 0), hi);
+        const int a1 = min(max(min(i0 + 1, win.S - 1) - win.x0, 0), hi);
+        if (n == 0) lo = a0;
+        const int j0 = min(a0 - lo, kFilterSpan - 1), j1 = min(a1 - lo, kFilterSpan - 1);
+        w[j0 * stride] += 1.0f - f;
+        w[j1 * stride] += f;
+        n = j1 + 1;
+    }
+    *first = lo;
+    return n;
+}
+
+// The 32 x th canvas tile (tx, ty) of wavelength b; block (32, 8).
+template <bool FUSED>
+__device__ __forceinline__ void resample_filtered(const PsfBankArgs& a, int tx, int ty, int b, int th,
+                                                  FilterSmem& fs) {
+    RingSmem<FUSED>& sm = *reinterpret_cast<RingSmem<FUSED>*>(fs.ring);
+    const WavelengthInfo* wi = a.wl + b;
+    const int tid = threadIdx.x + threadIdx.y * 32;
+    const int K = a.K, R = a.R;
+    const int tx0 = tx * kTile, ty0 = ty * th;
+    const int rbase = tile_ring_base(tx0, ty0, R, R, th);
+    sm.clear(tid);
     const Window w{a.win + static_cast<size_t>(b) * a.win_stride * a.win_stride, a.win_stride, wi->win_x0,
                    wi->win_n, a.S};
     const float kc = static_cast<float>(K - 1) * 0.5f;
@@ -418,168 +540,110 @@ __device__ void resample_tile(const PsfBankArgs& a, int b, int rbase, ResampleSm
     const int taps = wi->taps;
     const float step = wi->step;
     const float rc = a.raw_center;
-    float* canvas = a.canvas + static_cast<size_t>(b) * K * K;
-    float lsum = 0.0f;  // this thread's pixels; one double add per thread at the flush
-    unsigned int lpeak = 0u;
-    const int x = tx0 + threadIdx.x;
+    const int lane = threadIdx.x;
+    const int x = tx0 + lane;
     const bool in = x < K;
     const float dx = static_cast<float>(x) - kc;
-    StageBox bx;
-    if (stage_box(w, rc, kc, inv, taps, tx0, ty0, K, &bx)) {  // uniform per CTA
-        stage_load(w, bx, sm.stage, tid);
-        __syncthreads();
-        const ColTap ct = col_tap(w, rc + dx * inv);
-        const int sx0 = ct.ax0 - bx.cx0, sx1 = ct.ax1 - bx.cx0;
-#pragma unroll 4
-        for (int i = 0; i < kTallH / 8; ++i) {
-            const int y = ty0 + threadIdx.y + 8 * i;
-            if (y >= K) break;  // uniform: a warp is one canvas row
-            const float dy = static_cast<float>(y) - kc;
-            const float v = staged_sample(w, ct, sx0, sx1, bx.cy0, sm.stage, in, rc + dy * inv);
-            if (in) canvas[static_cast<size_t>(y) * K + x] = v;
-            lsum += v;
-            if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
-            warp_runs_accumulate<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v, sm.ring, sm.ring_p);
+    int c0 = 0, cn = 0;
+    if (threadIdx.y == 7) {  // the last warp: column weights (the rows' threads come first)
+        if (in) cn = tap_weights(w, rc + dx * inv, inv, taps, step, &fs.cw[0][lane], kTile, &c0);
+        const int lo = __reduce_min_sync(0xffffffffu, cn > 0 ? c0 : INT_MAX);
+        const int hi = __reduce_max_sync(0xffffffffu, cn > 0 ? c0 + cn : 0);
+        if (lane == 0) {
+            fs.cx0 = hi > 0 ? lo : 0;
+            fs.span = hi > 0 ? min(hi - lo, kFilterRow) : 0;
         }
-    } else {
-        __syncthreads();
-        const ColTap ct = col_tap(w, rc + dx * inv);
-#pragma unroll 4
-        for (int i = 0; i < kTallH / 8; ++i) {
-            const int y = ty0 + threadIdx.y + 8 * i;
-            if (y >= K) break;  // uniform: a warp is one canvas row (the last tile row is mostly past K)
-            const float dy = static_cast<float>(y) - kc;
-            float v = 0.0f;
-            if (in) {
-                v = taps == 0 ? sample_row(w, ct, rc + dy * inv)
-                              : sample_filtered(w, rc + dx * inv, rc + dy * inv, inv, taps, step);
-                canvas[static_cast<size_t>(y) * K + x] = v;
-                lsum += v;
-                if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
+        fs.row[0][lane] = __int_as_float(c0);  // handed to the other warps, which share the columns
+        fs.row[1][lane] = __int_as_float(cn);
+    }
+    for (int r = tid; r < th; r += 224) {
+        if (tid >= 224) break;
+        const float dy = static_cast<float>(ty0 + r) - kc;
+        fs.rn[r] = ty0 + r < K ? tap_weights(w, rc + dy * inv, inv, taps, step, fs.rw[r], 1, &fs.r0[r]) : 0;
+    }
+    __syncthreads();
+    const int cx0 = fs.cx0, span = fs.span;
+    c0 = __float_as_int(fs.row[0][lane]) - cx0;
+    cn = __float_as_int(fs.row[1][lane]);
+    const int cmax = __reduce_max_sync(0xffffffffu, cn);
+    __syncthreads();  // row[] is free
+    const float area = static_cast<float>(taps * taps);
+    float* canvas = a.canvas + static_cast<size_t>(b) * K * K;
+    float* vrow = fs.row[threadIdx.y];
+    float lsum = 0.0f;
+    unsigned int lpeak = 0u;
+    const int rows = th / 8;
+    for (int i = 0; i < rows; ++i) {
+        const int r = threadIdx.y + 8 * i;
+        const int y = ty0 + r;
+        if (y >= K) break;  // uniform: a warp is one canvas row
+        const int rn = fs.rn[r];
+        float v = 0.0f;
+        if (rn > 0 && span > 0) {  // uniform
+            const float* base = w.p + static_cast<size_t>(fs.r0[r]) * w.stride + cx0;
+            // kU window columns per lane, kJ rows at a time: twenty reads in
+            // flight per lane, since the windows come from L2 or HBM (with
+            // eight in flight the HD bank took 103 us instead of 69)
+            constexpr int kU = 2, kJ = 10;
+            for (int c = lane; c < span; c += 32 * kU) {
+                const int o0 = c, o1 = min(c + 32, span - 1);
+                float acc0 = 0.0f, acc1 = 0.0f;
+                for (int j0 = 0; j0 < rn; j0 += kJ) {
+                    float v0[kJ], v1[kJ];
+#pragma unroll
+                    for (int j = 0; j < kJ; ++j) {
+                        const float* p = base + min(j0 + j, rn - 1) * w.stride;  // past the run: weight 0
+                        v0[j] = __ldg(p + o0);
+                        v1[j] = __ldg(p + o1);
+                    }
+#pragma unroll
+                    for (int j = 0; j < kJ; ++j) {
+                        acc0 += fs.rw[r][j0 + j] * v0[j];
+                        acc1 += fs.rw[r][j0 + j] * v1[j];
+                    }
+                }
+                vrow[c] = acc0;
+                if (c + 32 < span) vrow[c + 32] = acc1;
             }
-            warp_runs_accumulate<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v, sm.ring, sm.ring_p);
+            __syncwarp();
+            float sum = 0.0f;
+            for (int j = 0; j < cmax; ++j)
+                if (j < cn) sum += fs.cw[j][lane] * vrow[c0 + j];
+            v = sum / area;
+            __syncwarp();
         }
+        if (in) canvas[static_cast<size_t>(y) * K + x] = v;
+        lsum += v;
+        if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
+        const float dy = static_cast<float>(y) - kc;
+        warp_runs_accumulate<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v, v, sm.ring, sm.ring_p);
     }
     resample_flush<FUSED>(a, b, rbase, sm, lsum, lpeak, tid);
 }
 
-// grid (ceil(K/32), ceil(K/128), B), block (32, 8): wavelength blockIdx.z.
+// The rescale of a whole bank, 1-D grid, block (32, 8): nq quadrant tiles
+// (qx x qy per wavelength), then the box-filtered tiles (fx x fy per
+// wavelength).  Each wavelength's work is in the tiles of its own kind.
+struct ResampleGrid {
+    int nq, qx, qy, qth, sw, sh;
+    int fx, fy, fth;
+};
 template <bool FUSED>
-__global__ void __launch_bounds__(256) resample_kernel(PsfBankArgs a) {
-    __shared__ ResampleSmem<FUSED> sm;
-    const int tid = threadIdx.x + threadIdx.y * 32;
-    const int rbase = tile_ring_base<kTallH>(blockIdx.x * kTile, blockIdx.y * kTallH, a.R, a.R);
-    resample_tile<FUSED>(a, blockIdx.z, rbase, sm, tid);
-}
-
-// warp_runs_accumulate for the same pixels of two wavelengths: one ring
-// geometry (slot, run heads) for both, each wavelength's run sums and peaks
-// formed by the same scan steps in the same order as the single form.
-template <bool PEAK>
-__device__ __forceinline__ void warp_runs_accumulate2(int slot, float v0, float v1, float* ring0,
-                                                      unsigned int* peak0, float* ring1, unsigned int* peak1) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int prev = __shfl_up_sync(full, slot, 1);
-    const unsigned heads = __ballot_sync(full, lane == 0 || prev != slot);
-    const int head = 31 - __clz(heads & (full >> (31 - lane)));
-    float s0 = v0, s1 = v1, m0 = v0, m1 = v1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float t0 = __shfl_up_sync(full, s0, o);
-        const float t1 = __shfl_up_sync(full, s1, o);
-        const float u0 = PEAK ? __shfl_up_sync(full, m0, o) : 0.0f;
-        const float u1 = PEAK ? __shfl_up_sync(full, m1, o) : 0.0f;
-        if (lane - o >= head) {
-            s0 += t0;
-            s1 += t1;
-            if (PEAK) {
-                m0 = fmaxf(m0, u0);
-                m1 = fmaxf(m1, u1);
-            }
-        }
+__global__ void __launch_bounds__(256) resample_kernel(PsfBankArgs a, ResampleGrid g) {
+    extern __shared__ float2 smem[];
+    int i = blockIdx.x;
+    if (i < g.nq) {
+        const int b = i / (g.qx * g.qy);
+        if (a.wl[b].taps != 0) return;
+        i -= b * g.qx * g.qy;
+        resample_quad<FUSED>(a, i % g.qx, i / g.qx, b, g.qth, g.sw, g.sh, smem);
+    } else {
+        i -= g.nq;
+        const int b = i / (g.fx * g.fy);
+        if (a.wl[b].taps == 0) return;
+        i -= b * g.fx * g.fy;
+        resample_filtered<FUSED>(a, i % g.fx, i / g.fx, b, g.fth, *reinterpret_cast<FilterSmem*>(smem));
     }
-    const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u) != 0u;
-    if (tail && slot >= 0) {
-        if (s0 != 0.0f) atomicAdd(&ring0[slot], s0);
-        if (s1 != 0.0f) atomicAdd(&ring1[slot], s1);
-        if (PEAK && m0 != 0.0f) atomicMax(&peak0[slot], __float_as_uint(m0));
-        if (PEAK && m1 != 0.0f) atomicMax(&peak1[slot], __float_as_uint(m1));
-    }
-}
-
-// grid (ceil(K/32), ceil(K/128), B / 2), block (32, 8): wavelengths 2z and
-// 2z + 1 of the same tile.  When both are staged, one pass over the tile
-// samples both from their staged windows and takes each pixel's ring slot and
-// run boundaries once for the two; otherwise the two tiles run in turn.  The
-// canvases and every statistic equal those of resample_kernel.
-template <bool FUSED>
-__global__ void __launch_bounds__(256) resample_pair_kernel(PsfBankArgs a) {
-    __shared__ ResampleSmem<FUSED> sm[2];
-    const int tid = threadIdx.x + threadIdx.y * 32;
-    const int K = a.K, R = a.R;
-    const int tx0 = blockIdx.x * kTile, ty0 = blockIdx.y * kTallH;
-    const int rbase = tile_ring_base<kTallH>(tx0, ty0, R, R);
-    const int b0 = 2 * blockIdx.z, b1 = b0 + 1;
-    const WavelengthInfo* wi0 = a.wl + b0;
-    const WavelengthInfo* wi1 = a.wl + b1;
-    const size_t wsz = static_cast<size_t>(a.win_stride) * a.win_stride;
-    const Window w0{a.win + b0 * wsz, a.win_stride, wi0->win_x0, wi0->win_n, a.S};
-    const Window w1{a.win + b1 * wsz, a.win_stride, wi1->win_x0, wi1->win_n, a.S};
-    const float kc = static_cast<float>(K - 1) * 0.5f;
-    const float rc = a.raw_center;
-    const float inv0 = wi0->inv_scale, inv1 = wi1->inv_scale;
-    StageBox bx0, bx1;
-    const bool joint = stage_box(w0, rc, kc, inv0, wi0->taps, tx0, ty0, K, &bx0) &&
-                       stage_box(w1, rc, kc, inv1, wi1->taps, tx0, ty0, K, &bx1);  // uniform per CTA
-    if (!joint) {
-        resample_tile<FUSED>(a, b0, rbase, sm[0], tid);
-        resample_tile<FUSED>(a, b1, rbase, sm[1], tid);
-        return;
-    }
-    for (int i = tid; i < kRingSpanTall; i += 256) {
-        sm[0].ring[i] = 0.0f;
-        sm[1].ring[i] = 0.0f;
-        if constexpr (FUSED) {
-            sm[0].ring_p[i] = 0u;
-            sm[1].ring_p[i] = 0u;
-        }
-    }
-    stage_load(w0, bx0, sm[0].stage, tid);
-    stage_load(w1, bx1, sm[1].stage, tid);
-    __syncthreads();
-    const int x = tx0 + threadIdx.x;
-    const bool in = x < K;
-    const float dx = static_cast<float>(x) - kc;
-    const ColTap ct0 = col_tap(w0, rc + dx * inv0), ct1 = col_tap(w1, rc + dx * inv1);
-    const int s00 = ct0.ax0 - bx0.cx0, s01 = ct0.ax1 - bx0.cx0;
-    const int s10 = ct1.ax0 - bx1.cx0, s11 = ct1.ax1 - bx1.cx0;
-    float* canvas0 = a.canvas + static_cast<size_t>(b0) * K * K;
-    float* canvas1 = a.canvas + static_cast<size_t>(b1) * K * K;
-    float lsum0 = 0.0f, lsum1 = 0.0f;
-    unsigned int lpeak0 = 0u, lpeak1 = 0u;
-#pragma unroll 2
-    for (int i = 0; i < kTallH / 8; ++i) {
-        const int y = ty0 + threadIdx.y + 8 * i;
-        if (y >= K) break;  // uniform: a warp is one canvas row
-        const float dy = static_cast<float>(y) - kc;
-        const float v0 = staged_sample(w0, ct0, s00, s01, bx0.cy0, sm[0].stage, in, rc + dy * inv0);
-        const float v1 = staged_sample(w1, ct1, s10, s11, bx1.cy0, sm[1].stage, in, rc + dy * inv1);
-        if (in) {
-            canvas0[static_cast<size_t>(y) * K + x] = v0;
-            canvas1[static_cast<size_t>(y) * K + x] = v1;
-        }
-        lsum0 += v0;
-        lsum1 += v1;
-        if constexpr (FUSED) {
-            lpeak0 = max(lpeak0, __float_as_uint(v0));
-            lpeak1 = max(lpeak1, __float_as_uint(v1));
-        }
-        warp_runs_accumulate2<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v0, v1, sm[0].ring, sm[0].ring_p,
-                                     sm[1].ring, sm[1].ring_p);
-    }
-    resample_flush<FUSED>(a, b0, rbase, sm[0], lsum0, lpeak0, tid);
-    resample_flush<FUSED>(a, b1, rbase, sm[1], lsum1, lpeak1, tid);
 }
 
 // Sum over rings of the unnormalised azimuthal mean, i.e. the normaliser of
@@ -623,7 +687,7 @@ __global__ void __launch_bounds__(256) ring_sums_kernel(PsfBankArgs a) {
     const int K = a.K, R = a.R;
     const int tx0 = blockIdx.x * kTile, ty0 = blockIdx.y * kTallH;
     const int tid = threadIdx.x + threadIdx.y * 32;
-    const int rbase = tile_ring_base<kTallH>(tx0, ty0, R, R);
+    const int rbase = tile_ring_base(tx0, ty0, R, R, kTallH);
     for (int i = tid; i < kRingSpanTall; i += 256) ring[i] = 0.0f;
     __syncthreads();
     const float kc = static_cast<float>(K - 1) * 0.5f;
@@ -640,7 +704,7 @@ __global__ void __launch_bounds__(256) ring_sums_kernel(PsfBankArgs a) {
             v = __ldg(canvas + static_cast<size_t>(y) * K + x);
             slot = min(R, static_cast<int>(roundf(sqrtf(dx * dx + dy * dy)))) - rbase;
         }
-        warp_runs_accumulate<false>(slot, v, ring, nullptr);
+        warp_runs_accumulate<false>(slot, v, v, ring, nullptr);
     }
     __syncthreads();
     const size_t ro = static_cast<size_t>(b) * (R + 1);
@@ -661,7 +725,7 @@ __global__ void __launch_bounds__(256) shape_stats_kernel(PsfBankArgs a) {
     const double s1 = a.scalars[b].s1;
     const int K = a.K, R = a.R;
     const int tx0 = blockIdx.x * kTile, ty0 = blockIdx.y * kTallH;
-    const int rbase = tile_ring_base<kTallH>(tx0, ty0, R, R);
+    const int rbase = tile_ring_base(tx0, ty0, R, R, kTallH);
     // ring means (round(r) rings) the tile can touch
     const float* rm = a.ring_mean + static_cast<size_t>(b) * (R + 1);
     for (int i = tid; i < kRingSpanTall; i += 256) {
@@ -705,7 +769,7 @@ __global__ void __launch_bounds__(256) shape_stats_kernel(PsfBankArgs a) {
             lpeak = max(lpeak, __float_as_uint(v));
             slot = min(R, static_cast<int>(ceilf(rad))) - rbase;
         }
-        warp_runs_accumulate<true>(slot, v, ring_e, ring_p);
+        warp_runs_accumulate<true>(slot, v, v, ring_e, ring_p);
     }
     __syncthreads();
     const size_t ro = static_cast<size_t>(b) * (R + 1);
@@ -1257,43 +1321,41 @@ void launch_psf_cols(const PsfBankArgs& a, cudaStream_t s) {
 
 bool fused_shaping(const PsfBankArgs& a) { return a.gain == 1.0f; }
 
-// The bank's wavelengths from b0 on, as a bank of their own (the per-wavelength
-// arrays the canvas passes index by wavelength, advanced to b0).
-PsfBankArgs bank_from(const PsfBankArgs& a, int b0) {
-    PsfBankArgs t = a;
-    const size_t rr = static_cast<size_t>(a.R) + 1;
-    t.wl = a.wl + b0;
-    t.win = a.win + static_cast<size_t>(b0) * a.win_stride * a.win_stride;
-    t.canvas = a.canvas + static_cast<size_t>(b0) * a.K * a.K;
-    t.ring_round = a.ring_round + b0 * rr;
-    t.ring_ceil = a.ring_ceil + b0 * rr;
-    t.ring_peak = a.ring_peak + b0 * rr;
-    t.ring_mean = a.ring_mean ? a.ring_mean + b0 * rr : nullptr;
-    t.scalars = a.scalars + b0;
-    t.B = a.B - b0;
-    return t;
-}
-
-// Wavelengths in pairs (resample_pair_kernel) when none is box-filtered, the
-// last one of an odd count on its own; else one per CTA.
-void launch_resample(const PsfBankArgs& a, bool pairs, cudaStream_t s) {
-    const bool fused = fused_shaping(a);
-    if (!pairs) {
-        if (fused) resample_kernel<true><<<tall_grid(a), dim3(32, 8), 0, s>>>(a);
-        else resample_kernel<false><<<tall_grid(a), dim3(32, 8), 0, s>>>(a);
-        return;
+// filtered: some wavelength is box-filtered; inv_max: the largest sample
+// distance of the others (0: none).
+// Filtered tiles: 32 rows, or 16 where 128-row tiles would not give every SM
+// one CTA.  The canvas under a box filter reaches far outside the PSF, where
+// its pixels are zero, so only the central tiles have work and short ones
+// spread it: 128 / 64 / 32 / 16 / 8 rows took 197 / 70 / 69 / 78 / 100 us for
+// 16 wavelengths at K = 513, 73 / 24 / 26 / 16 / 14 us for 3 at K = 257.
+// Quadrant tiles: 128 rows (112 us for 31 wavelengths at K = 1025 and
+// inv_scale <= 0.40, 118 us with 64), 64 where the staged boxes of 128 rows
+// would take over 25 KB and cost resident CTAs (inv_max > 0.5), 16 where 64
+// rows would not give every SM two CTAs.
+void launch_resample(const PsfBankArgs& a, bool filtered, float inv_max, cudaStream_t s) {
+    ResampleGrid g{};
+    size_t sm = 0;
+    int grid = 0;
+    if (inv_max > 0.0f) {
+        g.qx = (a.R + kTile) / kTile;
+        g.qth = g.qx * ((a.R + 64) / 64) * a.B < 2 * 148 ? 16 : (inv_max <= 0.5f ? kQuadH : 64);
+        g.qy = (a.R + g.qth) / g.qth;
+        g.sw = quad_stage(kTile, inv_max);
+        g.sh = quad_stage(g.qth, inv_max);
+        g.nq = g.qx * g.qy * a.B;
+        sm = kQuadRingBytes + 4 * sizeof(float) * g.sw * g.sh;
+        grid = g.nq;
     }
-    if (a.B >= 2) {
-        dim3 g = tall_grid(a);
-        g.z = a.B / 2;
-        if (fused) resample_pair_kernel<true><<<g, dim3(32, 8), 0, s>>>(a);
-        else resample_pair_kernel<false><<<g, dim3(32, 8), 0, s>>>(a);
+    if (filtered) {
+        const dim3 tall = tall_grid(a);
+        g.fth = tall.x * tall.y * tall.z < 148 ? 16 : kTile;
+        g.fx = tall.x;
+        g.fy = (a.K + g.fth - 1) / g.fth;
+        sm = std::max(sm, sizeof(FilterSmem));
+        grid += g.fx * g.fy * a.B;
     }
-    if (a.B & 1) {
-        const PsfBankArgs t = bank_from(a, a.B - 1);
-        if (fused) resample_kernel<true><<<tall_grid(t), dim3(32, 8), 0, s>>>(t);
-        else resample_kernel<false><<<tall_grid(t), dim3(32, 8), 0, s>>>(t);
-    }
+    if (fused_shaping(a)) resample_kernel<true><<<grid, dim3(32, 8), sm, s>>>(a, g);
+    else resample_kernel<false><<<grid, dim3(32, 8), sm, s>>>(a, g);
 }
 
 void launch_shape_stats(const PsfBankArgs& a, cudaStream_t s) {
@@ -1352,6 +1414,9 @@ void launch_normalize_psf(float* psf, int n, const PsfScalars* sc, cudaStream_t 
 }
 
 void configure_psf_kernels() {
+    const size_t quad = kQuadRingBytes + 4 * sizeof(float) * quad_stage(kTile, 1.0f) * quad_stage(64, 1.0f);
+    opt_in(resample_kernel<true>, quad);
+    opt_in(resample_kernel<false>, quad);
     opt_in(psf_rows_kernel<kE25>, 12800 * 8);
     opt_in(psf_rows_kernel<kE16>, 16384 * 8);
     opt_in(psf_cols_kernel<kE25, 4>, 2048 * 4 * 8);
