@@ -252,20 +252,22 @@ _SCALAR_MAP = {
 }
 
 
+# (attribute, C field, conversion) of every scalar, resolved once: looking the
+# C types up per call made a conversion take 160 us, most of a small frame's time.
+_SCALARS = [(src, dst, int if dict(_PARAM_FIELDS)[dst] is c_i32 else float) for src, dst in _SCALAR_MAP.items()]
+
+
 def to_abi_params(p: LensDiffParams) -> ld_params:
     """Packs a LensDiffParams into the C struct (a field-by-field copy)."""
     out = ld_params()
-    for src, dst in _SCALAR_MAP.items():
-        v = getattr(p, src)
-        ftype = dict(_PARAM_FIELDS)[dst]
-        setattr(out, dst, int(v) if ftype is c_i32 else float(v))
+    for src, dst, conv in _SCALARS:
+        setattr(out, dst, conv(getattr(p, src)))
     if p.wavelengthsNm:
-        w = list(p.wavelengthsNm)
+        w = [float(x) for x in p.wavelengthsNm]
         if len(w) > MAX_WAVELENGTHS:
             raise ValueError(f"at most {MAX_WAVELENGTHS} wavelengths")
         out.wavelength_count = len(w)
-        for i, x in enumerate(w):
-            out.wavelengths_nm[i] = float(x)
+        out.wavelengths_nm[:len(w)] = w
     out.rgb_mode = int(p.rgbMode)
     out.field_grid = int(p.fieldGrid)
     nb = len(resolved_wavelengths(p))
@@ -275,14 +277,12 @@ def to_abi_params(p: LensDiffParams) -> ld_params:
             for r in range(3):
                 if len(mat[r]) < nb:
                     raise ValueError(f"{name} row {r} needs {nb} entries")
-                for b in range(nb):
-                    arr[r * nb + b] = float(mat[r][b])
-    for i in range(3):
-        out.rgb_gauss_center_nm[i] = float(p.rgbGaussCenterNm[i])
+                arr[r * nb:(r + 1) * nb] = [float(mat[r][b]) for b in range(nb)]
+    out.rgb_gauss_center_nm[:] = [float(p.rgbGaussCenterNm[i]) for i in range(3)]
     out.rgb_gauss_sigma_nm = float(p.rgbGaussSigmaNm)
     if p.noll is not None:
-        for j, v in enumerate(p.noll[:NOLL_COUNT]):
-            out.noll[j] = float(v)
+        noll = [float(v) for v in p.noll[:NOLL_COUNT]]
+        out.noll[:len(noll)] = noll
     out.fft_form = int(p.fftForm)
     return out
 
