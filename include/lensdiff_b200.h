@@ -240,8 +240,8 @@ enum {
     LD_STAGE_PUPIL, LD_STAGE_COMPOSITE, LD_STAGE_SCATTER, LD_STAGE_WORKING_SOURCE,
     LD_STAGE_DFT_GEMM, LD_STAGE_COUNT
 };
-/* Per-frame chains are captured into CUDA graphs on first use and replayed
- * when a later frame issues identical launches (same buffers, geometry and
+/* Per-frame chains are captured into CUDA graphs on their second use and
+ * replayed when a later frame issues identical launches (same buffers, geometry and
  * parameters); enable = 0 launches every kernel directly.  On by default;
  * graphs are never used while stage profiling is on or when the caller's
  * stream is being captured.  No counterpart in the reference. */

@@ -121,6 +121,8 @@ struct ld_ctx {
     };
     std::vector<GraphEntry> graphs;
     uint64_t graph_clock = 0;
+    std::vector<size_t> graph_seen;  // hashes of the last chains launched without a graph (run_chain)
+    size_t graph_seen_next = 0;
     bool graphs_enabled = true;
     // work buffers, grown on demand
     DevBuf rows, win, combine_out, kspec_rows, frameA, frameB, calib, calib_psf, pupil_pre, effect;
@@ -2154,6 +2156,7 @@ int ld_gaussian_rgb_matrix(const float* wl, int32_t count, const float* center, 
 namespace {
 
 constexpr size_t kGraphCache = 4;
+constexpr size_t kGraphSeen = 4;  // covers the three spectra slots that a stream of new lenses rotates through
 
 // ---------------------------------------------------------------------------
 // Autotuner of the fixed transform plans (ld_fxplans.h)
@@ -2240,9 +2243,14 @@ void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
     }
 }
 
-// Issues a frame chain through a cached CUDA graph: on the first call with a
-// given key the chain is captured (thread-local capture mode) and
-// instantiated, later calls with the same key launch the graph.  The key is
+// Issues a frame chain through a cached CUDA graph: the first call with a
+// given key launches the chain directly, the second within the last
+// kGraphSeen new keys captures it (thread-local capture mode) and
+// instantiates it, later calls with the same key launch the graph.  A capture
+// costs ~100 us of host time, four times the direct launches, so a program
+// that moves through more lenses or frames than kGraphCache never pays for
+// graphs that it will not replay (24 lenses in turn: 138 us of host time a
+// render capturing each, 37 us launching).  The key is
 // the bytes of every argument the chain's launches take, so a graph is only
 // replayed for identical launches (buffer contents may differ: the kernels
 // read them when the graph runs).  Direct launches when profiling (stage
@@ -2262,6 +2270,14 @@ void run_chain(ld_ctx* c, cudaStream_t s, const std::string& key, const std::fun
             check_cuda(cudaGraphLaunch(g.exec, s), "graph-launch");
             return;
         }
+    }
+    const size_t hash = std::hash<std::string>()(key);
+    if (std::find(c->graph_seen.begin(), c->graph_seen.end(), hash) == c->graph_seen.end()) {
+        if (c->graph_seen.size() < kGraphSeen) c->graph_seen.push_back(hash);
+        else c->graph_seen[c->graph_seen_next] = hash;
+        c->graph_seen_next = (c->graph_seen_next + 1) % kGraphSeen;
+        chain();
+        return;
     }
     const int before = c->launches;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
