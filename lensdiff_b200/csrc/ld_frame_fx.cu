@@ -1,6 +1,7 @@
-// ld_frame_fx.cu — the frame chain's FFT kernels instantiated on the fixed
-// plans of ld_fxplans.h (compile-time length and radix order, ld_fftx.cuh),
-// their launchers, and the FP64 generation of the plans' stage twiddle tables.
+// ld_frame_fx.cu — the frame chain's row kernels instantiated on the row plans
+// of ld_fxplans.h (compile-time length and radix order, ld_fftx.cuh), the
+// launchers of every fixed plan (the column plans' kernels are in
+// ld_fx_cols*.cu), and the FP64 generation of the plans' stage twiddle tables.
 //
 // Each fx_launch_* returns false when no fixed instantiation covers the
 // launch (another length, channel count or form); the caller then launches
@@ -15,30 +16,19 @@
 namespace ld {
 namespace {
 
-// Fixed plan ID: its transform type, the passes it serves (kRowPlan: the
-// frame's row transforms, length M; kColPlan: its column transforms, length
-// Py) and the elements per thread E its kernels are compiled for (ld_fxplans.h).
-constexpr int kRowPlan = 1, kColPlan = 2;
+// Row plan ID: its transform type.
 template <int ID>
 struct FxType;
-template <class F, int ROLE, int FAM>
+template <class F>
 struct FxTypeOf {
     using type = F;
-    static constexpr int role = ROLE;
-    static constexpr int E = FAM;
 };
-template <> struct FxType<1> : FxTypeOf<FixedFft<2500, 25, 25, 4>, kRowPlan, kE25> {};
-template <> struct FxType<2> : FxTypeOf<FixedFft<2500, 25, 4, 25>, kRowPlan, kE25> {};
-template <> struct FxType<3> : FxTypeOf<FixedFft<3200, 25, 16, 8>, kColPlan, kE25> {};
-template <> struct FxType<4> : FxTypeOf<FixedFft<3200, 25, 8, 16>, kColPlan, kE25> {};
-template <> struct FxType<5> : FxTypeOf<FixedFft<1250, 25, 25, 2>, kRowPlan, kE25> {};
-template <> struct FxType<6> : FxTypeOf<FixedFft<1250, 25, 2, 25>, kRowPlan, kE25> {};
-template <> struct FxType<7> : FxTypeOf<FixedFft<1600, 25, 16, 4>, kColPlan, kE25> {};
-template <> struct FxType<8> : FxTypeOf<FixedFft<1600, 25, 4, 16>, kColPlan, kE25> {};
-template <> struct FxType<9> : FxTypeOf<FixedFft<1280, 5, 16, 16>, kRowPlan, kE25> {};
-template <> struct FxType<10> : FxTypeOf<FixedFft<1280, 16, 5, 16>, kRowPlan, kE25> {};
-template <> struct FxType<11> : FxTypeOf<FixedFft<3200, 5, 5, 16, 8>, kColPlan, kE16> {};
-template <> struct FxType<12> : FxTypeOf<FixedFft<1600, 5, 5, 16, 4>, kColPlan, kE16> {};
+template <> struct FxType<1> : FxTypeOf<FixedFft<2500, 25, 25, 4>> {};
+template <> struct FxType<2> : FxTypeOf<FixedFft<2500, 25, 4, 25>>  {};
+template <> struct FxType<5> : FxTypeOf<FixedFft<1250, 25, 25, 2>>  {};
+template <> struct FxType<6> : FxTypeOf<FixedFft<1250, 25, 2, 25>>  {};
+template <> struct FxType<9> : FxTypeOf<FixedFft<1280, 5, 16, 16>>  {};
+template <> struct FxType<10> : FxTypeOf<FixedFft<1280, 16, 5, 16>>  {};
 
 // Calls f(FxType<id>{}); false when there is no fixed plan `id`.
 template <class F>
@@ -46,16 +36,10 @@ bool fx_visit(int id, F&& f) {
     switch (id) {
         case 1: f(FxType<1>{}); return true;
         case 2: f(FxType<2>{}); return true;
-        case 3: f(FxType<3>{}); return true;
-        case 4: f(FxType<4>{}); return true;
         case 5: f(FxType<5>{}); return true;
         case 6: f(FxType<6>{}); return true;
-        case 7: f(FxType<7>{}); return true;
-        case 8: f(FxType<8>{}); return true;
         case 9: f(FxType<9>{}); return true;
         case 10: f(FxType<10>{}); return true;
-        case 11: f(FxType<11>{}); return true;
-        case 12: f(FxType<12>{}); return true;
         default: return false;
     }
 }
@@ -64,12 +48,6 @@ bool fx_visit(int id, F&& f) {
 // from __launch_bounds__(T, MINB)).
 constexpr int rows_c(int n) { return fft_threads(n, 2, kE25) <= 224 ? 2 : 4; }
 constexpr int minb_for(int t) { return t <= 128 ? 4 : (t <= 224 ? 3 : 2); }
-// column passes: as many CTAs per SM as the column's working set (four
-// sequences of n complex values) fits in shared memory, at most four
-constexpr int cols_minb(int n) {
-    return kMaxSmem / (32 * n + 1024) >= 4 ? 4 : (kMaxSmem / (32 * n + 1024) >= 3 ? 3 : 2);
-}
-
 template <class FFT>
 void rows_fixed(const FrameArgs& a, cudaStream_t s) {
     constexpr int N = FFT::n;
@@ -80,17 +58,6 @@ void rows_fixed(const FrameArgs& a, cudaStream_t s) {
     auto f = frame_rows_kernel<kE25, C, 1, T, minb_for(T), false, FFT>;
     b.ahead = resident_ctas(f, T, sm);
     f<<<a.Hp / C, T, sm, s>>>(b);
-}
-
-template <class D, bool H16>
-void cols_fixed(FrameArgs a, cudaStream_t s) {
-    using FFT = typename D::type;
-    constexpr int N = FFT::n;
-    constexpr int T = fft_threads(N, 3, D::E);
-    const size_t sm = frame_cols_smem(N, 3);
-    auto f = frame_cols_kernel<D::E, 3, T, cols_minb(N), H16, FFT>;
-    a.ahead = resident_ctas(f, T, sm);
-    f<<<a.g.cols, T, sm, s>>>(a);
 }
 
 template <class FFT, bool H16, int MINB>
@@ -113,17 +80,6 @@ void inverse_fixed(const FrameArgs& a, int rows, cudaStream_t s) {
     else inverse_fixed_m<FFT, H16, minb_for(T)>(a, rows, s);
 }
 
-template <class D, bool H16>
-void kspec_cols_fixed(KernelSpectraArgs a, cudaStream_t s) {
-    using FFT = typename D::type;
-    constexpr int N = FFT::n;
-    constexpr int T = fft_threads(N, 3, D::E);
-    const size_t sm = kspec_cols_smem(N, a.Kp, 3);
-    auto f = kspec_cols_kernel<D::E, 3, T, cols_minb(N), H16, FFT>;
-    a.ahead = resident_ctas(f, T, sm);
-    f<<<a.g.cols, T, sm, s>>>(a);
-}
-
 template <class FFT>
 void kspec_rows_fixed(const KernelSpectraArgs& a, cudaStream_t s) {
     constexpr int T = fft_threads(FFT::n, 3, kE25);
@@ -135,23 +91,15 @@ template <class D>
 void configure_fixed() {
     using FFT = typename D::type;
     constexpr int N = FFT::n;
-    if constexpr (D::role == kRowPlan) {
-        constexpr int C = rows_c(N);
-        constexpr int TR = fft_threads(N, C, kE25);
-        constexpr int T3 = fft_threads(N, 3, kE25);
-        set_smem(frame_rows_kernel<kE25, C, 1, TR, minb_for(TR), false, FFT>);
-        set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3), false, FFT>);
-        set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3), true, FFT>);
-        set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3) + 1, false, FFT>);
-        set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3) + 1, true, FFT>);
-        set_smem(kspec_rows_kernel<kE25, 3, T3, minb_for(T3) + 1, FFT>);
-    } else {
-        constexpr int T3 = fft_threads(N, 3, D::E);
-        set_smem(frame_cols_kernel<D::E, 3, T3, cols_minb(N), false, FFT>);
-        set_smem(frame_cols_kernel<D::E, 3, T3, cols_minb(N), true, FFT>);
-        set_smem(kspec_cols_kernel<D::E, 3, T3, cols_minb(N), false, FFT>);
-        set_smem(kspec_cols_kernel<D::E, 3, T3, cols_minb(N), true, FFT>);
-    }
+    constexpr int C = rows_c(N);
+    constexpr int TR = fft_threads(N, C, kE25);
+    constexpr int T3 = fft_threads(N, 3, kE25);
+    set_smem(frame_rows_kernel<kE25, C, 1, TR, minb_for(TR), false, FFT>);
+    set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3), false, FFT>);
+    set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3), true, FFT>);
+    set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3) + 1, false, FFT>);
+    set_smem(frame_inverse_kernel<kE25, 3, T3, minb_for(T3) + 1, true, FFT>);
+    set_smem(kspec_rows_kernel<kE25, 3, T3, minb_for(T3) + 1, FFT>);
 }
 
 }  // namespace
@@ -160,39 +108,32 @@ bool fx_launch_frame_rows(const FrameArgs& a, cudaStream_t s) {
     if (a.n_drv != 1 || a.drv_effect || a.g.fam_m != kE25) return false;
     bool done = false;
     fx_visit(a.g.plan_m.fixed, [&](auto d) {
-        using D = decltype(d);
-        if constexpr (D::role == kRowPlan) {
-            rows_fixed<typename D::type>(a, s);
-            done = true;
-        }
+        rows_fixed<typename decltype(d)::type>(a, s);
+        done = true;
     });
     return done;
 }
 
+namespace {
+bool cols_dispatch(int id, const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
+    return fx_cols_0(id, fa, ka, s) || fx_cols_1(id, fa, ka, s) || fx_cols_2(id, fa, ka, s) ||
+           fx_cols_3(id, fa, ka, s) || fx_cols_4(id, fa, ka, s) || fx_cols_5(id, fa, ka, s);
+}
+}  // namespace
+
 bool fx_launch_frame_cols(const FrameArgs& a, cudaStream_t s) {
-    if (a.n_drv != 1 || a.n_out != 3 || a.g.fam_py != kE25) return false;
-    bool done = false;
-    fx_visit(a.g.plan_py.fixed, [&](auto d) {
-        using D = decltype(d);
-        if constexpr (D::role == kColPlan) {
-            if (a.h16) cols_fixed<D, true>(a, s);
-            else cols_fixed<D, false>(a, s);
-            done = true;
-        }
-    });
-    return done;
+    if (a.n_drv != 1 || a.n_out != 3 || a.g.plan_py.fixed == 0) return false;
+    return cols_dispatch(a.g.plan_py.fixed, &a, nullptr, s);
 }
 
 bool fx_launch_frame_inverse(const FrameArgs& a, int rows, cudaStream_t s) {
     if (a.n_out != 3 || a.g.fam_m != kE25) return false;
     bool done = false;
     fx_visit(a.g.plan_m.fixed, [&](auto d) {
-        using D = decltype(d);
-        if constexpr (D::role == kRowPlan) {
-            if (a.h16) inverse_fixed<typename D::type, true>(a, rows, s);
-            else inverse_fixed<typename D::type, false>(a, rows, s);
-            done = true;
-        }
+        using F = typename decltype(d)::type;
+        if (a.h16) inverse_fixed<F, true>(a, rows, s);
+        else inverse_fixed<F, false>(a, rows, s);
+        done = true;
     });
     return done;
 }
@@ -201,31 +142,19 @@ bool fx_launch_kspec_rows(const KernelSpectraArgs& a, cudaStream_t s) {
     if (a.n_ker != 3 || a.g.fam_m != kE25) return false;
     bool done = false;
     fx_visit(a.g.plan_m.fixed, [&](auto d) {
-        using D = decltype(d);
-        if constexpr (D::role == kRowPlan) {
-            kspec_rows_fixed<typename D::type>(a, s);
-            done = true;
-        }
+        kspec_rows_fixed<typename decltype(d)::type>(a, s);
+        done = true;
     });
     return done;
 }
 
 bool fx_launch_kspec_cols(const KernelSpectraArgs& a, cudaStream_t s) {
-    if (a.n_ker != 3 || a.g.fam_py != kE25) return false;
-    bool done = false;
-    fx_visit(a.g.plan_py.fixed, [&](auto d) {
-        using D = decltype(d);
-        if constexpr (D::role == kColPlan) {
-            if (a.h16) kspec_cols_fixed<D, true>(a, s);
-            else kspec_cols_fixed<D, false>(a, s);
-            done = true;
-        }
-    });
-    return done;
+    if (a.n_ker != 3 || a.g.plan_py.fixed == 0) return false;
+    return cols_dispatch(a.g.plan_py.fixed, nullptr, &a, s);
 }
 
 void fx_configure() {
-    for (int id = 1; id <= kFxPlanCount; ++id) fx_visit(id, [](auto d) { configure_fixed<decltype(d)>(); });
+    for (const FxPlanDesc& d : kFxPlans) fx_visit(d.id, [](auto t) { configure_fixed<decltype(t)>(); });
 }
 
 // Stage twiddle tables of fixed plan `id`: for every stage after the first,

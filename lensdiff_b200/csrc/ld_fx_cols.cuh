@@ -1,0 +1,257 @@
+// ld_fx_cols.cuh — the column passes on compiled three-stage transforms
+// (ld_fxpass.cuh): the frame's (forward, spectral multiply, inverse) and the
+// kernel spectra's.  Included by the translation units that instantiate the
+// plans' kernels (ld_fx_cols*.cu).
+#pragma once
+
+#include "ld_frame_kernels.cuh"
+#include "ld_fxpass.cuh"
+
+namespace ld {
+namespace {
+
+// Bytes ahead of a column pass's data: mbarriers and the warps' maxima.
+constexpr int kColsHeader = 256;
+struct ColsHeader {
+    uint64_t bar[3];
+    float part[32];
+};
+
+constexpr size_t cols_bytes(int n) { return kColsHeader + static_cast<size_t>(n) * 4 * sizeof(float2); }
+
+// Threads of a column pass over three interleaved sequences: the multiple of
+// 32 with the most useful element slots in flight per SM.  A stage of radix
+// R keeps ceil(3 n / R / T) butterflies of R values per thread in registers
+// (at most 32 values); a thread needs 80 registers, and each CTA its share of
+// shared memory (cols_bytes).
+struct ColsShape {
+    int threads, ctas;
+};
+template <class P>
+constexpr ColsShape cols_shape() {
+    const int radix[3] = {P::R1, P::R2, P::R3};
+    ColsShape best{0, 0};
+    double score = -1.0;
+    for (int t = 96; t <= 800; t += 32) {
+        int steps = 0;
+        bool fits = true;
+        for (int r : radix) {
+            const int it = (3 * P::n / r + t - 1) / t;
+            steps += it * r;
+            if (it * r > 32) fits = false;
+        }
+        const int by_smem = static_cast<int>((228 * 1024) / (cols_bytes(P::n) + 1024));
+        const int by_regs = 65536 / (80 * t);
+        int ctas = by_smem < by_regs ? by_smem : by_regs;
+        if (ctas > 8) ctas = 8;
+        if (!fits || ctas < 1) continue;
+        const double s = 9.0 * P::n / steps * ctas;  // useful slots per SM
+        if (s > score) {
+            score = s;
+            best = ColsShape{t, ctas};
+        }
+    }
+    return best;
+}
+
+// Column k = blockIdx.x: its row spectra transformed, multiplied by its three
+// kernel spectra, the products transformed back, the first Hp rows stored to
+// B.  Shared memory: the header, F [n] (the column's spectrum), W [n][3].
+// H16: the half2 row spectra and their row exponents arrive at the start of W
+// (widened as the forward transform's first stage loads them), the half2
+// kernel spectra in W's upper half (multiplied with F as the inverse's first
+// stage loads them); the forward stages alternate between F and W's lower
+// half, so they need one barrier each.  FP32: the row spectra arrive in F,
+// the kernel spectra fill W.  The inverse's last stage stays in registers:
+// its largest component (H16: the column's scale) and the store come from
+// there.
+// Bound by the latency of its stages: at n = 3200, 24 warps per SM of which the
+// forward stages (a third of the inverse's butterflies) use some, 50 % of the
+// issue slots.  H16 / FP32 launch times, against the passes before it
+// (compiled transforms in place between a fill, a product and a drain; at the
+// other lengths the runtime-planned transforms):
+//   2501 columns of 3200: 138 us (175) / 130 us (155)
+//   4097 columns of 5120: 402 us (757)
+//   1126 columns of 1800: 42 us (101)
+//   1251 columns of 1600: 37 us (50)
+//   1201 columns of 1152: 29 us FP32 (72)
+template <class P, int T, int MINB, bool H16>
+__global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    constexpr int N = P::n;
+    ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
+    float2* F = reinterpret_cast<float2*>(smraw + kColsHeader);
+    float2* W = F + N;
+    const int Hp = a.Hp, cols = a.g.cols;
+    const int k = blockIdx.x;
+    const uint32_t a_bytes = static_cast<uint32_t>(Hp * (H16 ? sizeof(__half2) : sizeof(float2)));
+    constexpr uint32_t k_bytes = static_cast<uint32_t>(N * 3 * (H16 ? sizeof(__half2) : sizeof(float2)));
+    const char* asrc = reinterpret_cast<const char*>(a.A) + static_cast<size_t>(k) * a_bytes;
+    const char* ksrc = reinterpret_cast<const char*>(a.spectra) + static_cast<size_t>(k) * k_bytes;
+    __half2* ah = reinterpret_cast<__half2*>(W);
+    signed char* aex = reinterpret_cast<signed char*>(ah + Hp);
+    __half2* kh = reinterpret_cast<__half2*>(W) + 3 * N;
+    if (threadIdx.x == 0) {
+        mbar_init(&h->bar[0], 1);
+        mbar_init(&h->bar[1], 1);
+        if (H16) mbar_init(&h->bar[2], 1);
+        mbar_init_fence();
+        bulk_load_checked(H16 ? static_cast<void*>(ah) : static_cast<void*>(F), asrc, a_bytes, &h->bar[0], smraw, a.err);
+        if (H16)
+            bulk_load_checked(aex, a.aexp, static_cast<uint32_t>((Hp + 15) & ~15), &h->bar[2], smraw, a.err);
+        bulk_load_checked(H16 ? static_cast<void*>(kh) : static_cast<void*>(W), ksrc, k_bytes, &h->bar[1], smraw, a.err);
+        const int later = k + a.ahead;  // bit 1 of the column plan's shape: no look-ahead (autotuned)
+        if (later < cols && (a.g.plan_py.shape & 2) == 0) {
+            bulk_prefetch_l2(asrc + static_cast<size_t>(later - k) * a_bytes, a_bytes);
+            bulk_prefetch_l2(ksrc + static_cast<size_t>(later - k) * k_bytes, k_bytes);
+        }
+    }
+    __syncthreads();  // barriers initialised before anyone waits on them
+    const float2* tw = a.g.plan_py.stw;
+    if (__syncthreads_or(!mbar_wait(&h->bar[0], 0, a.err) || (H16 && !mbar_wait(&h->bar[2], 0, a.err)))) return;
+    auto ldF = [&](int e) { return F[e]; };
+    auto stF = [&](int e, float2 v) { F[e] = v; };
+    auto ldW = [&](int e) { return W[e]; };
+    auto stW = [&](int e, float2 v) { W[e] = v; };
+    const float2 zero = make_float2(0.0f, 0.0f);
+    if constexpr (H16) {
+        fp_stage<N, 1, T, false, P::R1, 1, false>(
+            nullptr, [&](int e) { return e < Hp ? from_half2(ah[e], exp2_int(aex[e])) : zero; }, stF);
+        __syncthreads();
+        fp_stage<N, 1, T, false, P::R2, P::R1, false>(tw + P::tab2, ldF, stW);
+        __syncthreads();
+        fp_stage<N, 1, T, false, P::R3, P::R1 * P::R2, false>(tw + P::tab3, ldW, stF);
+    } else {
+        fp_stage<N, 1, T, false, P::R1, 1, true>(nullptr, [&](int e) { return e < Hp ? F[e] : zero; }, stF);
+        __syncthreads();
+        fp_stage<N, 1, T, false, P::R2, P::R1, true>(tw + P::tab2, ldF, stF);
+        __syncthreads();
+        fp_stage<N, 1, T, false, P::R3, P::R1 * P::R2, true>(tw + P::tab3, ldF, stF);
+    }
+    if (__syncthreads_or(!mbar_wait(&h->bar[1], 0, a.err))) return;
+    fp_stage<N, 3, T, true, P::R1, 1, true>(
+        nullptr, [&](int e) { return cmul(H16 ? __half22float2(kh[e]) : W[e], F[e / 3]); }, stW);
+    __syncthreads();
+    fp_stage<N, 3, T, true, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+    __syncthreads();
+    LastStage<N, 3, T, true, P::R3> last;
+    last.run(tw + P::tab3, ldW);
+    // element e = row * 3 + c of column k goes to B's group of four columns
+    const int64_t base = (static_cast<int64_t>(k / kBGroup) * Hp * kBGroup + k % kBGroup) * 3;
+    constexpr int step = kBGroup * 3;
+    if constexpr (H16) {
+        float m = 0.0f;
+        last.each([&](int e, float2 v) {
+            if (e < Hp * 3) m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+        });
+        m = cta_max<T>(m, h->part);
+        const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
+        // the kernel spectra's own scale joins the outputs' here
+        if (threadIdx.x == 0) a.bscale[k] = (m > 0.0f ? m / kHalfTop : 1.0f) * a.kscale[k];
+        __half2* out = reinterpret_cast<__half2*>(a.Bout) + base;
+        last.each([&](int e, float2 v) {
+            const int row = e / 3;
+            if (row < Hp) out[row * step + (e - row * 3)] = to_half2(v, sc);
+        });
+    } else {
+        float2* out = a.Bout + base;
+        last.each([&](int e, float2 v) {
+            const int row = e / 3;
+            if (row < Hp) out[row * step + (e - row * 3)] = v;
+        });
+    }
+}
+
+// Column k of the kernel spectra: the row spectra of the canvas rows (Kp x 3)
+// arrive by bulk copy behind W, take their wrapped grid rows as the first
+// stage loads them, and the last stage's registers go out to KS[k] (H16: in
+// FP16 with the column's scale).  2501 columns of 3200 take 97 us (128 before,
+// see above), 4097 of 5120 284 us (517), 1126 of 1800 28 us (66).
+template <class P, int T, int MINB, bool H16>
+__global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArgs a) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    constexpr int N = P::n;
+    ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
+    float2* W = reinterpret_cast<float2*>(smraw + kColsHeader);
+    float2* Rb = W + 3 * N;
+    const int cols = a.g.cols, Kp = a.Kp, R = a.R;
+    const int k = blockIdx.x;
+    const uint32_t r_bytes = static_cast<uint32_t>(Kp * 3 * sizeof(float2));
+    if (threadIdx.x == 0) {
+        mbar_init(&h->bar[0], 1);
+        mbar_init_fence();
+        bulk_load_checked(Rb, a.rows + static_cast<size_t>(k) * Kp * 3, r_bytes, &h->bar[0], smraw, a.err);
+        const int later = k + a.ahead;
+        if (later < cols) bulk_prefetch_l2(a.rows + static_cast<size_t>(later) * Kp * 3, r_bytes);
+    }
+    __syncthreads();  // barrier initialised before anyone waits on it
+    const float2* tw = a.g.plan_py.stw;
+    if (__syncthreads_or(!mbar_wait(&h->bar[0], 0, a.err))) return;
+    auto ldW = [&](int e) { return W[e]; };
+    auto stW = [&](int e, float2 v) { W[e] = v; };
+    // grid row v holds canvas row v + R (v <= R) or v - N + R (v >= N - R)
+    fp_stage<N, 3, T, false, P::R1, 1, false>(
+        nullptr,
+        [&](int e) {
+            const int lo = e + 3 * R, hi = e - 3 * (N - R);
+            if (e < 3 * (R + 1)) return Rb[lo];
+            if (hi >= 0) return Rb[hi];
+            return make_float2(0.0f, 0.0f);
+        },
+        stW);
+    __syncthreads();
+    fp_stage<N, 3, T, false, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+    __syncthreads();
+    LastStage<N, 3, T, false, P::R3> last;
+    last.run(tw + P::tab3, ldW);
+    if constexpr (H16) {
+        float m = 0.0f;
+        last.each([&](int, float2 v) { m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))); });
+        m = cta_max<T>(m, h->part);
+        const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
+        if (threadIdx.x == 0) a.kscale[k] = m > 0.0f ? m / kHalfTop * a.scale : 1.0f;
+        __half2* out = reinterpret_cast<__half2*>(a.spectra) + static_cast<size_t>(k) * N * 3;
+        last.each([&](int e, float2 v) { out[e] = to_half2(v, sc); });
+    } else {
+        float2* out = a.spectra + static_cast<size_t>(k) * N * 3;
+        const float sc = a.scale;
+        last.each([&](int e, float2 v) { out[e] = cscale(v, sc); });
+    }
+}
+
+template <class P, bool H16>
+void frame_cols_fx(FrameArgs a, cudaStream_t s) {
+    constexpr ColsShape sh = cols_shape<P>();
+    static KernelState state;
+    auto f = fx_frame_cols_kernel<P, sh.threads, sh.ctas, H16>;
+    const size_t sm = cols_bytes(P::n);
+    a.ahead = state.get(f, sh.threads, sm);
+    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+}
+
+template <class P, bool H16>
+bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
+    constexpr ColsShape sh = cols_shape<P>();
+    static KernelState state;
+    auto f = fx_kspec_cols_kernel<P, sh.threads, sh.ctas, H16>;
+    const size_t sm = kColsHeader + (static_cast<size_t>(P::n) + a.Kp) * 3 * sizeof(float2);
+    if (sm > kSmemOptIn) return false;
+    a.ahead = state.get(f, sh.threads, cols_bytes(P::n));
+    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+    return true;
+}
+
+// The launch of plan P: the frame's column pass (fa) or the kernel spectra's
+// (ka); false when it does not fit.
+template <class P>
+bool cols_launch(const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
+    if (fa) {
+        if (fa->h16) frame_cols_fx<P, true>(*fa, s);
+        else frame_cols_fx<P, false>(*fa, s);
+        return true;
+    }
+    return ka->h16 ? kspec_cols_fx<P, true>(*ka, s) : kspec_cols_fx<P, false>(*ka, s);
+}
+
+}  // namespace
+}  // namespace ld

@@ -90,8 +90,9 @@ struct ld_ctx {
     std::mutex mu;
     std::map<int, DevBuf> twiddles;
     std::map<int, DevBuf> stage_twiddles;  // by fixed plan id
-    std::map<int, int> fixed_choice;       // transform length -> fixed plan id | shape << 8 (autotuner)
-    std::map<int, double> fixed_ms;        // transform length -> the winner's timed ms
+    // (transform length, role) -> fixed plan id | shape << 8 and the winner's timed ms (autotuner)
+    std::map<std::pair<int, int>, int> fixed_choice;
+    std::map<std::pair<int, int>, double> fixed_ms;
     int autotune = 1;  // 1: tune, 0: first compiled order, -1: runtime-planned transforms only
     int fail_alloc_after = -1;  // fault injection: allocations until one fails (-1: off)
     CustomAperture custom;      // the Custom aperture mode's image
@@ -484,21 +485,23 @@ const float2* stage_twiddles(ld_ctx* c, int id) {
 // one, else the first compiled radix order of that length (0: none).
 // Mode 2 + k pins the k-th compiled order of every length (its last when it
 // has fewer).
-int fixed_plan_for(ld_ctx* c, int n, bool allow25) {
-    if (!allow25 || c->autotune < 0) return 0;  // the fixed launchers serve grids of the 25-element family
+int fixed_plan_for(ld_ctx* c, int n, int role) {
+    if (role == 0 || c->autotune < 0) return 0;
     int ids[8];
-    const int count = fx_candidates(n, ids, 8);
+    const int count = fx_candidates(n, role, ids, 8);
     if (c->autotune >= 2) return count > 0 ? ids[std::min(c->autotune - 2, count - 1)] : 0;
-    auto it = c->fixed_choice.find(n);
+    auto it = c->fixed_choice.find({n, role});
     if (it != c->fixed_choice.end()) return it->second;
     return count > 0 ? ids[0] : 0;
 }
 
-FftPlan make_plan(ld_ctx* c, int n, bool allow25) {
+// The plan of length n: runtime-planned stages, and the fixed plan of `role`
+// (0: none) when one is compiled.
+FftPlan make_plan(ld_ctx* c, int n, bool allow25, int role = 0) {
     FftPlan p{};
     if (!factor_plan(n, allow25, &p)) throw Fail{LD_ERR_UNSUPPORTED, "fft-length-not-5-smooth"};
     p.tw = twiddles(c, n);
-    const int choice = fixed_plan_for(c, n, allow25);
+    const int choice = fixed_plan_for(c, n, role);
     p.fixed = choice & 255;
     p.shape = choice >> 8;
     p.stw = p.fixed ? stage_twiddles(c, p.fixed) : nullptr;
@@ -1542,13 +1545,20 @@ int choose_length(int n, int mult, int C) {
     return best;
 }
 
+// Whether the compiled column plans serve a chain: one driver and three
+// kernels and outputs (the spectral modes without the luma lock).
+bool fx_cols_chain(const Combination& cb, const ld_params& p) {
+    return cb.n_drv == 1 && cb.n_ker == 3 && cb.n_out == 3 && p.fft_form != LD_FFT_CUFFT;
+}
+
 // 5-smooth grid covering the linear convolution: Px = 2M with M the row
 // transform length, Py even (16-byte bulk-copy sizes).  The reference pads to
 // powers of two (LensDiffCpuReference.cpp:1172-1173); any grid of at least
 // W+K-1 x H+K-1 gives the same linear convolution.  c_rows / c_cols: the
 // most interleaved sequences any row / column kernel of the chain transforms
-// (they pick the FFT family).
-GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, int* req_w, int* req_h) {
+// (they pick the FFT family); fx_cols: the compiled column plans serve the
+// chain (fx_cols_chain).
+GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, bool fx_cols, int* req_w, int* req_h) {
     GridGeom g{};
     *req_w = W + K - 1;
     *req_h = H + K - 1;
@@ -1562,8 +1572,8 @@ GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, i
     const int Kp = K + (K & 1);
     if (frame_cols_smem(g.Py, c_cols) > kSmemBudget || kspec_cols_smem(g.Py, Kp, c_cols) > kSmemBudget)
         throw Fail{LD_ERR_UNSUPPORTED, "frame-too-large-for-column-pass"};
-    g.plan_m = make_plan(c, g.M, g.fam_m == kE25);
-    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25);
+    g.plan_m = make_plan(c, g.M, g.fam_m == kE25, g.fam_m == kE25 ? kFxRows : 0);
+    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25, fx_cols ? kFxCols : 0);
     g.tw_px = twiddles(c, g.Px);
     return g;
 }
@@ -1978,7 +1988,7 @@ SpectraGeometry spectra_geometry(ld_ctx* c, const ld_params& p, int W, int H) {
     const int c_rows = std::max(std::max(sg.cb.n_drv == 1 ? 4 : 3, sg.cb.n_out), sg.cb.n_ker);
     const int c_cols = std::max(std::max(sg.cb.n_out, sg.cb.n_ker), sg.cb.n_drv);
     int rw = 0, rh = 0;
-    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, &rw, &rh);
+    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_cols_chain(sg.cb, p), &rw, &rh);
     sg.key = spectra_key_for(bank_key(p, wl), sg.cb, sg.g);
     const bool h16 = chosen_h16(p);
     sg.bytes = sg.cb.parts * (ks_part_bytes(sg.cb.n_ker, sg.g, h16) + static_cast<size_t>(sg.g.cols) * sizeof(float));
@@ -2164,16 +2174,12 @@ constexpr size_t kGraphSeen = 4;  // covers the three spectra slots that a strea
 // Times launch(id, shape) for every compiled radix order of length n and
 // every launch shape in [0, shapes) on stream s (one untimed launch, then
 // kTuneReps between two events) and records the fastest as
-// c->fixed_choice[n] = id | shape << 8.  A single candidate is recorded untimed.
-void tune_length(ld_ctx* c, int n, const std::vector<int>& shapes, cudaStream_t s,
+// c->fixed_choice[{n, role}] = id | shape << 8.
+void tune_length(ld_ctx* c, int n, int role, const std::vector<int>& shapes, cudaStream_t s,
                  const std::function<void(int, int)>& launch) {
     int ids[8];
-    const int k = fx_candidates(n, ids, 8);
-    if (k == 0 || c->fixed_choice.count(n)) return;
-    if (k == 1 && shapes.size() == 1) {
-        c->fixed_choice[n] = ids[0];
-        return;
-    }
+    const int k = fx_candidates(n, role, ids, 8);
+    if (k == 0 || c->fixed_choice.count({n, role})) return;
     constexpr int kTuneReps = 3;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     check_cuda(cudaEventCreate(&e0), "tune-event");
@@ -2201,8 +2207,8 @@ void tune_length(ld_ctx* c, int n, const std::vector<int>& shapes, cudaStream_t 
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     check_launch("autotune");
-    c->fixed_choice[n] = best;
-    c->fixed_ms[n] = best_ms;
+    c->fixed_choice[{n, role}] = best;
+    c->fixed_ms[{n, role}] = best_ms;
 }
 
 // Tunes the row length (frame_rows + frame_inverse, which share its plan; eight
@@ -2214,7 +2220,7 @@ void tune_length(ld_ctx* c, int n, const std::vector<int>& shapes, cudaStream_t 
 // the results it wrote before.
 void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
     if (c->autotune != 1 || fa.effect_mode != kEffectComposite) return;
-    if (c->fixed_choice.count(fa.g.M) && c->fixed_choice.count(fa.g.Py)) return;
+    if (c->fixed_choice.count({fa.g.M, kFxRows}) && c->fixed_choice.count({fa.g.Py, kFxCols})) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -2223,7 +2229,7 @@ void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
     if (fa.g.fam_m == kE25) {
         // shape bits: inverse at one more CTA per SM; row pass, inverse pass
         // without their look-ahead prefetch
-        tune_length(c, fa.g.M, {0, 1, 2, 3, 4, 5, 6, 7}, s, [&](int id, int shape) {
+        tune_length(c, fa.g.M, kFxRows, {0, 1, 2, 3, 4, 5, 6, 7}, s, [&](int id, int shape) {
             FrameArgs a = fa;
             a.g.plan_m.fixed = id;
             a.g.plan_m.shape = shape;
@@ -2232,8 +2238,8 @@ void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
             launch_frame_inverse(a, s);
         });
     }
-    if (fa.g.fam_py == kE25) {
-        tune_length(c, fa.g.Py, {0, 2}, s, [&](int id, int shape) {  // shape 2: no look-ahead prefetch
+    if (fa.n_drv == 1 && fa.n_out == 3) {
+        tune_length(c, fa.g.Py, kFxCols, {0, 2}, s, [&](int id, int shape) {  // shape 2: no look-ahead prefetch
             FrameArgs a = fa;
             a.g.plan_py.fixed = id;
             a.g.plan_py.shape = shape;
@@ -2485,14 +2491,15 @@ int ld_set_autotune(ld_ctx* c, int enable) {
 int ld_autotune_choice(ld_ctx* c, int32_t n, int32_t* radices_out, int32_t* shape_out, double* ms_out) {
     if (!c || !radices_out) return 0;
     std::lock_guard<std::mutex> lock(c->mu);
-    auto it = c->fixed_choice.find(n);
+    auto it = c->fixed_choice.find({n, kFxRows});
+    if (it == c->fixed_choice.end()) it = c->fixed_choice.find({n, kFxCols});
     if (it == c->fixed_choice.end()) return 0;
     const FxPlanDesc* d = fx_plan(it->second & 255);
     if (d == nullptr) return 0;
     for (int i = 0; i < d->count; ++i) radices_out[i] = d->radix[i];
     if (shape_out) *shape_out = it->second >> 8;
     if (ms_out) {
-        auto m = c->fixed_ms.find(n);
+        auto m = c->fixed_ms.find(it->first);
         *ms_out = m != c->fixed_ms.end() ? m->second : 0.0;
     }
     return d->count;
@@ -2687,8 +2694,9 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         const ZoneTiles zt = zones && p.fft_form != LD_FFT_CUFFT ? zone_tiles(Ww, Hw, zn) : ZoneTiles{};
         const bool tiled = zt.n > 0 && static_cast<double>(zt.wo + Kmax - 1) * (zt.ho + Kmax - 1) <=
                                            0.5 * static_cast<double>(Ww + Kmax - 1) * (Hw + Kmax - 1);
-        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, &rw, &rh)
-                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, &rw, &rh);
+        const bool fx_cols = fx_cols_chain(cb, p);
+        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx_cols, &rw, &rh)
+                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx_cols, &rw, &rh);
         // Spectra already cached (a warm frame)?  If not, the bank and kernel
         // spectra are built on s while the source's row transforms run on a
         // side stream: they do not depend on the lens.  (Tiles transform
@@ -2768,7 +2776,7 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         if (post.scatter) {
             const int Ks = 2 * std::max(1, static_cast<int>(std::ceil(std::max(0.5f, post.scatter_radius)))) + 1;
             int srw = 0, srh = 0;
-            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, &srw, &srh);
+            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, false, &srw, &srh);
         }
         // rows of the row spectra: the frame's, or a tile's input rows
         const int Hp = tiled ? ((zt.ho + Kmax - 1 + 3) & ~3) : ((Hw + 3) & ~3);
