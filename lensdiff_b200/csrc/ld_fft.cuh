@@ -49,12 +49,9 @@ struct FftPlan {
     unsigned long long codes;  // stage count of kPlanRadices[i] at bits 4i..4i+3
     const float2* tw;          // n entries, exp(-2 pi i k / n)
     // Compile-time plan (ld_fxplans.h) the launchers use for this length, 0
-    // for none, and its per-stage twiddle tables (ld_fftx.cuh)
+    // for none, and its per-stage twiddle tables (ld_fxpass.cuh)
     int fixed;
     const float2* stw;
-    // launch shape of the fixed plan's kernels (0: default; 1: one more CTA
-    // per SM for the inverse row pass, under a tighter register cap)
-    int shape;
 };
 
 __host__ __device__ inline int plan_count(const FftPlan& p, int i) {

@@ -296,7 +296,6 @@ void configure_kernels() {
     configure_dft_kernels();
     configure_e<kE25>();
     configure_e<kE16>();
-    fx_configure();
 }
 
 }  // namespace ld

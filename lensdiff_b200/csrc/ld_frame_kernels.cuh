@@ -1,10 +1,7 @@
 // ld_frame_kernels.cuh — device kernels of the per-frame FFT convolution chain
-// and of the kernel-spectrum build, shared by ld_frame.cu (runtime-planned
-// transforms) and ld_frame_fx.cu (compile-time transforms of the fixed plans).
-// Every FFT kernel takes its transform as the policy class FFT (ld_fftx.cuh):
-// GenericFft<E> plays the plan the host built at run time, FixedFft<N, R...> a
-// length and radix order fixed at compile time.
-//
+// and of the kernel-spectrum build on runtime-planned transforms, and the
+// device functions that the compiled plans' kernels (ld_fx_rows.cuh,
+// ld_fx_cols.cuh) share with them.
 //
 // Reference stages (LensDiffCpuReference.cpp):
 //   buildSelectionMask / applyMask / applyMaskScalarDriver :1219-1279
@@ -35,7 +32,7 @@
 #include <cuda_fp16.h>
 
 #include "ld_async.cuh"
-#include "ld_fftx.cuh"
+#include "ld_fft.cuh"
 #include "ld_internal.h"
 #include "ld_pixel.cuh"
 
@@ -198,95 +195,96 @@ __device__ __forceinline__ void store_bins_h16(int M, int C, int Hp, int y0, con
 // spare bin per sequence for the in-place bins of store_bins_h16).
 constexpr size_t rows_smem(int M, int C) { return (static_cast<size_t>(M) + 1) * C * sizeof(float2); }
 
-// Spectral (NDRV = 1): C = 4 frame rows per CTA, the scalar driver of each.
-// Mono (NDRV = 3): C = 3, one frame row per CTA, its three colour drivers.
-// Column col of the transform is row y0 + col / NDRV, driver col % NDRV; its
-// spectrum goes to A[k][y0 + col / NDRV][col % NDRV].
-// FROM_EFFECT (scatter, NDRV = 3): the drivers are the stored effect's RGB.
-template <int E, int C, int NDRV, int MAXT = Fam<E>::max_threads, int MINB = 1, bool FROM_EFFECT = false,
-          class FFT = GenericFft<E>>
-__global__ void __launch_bounds__(MAXT, MINB) frame_rows_kernel(FrameArgs a) {
-    extern __shared__ float2 smem[];
+// The drivers of a forward row pass's CTA into smem[idx * C + col]: spectral
+// (NDRV = 1): C frame rows, the scalar driver of each; Mono (NDRV = 3): C = 3,
+// one frame row, its three colour drivers.  Column col is row y0 + col / NDRV,
+// driver col % NDRV; a complex value is a pair of pixels.  FROM_EFFECT
+// (scatter, NDRV = 3): the drivers are the stored effect's RGB.
+template <int C, int NDRV, bool FROM_EFFECT>
+__device__ __forceinline__ void fill_rows(const FrameArgs& a, int y0, int M, float2* smem) {
     constexpr int RPC = C / NDRV;  // frame rows per CTA
-    const int y0 = blockIdx.x * RPC;
     const int64_t pitch = a.src_pitch;
     const bool aligned = ((reinterpret_cast<uintptr_t>(a.src) | static_cast<uintptr_t>(pitch)) & 15) == 0;
-    const int W = a.W, H = a.H, M = a.g.M;
+    const int W = a.W, H = a.H;
     const int tx0 = a.tile_x0, ty0 = a.tile_y0;  // grid origin in frame pixels (tiles)
-    // the source rows of this CTA and of the CTA one resident generation
-    // later (their part under the grid) go to L2 through the bulk-copy
-    // engine while this CTA loads
-    // (bit 1 of the row plan's launch shape turns the later generation's
-    // prefetch off; the autotuner times both)
+    // this CTA's source rows (their part under the grid) go to L2 through the
+    // bulk-copy engine while it loads (the rows of a later CTA as well cost 5 %
+    // at UHD: they are evicted before their use)
     if (!FROM_EFFECT && aligned && threadIdx.x == 0) {
         const int px0 = max(0, tx0), px1 = min(W, tx0 + 2 * M);
         const uint32_t span = px1 > px0 ? static_cast<uint32_t>(px1 - px0) * 16u : 0u;
-        const int later = y0 + a.ahead * RPC;
-        const bool ahead = a.ahead > 0 && (a.g.plan_m.shape & 2) == 0;
         for (int r = 0; r < RPC && span > 0; ++r) {
-            const int fy = y0 + r + ty0, fl = later + r + ty0;
+            const int fy = y0 + r + ty0;
             if (fy >= 0 && fy < H) bulk_prefetch_l2(a.src + static_cast<int64_t>(fy) * pitch + px0 * 16, span);
-            if (ahead && fl >= 0 && fl < H) bulk_prefetch_l2(a.src + static_cast<int64_t>(fl) * pitch + px0 * 16, span);
         }
     }
     const SelectionParams sel = a.sel;
-    // one thread per (row, pixel pair): the selection mask is evaluated once
-    // per pixel and feeds every driver plane.  kU pairs per thread are loaded
-    // before any is used, so enough source reads are in flight to cover HBM
-    // latency at one CTA per SM.
-    constexpr int kU = 4;
-    const int T = blockDim.x;
-    for (int i0 = threadIdx.x; i0 < RPC * M; i0 += kU * T) {
-        float4 px[kU][2];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int i = i0 + u * T;
-            const int r = i / M;
-            const int idx = i - r * M;
-            const int y = y0 + r + ty0;   // frame row
-            const int x0 = 2 * idx + tx0;  // frame column of the pair's first pixel
-            const unsigned char* row = a.src + static_cast<int64_t>(y) * pitch;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const bool in = i < RPC * M && y >= 0 && y < H && x0 + h >= 0 && x0 + h < W;
-                if constexpr (FROM_EFFECT)
-                    px[u][h] = in ? a.effect[static_cast<int64_t>(y) * W + x0 + h] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                else
-                    px[u][h] = in ? decode_px(a.transfer, load_px(row, x0 + h, aligned)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+    // one thread per pixel pair: the selection mask is evaluated once per pixel
+    // and feeds every driver plane
+    auto put = [&](int r, int idx, float4 p0, float4 p1) {
+        float sig0, sig1;
+        // zero pixels (outside the frame or black) give a zero driver
+        const float m0 = FROM_EFFECT ? 1.0f : selection_mask(sel, p0.x, p0.y, p0.z, &sig0) * sel.rscale;
+        const float m1 = FROM_EFFECT ? 1.0f : selection_mask(sel, p1.x, p1.y, p1.z, &sig1) * sel.rscale;
+        float2* q = smem + idx * C + r * NDRV;
+        if constexpr (NDRV == 1) {
+            q[0] = make_float2(sig0 * m0, sig1 * m1);
+        } else {
+            q[0] = make_float2(p0.x * m0, p1.x * m1);
+            q[1] = make_float2(p0.y * m0, p1.y * m1);
+            q[2] = make_float2(p0.z * m0, p1.z * m1);
         }
+    };
+    const int T = blockDim.x;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // pairs [ia, ib) lie in the frame; the others are zero padding, up to a
+    // pair that the frame's edge cuts
+    const int ia = min(M, max(0, (1 - tx0) >> 1)), ib = max(ia, min(M, (W - tx0) >> 1));
+#pragma unroll 1
+    for (int r = 0; r < RPC; ++r) {
+        const int y = y0 + r + ty0;  // frame row
+        const bool row_in = y >= 0 && y < H;
+        const unsigned char* row = a.src + static_cast<int64_t>(y) * pitch;
+        const float4* erow = a.effect + static_cast<int64_t>(y) * W;
+        auto load = [&](int x) {
+            if constexpr (FROM_EFFECT) return erow[x];
+            else return decode_px(a.transfer, load_px(row, x, aligned));
+        };
+        for (int idx = threadIdx.x; idx < M; idx += T) {
+            if (row_in && idx >= ia && idx < ib) continue;
+            const int x = 2 * idx + tx0;
+            const bool in0 = row_in && x >= 0 && x < W, in1 = row_in && x + 1 >= 0 && x + 1 < W;
+            put(r, idx, in0 ? load(x) : none, in1 ? load(x + 1) : none);
+        }
+        if (!row_in) continue;
+        // kU pairs per thread are loaded before any is used, so enough source
+        // reads are in flight to cover HBM latency
+        constexpr int kU = 4;
+        for (int i0 = ia + threadIdx.x; i0 < ib; i0 += kU * T) {
+            float4 px[kU][2];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int i = i0 + u * T;
-            if (i >= RPC * M) break;
-            const int r = i / M;
-            const int idx = i - r * M;
-            float2 v[NDRV];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float4 p = px[u][h];
-                float sig;
-                // zero pixels (outside the frame or black) give a zero driver
-                const float m = FROM_EFFECT ? 1.0f : selection_mask(sel, p.x, p.y, p.z, &sig) * sel.rscale;
-                if (NDRV == 1) {
-                    const float dv = sig * m;
-                    if (h == 0) v[0].x = dv;
-                    else v[0].y = dv;
-                } else {
-                    const float c3[3] = {p.x * m, p.y * m, p.z * m};
-#pragma unroll
-                    for (int d = 0; d < NDRV; ++d) {
-                        if (h == 0) v[d].x = c3[d];
-                        else v[d].y = c3[d];
-                    }
-                }
+            for (int u = 0; u < kU; ++u) {
+                const int x = 2 * min(i0 + u * T, ib - 1) + tx0;
+                px[u][0] = load(x);
+                px[u][1] = load(x + 1);
             }
 #pragma unroll
-            for (int d = 0; d < NDRV; ++d) smem[idx * C + r * NDRV + d] = v[d];
+            for (int u = 0; u < kU; ++u)
+                if (i0 + u * T < ib) put(r, i0 + u * T, px[u][0], px[u][1]);
         }
     }
+}
+
+// C sequences of length M per CTA (fill_rows): the spectrum of column col goes
+// to A[k][y0 + col / NDRV][col % NDRV].
+template <int E, int C, int NDRV, int MAXT = Fam<E>::max_threads, int MINB = 1, bool FROM_EFFECT = false>
+__global__ void __launch_bounds__(MAXT, MINB) frame_rows_kernel(FrameArgs a) {
+    extern __shared__ float2 smem[];
+    const int y0 = blockIdx.x * (C / NDRV);
+    const int M = a.g.M;
+    fill_rows<C, NDRV, FROM_EFFECT>(a, y0, M, smem);
     __syncthreads();
-    FFT::template run<C, false, MAXT>(a.g.plan_m, smem);
+    fft_run<E, C, false>(a.g.plan_m, smem);
     if (NDRV == 1 && !FROM_EFFECT && a.h16)
         store_bins_h16(M, C, a.Hp, y0, a.g.tw_px, smem, reinterpret_cast<__half2*>(a.A), a.aexp);
     else
@@ -302,7 +300,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_rows_kernel(FrameArgs a) {
 // H16: the half2 row spectra land at the start of Wk and the rows' exponents
 // right after them (a third mbarrier), and are widened into F; the half2
 // kernel spectra land in the upper half of Wk and are widened in the multiply.
-template <int E, int NOUT, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false, class FFT = GenericFft<E>>
+template <int E, int NOUT, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
 __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     const int Py = a.g.Py, Hp = a.Hp, cols = a.g.cols;
@@ -331,8 +329,8 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
         bulk_load_checked(adst, asrc, a_bytes, &bars[0], smraw, a.err);
         if (H16) bulk_load_checked(aex, a.aexp, static_cast<uint32_t>((Hp + 15) & ~15), &bars[2], smraw, a.err);
         bulk_load_checked(kdst, ksrc, k_bytes, &bars[1], smraw, a.err);
-        const int later = k + a.ahead;  // bit 1 of the column plan's shape: no look-ahead (autotuned)
-        if (later < cols && (a.g.plan_py.shape & 2) == 0) {
+        const int later = k + a.ahead;
+        if (later < cols) {
             bulk_prefetch_l2(asrc + (later - k) * static_cast<size_t>(a_bytes), a_bytes);
             bulk_prefetch_l2(static_cast<const char*>(ksrc) + (later - k) * static_cast<size_t>(k_bytes), k_bytes);
         }
@@ -347,7 +345,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
         for (int i = Hp + threadIdx.x; i < Py; i += blockDim.x) F[i] = make_float2(0.0f, 0.0f);
         if (__syncthreads_or(!mbar_wait(&bars[0], 0, a.err))) return;
     }
-    FFT::template run<1, false, MAXT>(a.g.plan_py, F);
+    fft_run<E, 1, false>(a.g.plan_py, F);
     if (__syncthreads_or(!mbar_wait(&bars[1], 0, a.err))) return;
     if constexpr (H16) {
         // every thread widens its (at most E) kernel values before any
@@ -370,7 +368,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
         for (int i = threadIdx.x; i < Py * NOUT; i += blockDim.x) Wk[i] = cmul(Wk[i], F[i / NOUT]);
     }
     __syncthreads();
-    FFT::template run<NOUT, true, MAXT>(a.g.plan_py, Wk);
+    fft_run<E, NOUT, true>(a.g.plan_py, Wk);
     if constexpr (H16)
         store_b_column_h16(Wk, reinterpret_cast<__half2*>(a.Bout), a.bscale, k, Hp, NOUT);
     else
@@ -421,14 +419,11 @@ __global__ void __launch_bounds__(Fam<E>::max_threads, 1) frame_cols_mono_kernel
 // The spectral map of pixel sx of the inverse-transformed row in smem.
 template <int C>
 __device__ __forceinline__ float3 mapped_effect(const FrameArgs& a, const float2* smem, int sx) {
-    const int nn = sx >> 1;
-    const bool odd = sx & 1;
+    // pixel sx is component sx & 1 of the complex value sx >> 1
+    const float* p = reinterpret_cast<const float*>(smem) + (sx >> 1) * (2 * C) + (sx & 1);
     float e[C];
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-        const float2 z = smem[nn * C + c];
-        e[c] = odd ? z.y : z.x;
-    }
+    for (int c = 0; c < C; ++c) e[c] = p[2 * c];
     return map_effect<C>(a, e);
 }
 
@@ -446,78 +441,45 @@ __device__ __forceinline__ float zone_weight(int v, int extent, int z, int n) {
     return fmaxf(0.0f, 1.0f - fabsf(pv - static_cast<float>(z)));
 }
 
-// One row per CTA; smem M * C float2 (C = n_out interleaved channels).  The
-// row is output row out_y1 + blockIdx.x (kEffectComposite), source row
-// blockIdx.x (kEffectStore, kEffectScatter) or source row row0 + blockIdx.x
-// (kEffectAccumulate); see FrameArgs::effect_mode.
-template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false, class FFT = GenericFft<E>>
-__global__ void __launch_bounds__(MAXT, MINB) frame_inverse_kernel(FrameArgs a) {
-    extern __shared__ float2 smem[];
+// The row of an inverse-pass CTA: output row out_y1 + blockIdx.x
+// (kEffectComposite), source row blockIdx.x (kEffectStore, kEffectScatter) or
+// source row row0 + blockIdx.x (kEffectAccumulate); see FrameArgs::effect_mode.
+struct InverseRow {
+    int yo, sy;  // output row, working-frame row
+    int by;      // the grid row of frame row sy
+    bool have;   // sy lies in the frame and its row in B
+};
+__device__ __forceinline__ InverseRow inverse_row(const FrameArgs& a) {
     const int bid = static_cast<int>(blockIdx.x);
-    const int yo = a.effect_mode == kEffectComposite ? a.out_y1 + bid
-                                                     : a.src_y1 + (a.effect_mode == kEffectAccumulate ? a.row0 + bid : bid);
-    const int sy = yo - a.src_y1;
-    const int by = sy - a.tile_y0;  // the grid row of frame row sy
-    const bool have = sy >= 0 && sy < a.H && by >= 0 && by < a.Hp;
-    const int M = a.g.M;
-    // composite: this row's source pixels, and those of the row one resident
-    // generation later (unless bit 2 of the row plan's shape is set; the
-    // autotuner times both), go to L2 while the row's spectrum loads and
-    // transforms
+    InverseRow w;
+    w.yo = a.effect_mode == kEffectComposite ? a.out_y1 + bid
+                                             : a.src_y1 + (a.effect_mode == kEffectAccumulate ? a.row0 + bid : bid);
+    w.sy = w.yo - a.src_y1;
+    w.by = w.sy - a.tile_y0;
+    w.have = w.sy >= 0 && w.sy < a.H && w.by >= 0 && w.by < a.Hp;
+    return w;
+}
+
+// Composite: this row's source pixels, and those of the row one resident
+// generation later, go to L2 while the row's spectrum loads and transforms.
+__device__ __forceinline__ void inverse_prefetch(const FrameArgs& a, const InverseRow& w) {
     if (a.effect_mode == kEffectComposite && threadIdx.x == 0 &&
         ((reinterpret_cast<uintptr_t>(a.src) | static_cast<uintptr_t>(a.src_pitch)) & 15) == 0) {
         const uint32_t row_bytes = static_cast<uint32_t>(a.W) * 16u;
-        if (have) bulk_prefetch_l2(a.src + static_cast<int64_t>(sy) * a.src_pitch, row_bytes);
-        const int sl = sy + a.ahead;
-        if (a.ahead > 0 && (a.g.plan_m.shape & 4) == 0 && sl >= 0 && sl < a.H &&
-            bid + a.ahead < static_cast<int>(gridDim.x))
+        if (w.have) bulk_prefetch_l2(a.src + static_cast<int64_t>(w.sy) * a.src_pitch, row_bytes);
+        const int sl = w.sy + a.ahead;
+        if (a.ahead > 0 && sl >= 0 && sl < a.H &&
+            static_cast<int>(blockIdx.x) + a.ahead < static_cast<int>(gridDim.x))
             bulk_prefetch_l2(a.src + static_cast<int64_t>(sl) * a.src_pitch, row_bytes);
     }
-    if (have) {
-        const float2* tw_px = a.g.tw_px;
-        // Hermitian pairs: one load of X[p] and X[M-p] per channel gives both
-        // Z[p] and Z[M-p] (p = 0 pairs with the Nyquist bin M and gives Z[0]
-        // only; p = M/2 pairs with itself).  kU pairs per thread are loaded
-        // before any is used: the reads are scattered, one run per bin group.
-        const int Hp = a.Hp;
-        const int half = M / 2;
-        const int npair = (half + 1) * C;
-        constexpr int kU = 4;
-        const int T = blockDim.x;
-        for (int i0 = threadIdx.x; i0 < npair; i0 += kU * T) {
-            float2 xp[kU], xq[kU], wp[kU], wq[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int i = i0 + u * T;
-                if (i < npair) {
-                    const int pk = i / C;
-                    const int c = i - pk * C;
-                    if constexpr (H16) {
-                        const __half2* Bh = reinterpret_cast<const __half2*>(a.Bout);
-                        xp[u] = from_half2(__ldcs(&Bh[b_index(pk, by, c, Hp, C)]), __ldg(&a.bscale[pk]));
-                        xq[u] = from_half2(__ldcs(&Bh[b_index(M - pk, by, c, Hp, C)]), __ldg(&a.bscale[M - pk]));
-                    } else {
-                        xp[u] = __ldcs(&a.Bout[b_index(pk, by, c, Hp, C)]);
-                        xq[u] = __ldcs(&a.Bout[b_index(M - pk, by, c, Hp, C)]);
-                    }
-                    wp[u] = __ldg(&tw_px[pk]);
-                    wq[u] = __ldg(&tw_px[M - pk]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int i = i0 + u * T;
-                if (i < npair) {
-                    const int pk = i / C;
-                    const int c = i - pk * C;
-                    if (pk < M) smem[pk * C + c] = c2r_pre(xp[u], xq[u], wp[u]);
-                    if (pk > 0 && M - pk != pk && M - pk < M) smem[(M - pk) * C + c] = c2r_pre(xq[u], xp[u], wq[u]);
-                }
-            }
-        }
-        __syncthreads();
-        FFT::template run<C, true, MAXT>(a.g.plan_m, smem);
-    }
+}
+
+// What the inverse pass does with its transformed row (smem, C interleaved
+// channels of M float2); see FrameArgs::effect_mode.
+template <int C>
+__device__ __forceinline__ void inverse_epilogue(const FrameArgs& a, const InverseRow& w, const float2* smem) {
+    const int yo = w.yo, sy = w.sy;
+    const bool have = w.have;
     const bool aligned_s = ((reinterpret_cast<uintptr_t>(a.src) | static_cast<uintptr_t>(a.src_pitch)) & 15) == 0;
     const unsigned char* srow = a.src + static_cast<int64_t>(sy) * a.src_pitch;
     if (a.effect_mode == kEffectAccumulate) {
@@ -577,25 +539,99 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_inverse_kernel(FrameArgs a) 
     unsigned char* drow = a.dst + static_cast<int64_t>(yo - a.dst_y1) * a.dst_pitch;
     constexpr int kV = 4;  // source pixels loaded ahead of use, per thread
     const int T = blockDim.x;
-    for (int x0 = a.out_x1 + threadIdx.x; x0 < a.out_x2; x0 += kV * T) {
+    // [xa, xb): the output pixels over source pixels, the others are opaque black
+    const int xa = have ? min(max(a.out_x1, a.src_x1), a.out_x2) : a.out_x2;
+    const int xb = have ? max(xa, min(a.out_x2, a.src_x1 + a.W)) : xa;
+    const float4 black = encode_px(a.transfer, make_float4(0.0f, 0.0f, 0.0f, 1.0f));
+    for (int x = a.out_x1 + threadIdx.x; x < xa; x += T) store_px(drow, x - a.dst_x1, aligned_d, black);
+    for (int x = xb + threadIdx.x; x < a.out_x2; x += T) store_px(drow, x - a.dst_x1, aligned_d, black);
+    if (aligned_s && aligned_d && a.transfer == kTransferLinear) {
+        // the common row: no test per pixel but the tail's
+        const float4* sp = reinterpret_cast<const float4*>(srow) - a.src_x1;
+        float4* dp = reinterpret_cast<float4*>(drow) - a.dst_x1;
+        int x0 = xa + threadIdx.x;
+        for (; x0 + (kV - 1) * T < xb; x0 += kV * T) {
+            float4 px[kV];
+#pragma unroll
+            for (int u = 0; u < kV; ++u) px[u] = __ldg(sp + x0 + u * T);
+#pragma unroll
+            for (int u = 0; u < kV; ++u)
+                dp[x0 + u * T] = composite_px(a, px[u], mapped_effect<C>(a, smem, x0 + u * T - a.src_x1));
+        }
+        for (; x0 < xb; x0 += T) dp[x0] = composite_px(a, __ldg(sp + x0), mapped_effect<C>(a, smem, x0 - a.src_x1));
+        return;
+    }
+    for (int x0 = xa + threadIdx.x; x0 < xb; x0 += kV * T) {
         float4 px[kV];
 #pragma unroll
-        for (int u = 0; u < kV; ++u) {
-            const int sx = x0 + u * T - a.src_x1;
-            px[u] = (have && x0 + u * T < a.out_x2 && sx >= 0 && sx < a.W)
-                        ? decode_px(a.transfer, load_px(srow, sx, aligned_s))
-                                                                           : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-        }
+        for (int u = 0; u < kV; ++u)
+            px[u] = x0 + u * T < xb ? decode_px(a.transfer, load_px(srow, x0 + u * T - a.src_x1, aligned_s))
+                                    : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
 #pragma unroll
         for (int u = 0; u < kV; ++u) {
             const int x = x0 + u * T;
-            if (x >= a.out_x2) break;
-            const int sx = x - a.src_x1;
-            float4 out = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-            if (have && sx >= 0 && sx < a.W) out = composite_px(a, px[u], mapped_effect<C>(a, smem, sx));
+            if (x >= xb) break;
+            const float4 out = composite_px(a, px[u], mapped_effect<C>(a, smem, x - a.src_x1));
             store_px(drow, x - a.dst_x1, aligned_d, encode_px(a.transfer, out));
         }
     }
+}
+
+// One row per CTA (inverse_row); smem M * C float2 (C = n_out interleaved channels).
+template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
+__global__ void __launch_bounds__(MAXT, MINB) frame_inverse_kernel(FrameArgs a) {
+    extern __shared__ float2 smem[];
+    const InverseRow w = inverse_row(a);
+    const bool have = w.have;
+    const int by = w.by;
+    const int M = a.g.M;
+    inverse_prefetch(a, w);
+    if (have) {
+        const float2* tw_px = a.g.tw_px;
+        // Hermitian pairs: one load of X[p] and X[M-p] per channel gives both
+        // Z[p] and Z[M-p] (p = 0 pairs with the Nyquist bin M and gives Z[0]
+        // only; p = M/2 pairs with itself).  kU pairs per thread are loaded
+        // before any is used: the reads are scattered, one run per bin group.
+        const int Hp = a.Hp;
+        const int half = M / 2;
+        const int npair = (half + 1) * C;
+        constexpr int kU = 4;
+        const int T = blockDim.x;
+        for (int i0 = threadIdx.x; i0 < npair; i0 += kU * T) {
+            float2 xp[kU], xq[kU], wp[kU], wq[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int i = i0 + u * T;
+                if (i < npair) {
+                    const int pk = i / C;
+                    const int c = i - pk * C;
+                    if constexpr (H16) {
+                        const __half2* Bh = reinterpret_cast<const __half2*>(a.Bout);
+                        xp[u] = from_half2(__ldcs(&Bh[b_index(pk, by, c, Hp, C)]), __ldg(&a.bscale[pk]));
+                        xq[u] = from_half2(__ldcs(&Bh[b_index(M - pk, by, c, Hp, C)]), __ldg(&a.bscale[M - pk]));
+                    } else {
+                        xp[u] = __ldcs(&a.Bout[b_index(pk, by, c, Hp, C)]);
+                        xq[u] = __ldcs(&a.Bout[b_index(M - pk, by, c, Hp, C)]);
+                    }
+                    wp[u] = __ldg(&tw_px[pk]);
+                    wq[u] = __ldg(&tw_px[M - pk]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int i = i0 + u * T;
+                if (i < npair) {
+                    const int pk = i / C;
+                    const int c = i - pk * C;
+                    if (pk < M) smem[pk * C + c] = c2r_pre(xp[u], xq[u], wp[u]);
+                    if (pk > 0 && M - pk != pk && M - pk < M) smem[(M - pk) * C + c] = c2r_pre(xq[u], xp[u], wq[u]);
+                }
+            }
+        }
+        __syncthreads();
+        fft_run<E, C, true>(a.g.plan_m, smem);
+    }
+    inverse_epilogue<C>(a, w, smem);
 }
 
 // Luma sums of the redistributed source and of the stored effect over the
@@ -850,7 +886,7 @@ __device__ __forceinline__ int canvas_index(int g, int P, int R) {
 
 // One canvas row i = blockIdx.x of all C kernels per CTA (rows >= K are zero):
 // KR[k][i][c], k < M + 1.
-template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, class FFT = GenericFft<E>>
+template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1>
 __global__ void __launch_bounds__(MAXT, MINB) kspec_rows_kernel(KernelSpectraArgs a) {
     extern __shared__ float2 smem[];
     const int i = blockIdx.x;
@@ -864,7 +900,7 @@ __global__ void __launch_bounds__(MAXT, MINB) kspec_rows_kernel(KernelSpectraArg
         const int j1 = canvas_index(2 * idx + 1, Px, R);
         return make_float2(j0 >= 0 ? p[j0] : 0.0f, j1 >= 0 ? p[j1] : 0.0f);
     });
-    FFT::template run<C, false, MAXT>(a.g.plan_m, smem);
+    fft_run<E, C, false>(a.g.plan_m, smem);
     store_bins(a.g.M, C, static_cast<int64_t>(a.Kp) * C, static_cast<int64_t>(i) * C, a.g.tw_px, smem, a.rows);
 }
 
@@ -872,7 +908,7 @@ __global__ void __launch_bounds__(MAXT, MINB) kspec_rows_kernel(KernelSpectraArg
 // copy; the wrap map places canvas row ci at grid row v and folds in the
 // inverse scale; the transformed column KS[k] (Py x C, contiguous) leaves by
 // one bulk store.
-template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false, class FFT = GenericFft<E>>
+template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
 __global__ void __launch_bounds__(MAXT, MINB) kspec_cols_kernel(KernelSpectraArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     const int Py = a.g.Py, cols = a.g.cols, Kp = a.Kp, R = a.R;
@@ -901,7 +937,7 @@ __global__ void __launch_bounds__(MAXT, MINB) kspec_cols_kernel(KernelSpectraArg
         W[i] = ci >= 0 ? cscale(Rb[ci * C + c], sc) : make_float2(0.0f, 0.0f);
     }
     __syncthreads();
-    FFT::template run<C, false, MAXT>(a.g.plan_py, W);
+    fft_run<E, C, false>(a.g.plan_py, W);
     if constexpr (H16) {
         const float m = block_absmax(W, Py * C);
         const float sc = m > 0.0f ? kHalfTop / m : 1.0f;

@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
         if (H16)
             bulk_load_checked(aex, a.aexp, static_cast<uint32_t>((Hp + 15) & ~15), &h->bar[2], smraw, a.err);
         bulk_load_checked(H16 ? static_cast<void*>(kh) : static_cast<void*>(W), ksrc, k_bytes, &h->bar[1], smraw, a.err);
-        const int later = k + a.ahead;  // bit 1 of the column plan's shape: no look-ahead (autotuned)
-        if (later < cols && (a.g.plan_py.shape & 2) == 0) {
+        const int later = k + a.ahead;
+        if (later < cols) {
             bulk_prefetch_l2(asrc + static_cast<size_t>(later - k) * a_bytes, a_bytes);
             bulk_prefetch_l2(ksrc + static_cast<size_t>(later - k) * k_bytes, k_bytes);
         }

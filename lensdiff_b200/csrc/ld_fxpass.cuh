@@ -1,8 +1,14 @@
-// ld_fxpass.cuh — the compile-time Stockham stages of ld_fftx.cuh with the first
-// stage fed from, and the last stage drained to, wherever the pass keeps its
+// ld_fxpass.cuh — Stockham stages of compile-time length and radix order, the
+// first stage fed from, and the last drained to, wherever the pass keeps its
 // data: global memory, staged bulk copies, a spectral product, a converted
 // store.  A pass of three stages then moves each value through shared memory
-// twice instead of five times (fill, three in-place stages, drain).
+// twice instead of five times (fill, three in-place stages, drain).  The
+// length, the radix and span of every stage and the thread count are
+// constants, so a butterfly's addresses are one base plus immediate offsets
+// and its divisions are by constants; the twiddles w^r of butterfly k come from
+// a per-stage table of pairs (w^2q, w^(2q+1)) laid out [q][k], read as 16-byte
+// loads that a warp's threads (consecutive k) make to consecutive addresses
+// (fx_stage_table in ld_frame_fx.cu).
 //
 // A stage of radix R over span NS takes butterfly b = j * C + c (j < N / R,
 // sequence c of C interleaved ones): its inputs are the elements
@@ -16,10 +22,15 @@
 #include <atomic>
 
 #include "ld_async.cuh"
-#include "ld_fftx.cuh"
+#include "ld_fft.cuh"
 #include "ld_internal.h"
 
 namespace ld {
+
+template <int R>
+struct FxPad {  // a stage table holds an even number of twiddles per span offset
+    static constexpr int value = (R + 1) & ~1;
+};
 
 // ---- small DFTs of the composite radices --------------------------------------
 // cos and sin of 2 pi m / R to double precision at compile time: the argument
@@ -252,8 +263,10 @@ struct KernelState {
         const int known = dev < 16 ? resident[dev].load(std::memory_order_relaxed) : 0;
         if (known > 0) return known;
         int sms = 148, per = 1;
+        cudaFuncAttributes fa{};
+        cudaFuncGetAttributes(&fa, kernel);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kSmemOptIn));
+                             static_cast<int>(kSmemOptIn - fa.sharedSizeBytes));
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess || per < 1) per = 1;
         if (dev < 16) resident[dev].store(sms * per, std::memory_order_relaxed);

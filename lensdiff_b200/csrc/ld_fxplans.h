@@ -2,13 +2,15 @@
 // plans, shared by the host (planning, twiddle tables, the autotuner's
 // candidate lists) and the kernels' translation units.
 //
-// Row plans (length M, half the grid's width) run on ld_fftx.cuh
-// (ld_frame_fx.cu), column plans (length Py) on ld_fxpass.cuh (ld_fx_cols*.cu):
-// every length from 300 to 5400 that the grid's cost model (choose_length in
-// ld_host.cu) picks for three column sequences has one.  Where a length has
-// several orders the autotuner times them on first use and keeps the fastest
-// (the first is the default).  Odd radices lead where the length has them:
-// their strided first-stage stores spread over the shared-memory banks.
+// Row plans (length M, half the grid's width: ld_fx_rows*.cu) and column plans
+// (length Py: ld_fx_cols*.cu) run on ld_fxpass.cuh.  Every length that the
+// grid's cost model (choose_length in ld_host.cu) picks for the spectral
+// chains has one: columns from 300 to 5400, rows from 256 to 4096.  Where a
+// length has several orders the autotuner times them on first use and keeps
+// the fastest (the first is the default).  Odd radices lead where the length
+// has them: their strided first-stage stores spread over the shared-memory
+// banks.  A row plan's last radix is also its inverse's first, and is taken in
+// pairs of mirrored butterflies: a small one.
 #pragma once
 
 namespace ld {
@@ -16,11 +18,10 @@ namespace ld {
 enum { kFxRows = 1, kFxCols = 2 };
 
 struct FxPlanDesc {
-    int id;         // 0 means "no fixed plan"
+    int id;         // 1 .. 255 (0 means "no fixed plan")
     int role;       // kFxRows, kFxCols
-    int count;      // stages
     int radix[3];   // radix of each stage, first stage first
-    constexpr int n() const { return radix[0] * radix[1] * (count > 2 ? radix[2] : 1); }
+    constexpr int n() const { return radix[0] * radix[1] * radix[2]; }
 };
 
 // Column plans X(id, R1, R2, R3), in the groups that the translation units
@@ -43,18 +44,36 @@ struct FxPlanDesc {
 #define LD_FX_COLS_5(X) \
     X(25, 5, 8, 12) X(31, 9, 8, 9) X(37, 15, 8, 8) X(43, 5, 16, 16) X(49, 9, 12, 16) \
     X(55, 9, 16, 16) X(61, 25, 16, 8) X(67, 15, 12, 24)
-#define LD_FX_COL_DESC(ID, A, B, C) {ID, kFxCols, 3, {A, B, C}},
+// Row plans X(id, R1, R2, R3), in the groups of ld_fx_rows0.cu .. ld_fx_rows5.cu.
+#define LD_FX_ROWS_0(X) \
+    X(100, 8, 8, 4) X(106, 5, 10, 9) X(112, 5, 16, 8) X(118, 9, 10, 10) X(124, 25, 10, 5) \
+    X(130, 25, 8, 8) X(136, 15, 16, 9) X(142, 25, 12, 10) X(148, 16, 16, 16)
+#define LD_FX_ROWS_1(X) \
+    X(101, 5, 12, 5) X(107, 5, 10, 10) X(113, 15, 9, 5) X(119, 15, 8, 8) X(125, 10, 16, 8) \
+    X(131, 9, 16, 12) X(137, 12, 16, 12) X(143, 25, 25, 5)
+#define LD_FX_ROWS_2(X) \
+    X(102, 5, 8, 8) X(108, 8, 8, 8) X(114, 9, 10, 8) X(120, 25, 5, 8) X(126, 9, 16, 9) \
+    X(132, 15, 12, 10) X(138, 25, 10, 10) X(144, 25, 16, 8)
+#define LD_FX_ROWS_3(X) \
+    X(103, 5, 15, 5) X(109, 9, 8, 8) X(115, 12, 8, 8) X(121, 16, 8, 8) X(127, 15, 9, 10) \
+    X(133, 25, 15, 5) X(139, 20, 16, 8) X(145, 24, 16, 9)
+#define LD_FX_ROWS_4(X) \
+    X(104, 5, 10, 8) X(110, 5, 12, 10) X(116, 5, 16, 10) X(122, 15, 15, 5) X(128, 15, 12, 8) \
+    X(134, 25, 10, 8) X(140, 15, 15, 12) X(146, 25, 16, 9)
+#define LD_FX_ROWS_5(X) \
+    X(105, 9, 12, 4) X(111, 5, 25, 5) X(117, 9, 12, 8) X(123, 15, 10, 8) X(129, 15, 10, 10) \
+    X(135, 16, 16, 8) X(141, 15, 16, 12) X(147, 20, 16, 12)
+
+#define LD_FX_COL_DESC(ID, A, B, C) {ID, kFxCols, {A, B, C}},
+#define LD_FX_ROW_DESC(ID, A, B, C) {ID, kFxRows, {A, B, C}},
 constexpr FxPlanDesc kFxPlans[] = {
-    {1, kFxRows, 3, {25, 25, 4}},
-    {2, kFxRows, 3, {25, 4, 25}},
-    {5, kFxRows, 3, {25, 25, 2}},
-    {6, kFxRows, 3, {25, 2, 25}},
-    {9, kFxRows, 3, {5, 16, 16}},
-    {10, kFxRows, 3, {16, 5, 16}},
     LD_FX_COLS_0(LD_FX_COL_DESC) LD_FX_COLS_1(LD_FX_COL_DESC) LD_FX_COLS_2(LD_FX_COL_DESC)
     LD_FX_COLS_3(LD_FX_COL_DESC) LD_FX_COLS_4(LD_FX_COL_DESC) LD_FX_COLS_5(LD_FX_COL_DESC)
+    LD_FX_ROWS_0(LD_FX_ROW_DESC) LD_FX_ROWS_1(LD_FX_ROW_DESC) LD_FX_ROWS_2(LD_FX_ROW_DESC)
+    LD_FX_ROWS_3(LD_FX_ROW_DESC) LD_FX_ROWS_4(LD_FX_ROW_DESC) LD_FX_ROWS_5(LD_FX_ROW_DESC)
 };
 #undef LD_FX_COL_DESC
+#undef LD_FX_ROW_DESC
 
 inline const FxPlanDesc* fx_plan(int id) {
     for (const FxPlanDesc& d : kFxPlans)

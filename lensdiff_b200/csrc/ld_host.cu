@@ -90,7 +90,7 @@ struct ld_ctx {
     std::mutex mu;
     std::map<int, DevBuf> twiddles;
     std::map<int, DevBuf> stage_twiddles;  // by fixed plan id
-    // (transform length, role) -> fixed plan id | shape << 8 and the winner's timed ms (autotuner)
+    // (transform length, role) -> fixed plan id and the winner's timed ms (autotuner)
     std::map<std::pair<int, int>, int> fixed_choice;
     std::map<std::pair<int, int>, double> fixed_ms;
     int autotune = 1;  // 1: tune, 0: first compiled order, -1: runtime-planned transforms only
@@ -501,9 +501,7 @@ FftPlan make_plan(ld_ctx* c, int n, bool allow25, int role = 0) {
     FftPlan p{};
     if (!factor_plan(n, allow25, &p)) throw Fail{LD_ERR_UNSUPPORTED, "fft-length-not-5-smooth"};
     p.tw = twiddles(c, n);
-    const int choice = fixed_plan_for(c, n, role);
-    p.fixed = choice & 255;
-    p.shape = choice >> 8;
+    p.fixed = fixed_plan_for(c, n, role);
     p.stw = p.fixed ? stage_twiddles(c, p.fixed) : nullptr;
     return p;
 }
@@ -1545,9 +1543,9 @@ int choose_length(int n, int mult, int C) {
     return best;
 }
 
-// Whether the compiled column plans serve a chain: one driver and three
+// Whether the compiled plans serve a chain: one driver and three
 // kernels and outputs (the spectral modes without the luma lock).
-bool fx_cols_chain(const Combination& cb, const ld_params& p) {
+bool fx_chain(const Combination& cb, const ld_params& p) {
     return cb.n_drv == 1 && cb.n_ker == 3 && cb.n_out == 3 && p.fft_form != LD_FFT_CUFFT;
 }
 
@@ -1556,9 +1554,9 @@ bool fx_cols_chain(const Combination& cb, const ld_params& p) {
 // powers of two (LensDiffCpuReference.cpp:1172-1173); any grid of at least
 // W+K-1 x H+K-1 gives the same linear convolution.  c_rows / c_cols: the
 // most interleaved sequences any row / column kernel of the chain transforms
-// (they pick the FFT family); fx_cols: the compiled column plans serve the
-// chain (fx_cols_chain).
-GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, bool fx_cols, int* req_w, int* req_h) {
+// (they pick the FFT family); fx: the compiled plans serve the chain
+// (fx_chain).
+GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, bool fx, int* req_w, int* req_h) {
     GridGeom g{};
     *req_w = W + K - 1;
     *req_h = H + K - 1;
@@ -1572,8 +1570,8 @@ GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, b
     const int Kp = K + (K & 1);
     if (frame_cols_smem(g.Py, c_cols) > kSmemBudget || kspec_cols_smem(g.Py, Kp, c_cols) > kSmemBudget)
         throw Fail{LD_ERR_UNSUPPORTED, "frame-too-large-for-column-pass"};
-    g.plan_m = make_plan(c, g.M, g.fam_m == kE25, g.fam_m == kE25 ? kFxRows : 0);
-    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25, fx_cols ? kFxCols : 0);
+    g.plan_m = make_plan(c, g.M, g.fam_m == kE25, fx ? kFxRows : 0);
+    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25, fx ? kFxCols : 0);
     g.tw_px = twiddles(c, g.Px);
     return g;
 }
@@ -1988,7 +1986,7 @@ SpectraGeometry spectra_geometry(ld_ctx* c, const ld_params& p, int W, int H) {
     const int c_rows = std::max(std::max(sg.cb.n_drv == 1 ? 4 : 3, sg.cb.n_out), sg.cb.n_ker);
     const int c_cols = std::max(std::max(sg.cb.n_out, sg.cb.n_ker), sg.cb.n_drv);
     int rw = 0, rh = 0;
-    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_cols_chain(sg.cb, p), &rw, &rh);
+    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_chain(sg.cb, p), &rw, &rh);
     sg.key = spectra_key_for(bank_key(p, wl), sg.cb, sg.g);
     const bool h16 = chosen_h16(p);
     sg.bytes = sg.cb.parts * (ks_part_bytes(sg.cb.n_ker, sg.g, h16) + static_cast<size_t>(sg.g.cols) * sizeof(float));
@@ -2171,37 +2169,32 @@ constexpr size_t kGraphSeen = 4;  // covers the three spectra slots that a strea
 // ---------------------------------------------------------------------------
 // Autotuner of the fixed transform plans (ld_fxplans.h)
 // ---------------------------------------------------------------------------
-// Times launch(id, shape) for every compiled radix order of length n and
-// every launch shape in [0, shapes) on stream s (one untimed launch, then
-// kTuneReps between two events) and records the fastest as
-// c->fixed_choice[{n, role}] = id | shape << 8.
-void tune_length(ld_ctx* c, int n, int role, const std::vector<int>& shapes, cudaStream_t s,
-                 const std::function<void(int, int)>& launch) {
+// Times launch(id) for every compiled radix order of length n on stream s (one
+// untimed launch, then kTuneReps between two events; a single order one timed
+// launch) and records the fastest as c->fixed_choice[{n, role}].
+void tune_length(ld_ctx* c, int n, int role, cudaStream_t s, const std::function<void(int)>& launch) {
     int ids[8];
     const int k = fx_candidates(n, role, ids, 8);
     if (k == 0 || c->fixed_choice.count({n, role})) return;
     constexpr int kTuneReps = 3;
+    const int reps = k > 1 ? kTuneReps : 1;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     check_cuda(cudaEventCreate(&e0), "tune-event");
     check_cuda(cudaEventCreate(&e1), "tune-event");
     int best = ids[0];
     float best_ms = 0.0f;
-    bool first = true;
     for (int i = 0; i < k; ++i) {
-        for (const int sh : shapes) {
-            launch(ids[i], sh);
-            check_cuda(cudaEventRecord(e0, s), "tune-record");
-            for (int r = 0; r < kTuneReps; ++r) launch(ids[i], sh);
-            check_cuda(cudaEventRecord(e1, s), "tune-record");
-            check_cuda(cudaEventSynchronize(e1), "tune-sync");
-            float ms = 0.0f;
-            check_cuda(cudaEventElapsedTime(&ms, e0, e1), "tune-elapsed");
-            ms /= kTuneReps;
-            if (first || ms < best_ms) {
-                best = ids[i] | (sh << 8);
-                best_ms = ms;
-                first = false;
-            }
+        if (k > 1) launch(ids[i]);
+        check_cuda(cudaEventRecord(e0, s), "tune-record");
+        for (int r = 0; r < reps; ++r) launch(ids[i]);
+        check_cuda(cudaEventRecord(e1, s), "tune-record");
+        check_cuda(cudaEventSynchronize(e1), "tune-sync");
+        float ms = 0.0f;
+        check_cuda(cudaEventElapsedTime(&ms, e0, e1), "tune-elapsed");
+        ms /= static_cast<float>(reps);
+        if (i == 0 || ms < best_ms) {
+            best = ids[i];
+            best_ms = ms;
         }
     }
     cudaEventDestroy(e0);
@@ -2211,42 +2204,30 @@ void tune_length(ld_ctx* c, int n, int role, const std::vector<int>& shapes, cud
     c->fixed_ms[{n, role}] = best_ms;
 }
 
-// Tunes the row length (frame_rows + frame_inverse, which share its plan; eight
-// launch shapes: the inverse pass at two CTAs-per-SM caps, the row pass and
-// the inverse pass each with and without the L2 prefetch of the rows one
-// resident generation later) and the column length (frame_cols, with and
-// without its look-ahead prefetch) of a
-// composite frame's grid, re-running the frame's own launches: each rewrites
-// the results it wrote before.
+// Tunes the row length (frame_rows + frame_inverse, which share its plan) and
+// the column length (frame_cols) of a composite frame's grid, re-running the
+// frame's own launches: each rewrites the results it wrote before.
 void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
-    if (c->autotune != 1 || fa.effect_mode != kEffectComposite) return;
+    if (c->autotune != 1 || fa.effect_mode != kEffectComposite || fa.n_drv != 1 || fa.n_out != 3) return;
     if (c->fixed_choice.count({fa.g.M, kFxRows}) && c->fixed_choice.count({fa.g.Py, kFxCols})) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return;
     }
-    if (fa.g.fam_m == kE25) {
-        // shape bits: inverse at one more CTA per SM; row pass, inverse pass
-        // without their look-ahead prefetch
-        tune_length(c, fa.g.M, kFxRows, {0, 1, 2, 3, 4, 5, 6, 7}, s, [&](int id, int shape) {
-            FrameArgs a = fa;
-            a.g.plan_m.fixed = id;
-            a.g.plan_m.shape = shape;
-            a.g.plan_m.stw = stage_twiddles(c, id);
-            launch_frame_rows(a, s);
-            launch_frame_inverse(a, s);
-        });
-    }
-    if (fa.n_drv == 1 && fa.n_out == 3) {
-        tune_length(c, fa.g.Py, kFxCols, {0, 2}, s, [&](int id, int shape) {  // shape 2: no look-ahead prefetch
-            FrameArgs a = fa;
-            a.g.plan_py.fixed = id;
-            a.g.plan_py.shape = shape;
-            a.g.plan_py.stw = stage_twiddles(c, id);
-            launch_frame_cols(a, s);
-        });
-    }
+    tune_length(c, fa.g.M, kFxRows, s, [&](int id) {
+        FrameArgs a = fa;
+        a.g.plan_m.fixed = id;
+        a.g.plan_m.stw = stage_twiddles(c, id);
+        launch_frame_rows(a, s);
+        launch_frame_inverse(a, s);
+    });
+    tune_length(c, fa.g.Py, kFxCols, s, [&](int id) {
+        FrameArgs a = fa;
+        a.g.plan_py.fixed = id;
+        a.g.plan_py.stw = stage_twiddles(c, id);
+        launch_frame_cols(a, s);
+    });
 }
 
 // Issues a frame chain through a cached CUDA graph: the first call with a
@@ -2494,15 +2475,15 @@ int ld_autotune_choice(ld_ctx* c, int32_t n, int32_t* radices_out, int32_t* shap
     auto it = c->fixed_choice.find({n, kFxRows});
     if (it == c->fixed_choice.end()) it = c->fixed_choice.find({n, kFxCols});
     if (it == c->fixed_choice.end()) return 0;
-    const FxPlanDesc* d = fx_plan(it->second & 255);
+    const FxPlanDesc* d = fx_plan(it->second);
     if (d == nullptr) return 0;
-    for (int i = 0; i < d->count; ++i) radices_out[i] = d->radix[i];
-    if (shape_out) *shape_out = it->second >> 8;
+    for (int i = 0; i < 3; ++i) radices_out[i] = d->radix[i];
+    if (shape_out) *shape_out = 0;
     if (ms_out) {
         auto m = c->fixed_ms.find(it->first);
         *ms_out = m != c->fixed_ms.end() ? m->second : 0.0;
     }
-    return d->count;
+    return 3;
 }
 
 size_t ld_estimate_device_bytes(const ld_params* params, int32_t width, int32_t height) {
@@ -2694,9 +2675,9 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         const ZoneTiles zt = zones && p.fft_form != LD_FFT_CUFFT ? zone_tiles(Ww, Hw, zn) : ZoneTiles{};
         const bool tiled = zt.n > 0 && static_cast<double>(zt.wo + Kmax - 1) * (zt.ho + Kmax - 1) <=
                                            0.5 * static_cast<double>(Ww + Kmax - 1) * (Hw + Kmax - 1);
-        const bool fx_cols = fx_cols_chain(cb, p);
-        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx_cols, &rw, &rh)
-                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx_cols, &rw, &rh);
+        const bool fx = fx_chain(cb, p);
+        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx, &rw, &rh)
+                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx, &rw, &rh);
         // Spectra already cached (a warm frame)?  If not, the bank and kernel
         // spectra are built on s while the source's row transforms run on a
         // side stream: they do not depend on the lens.  (Tiles transform

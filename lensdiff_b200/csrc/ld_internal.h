@@ -161,7 +161,6 @@ bool fx_launch_frame_cols(const FrameArgs& a, cudaStream_t s);
 bool fx_launch_frame_inverse(const FrameArgs& a, int rows, cudaStream_t s);
 bool fx_launch_kspec_rows(const KernelSpectraArgs& a, cudaStream_t s);
 bool fx_launch_kspec_cols(const KernelSpectraArgs& a, cudaStream_t s);
-void fx_configure();
 // The column passes of the plans LD_FX_COLS_0 .. _5 (ld_fx_cols*.cu): the
 // frame's (fa) or the kernel spectra's (ka); false when `id` is not among
 // them or the pass does not fit.
@@ -171,6 +170,16 @@ bool fx_cols_2(int id, const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStr
 bool fx_cols_3(int id, const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s);
 bool fx_cols_4(int id, const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s);
 bool fx_cols_5(int id, const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s);
+// The row passes of the plans LD_FX_ROWS_0 .. _5 (ld_fx_rows*.cu): pass
+// kFxPassRows (the frame's forward rows) or kFxPassInverse (`rows` inverse
+// rows) of fa, or kFxPassKspecRows of ka; false when `id` is not among them.
+enum { kFxPassRows = 0, kFxPassInverse = 1, kFxPassKspecRows = 2 };
+bool fx_rows_0(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+bool fx_rows_1(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+bool fx_rows_2(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+bool fx_rows_3(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+bool fx_rows_4(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+bool fx_rows_5(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
 // ld_selftest.cu: one bounded-wait self-test (LD_SELFTEST_*) on `err`.
 int launch_wait_selftest(int mode, long long budget, float4* scratch, int* err, cudaStream_t s);
 // FP64 stage twiddle tables of fixed plan `id` (ld_fxplans.h).

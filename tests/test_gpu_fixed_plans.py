@@ -1,7 +1,7 @@
-"""Every compiled column length: a narrow frame whose grid takes exactly that
-length, against the FP64 oracle, and against the runtime-planned transforms
-on the same grid (to the FP32 rounding that separates two orders of one
-transform)."""
+"""Every compiled column and row length: a narrow (or low) frame whose grid takes
+exactly that length, against the FP64 oracle, and against the runtime-planned
+transforms on the same grid (to the FP32 rounding that separates two orders
+of one transform)."""
 import os
 import re
 
@@ -20,9 +20,8 @@ _PLANS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))
 R = 16
 
 
-def _lengths():
-    text = open(_PLANS).read()
-    text = text[text.index("#define LD_FX_COLS_0"):text.index("LD_FX_COL_DESC")]
+def _lengths(kind):
+    text = "\n".join(re.findall(rf"#define LD_FX_{kind}_\d\(X\) \\\n((?:.*\\\n)*.*)", open(_PLANS).read()))
     return sorted({int(a) * int(b) * int(c) for a, b, c in re.findall(r"X\(\d+, (\d+), (\d+), (\d+)\)", text)})
 
 
@@ -56,16 +55,30 @@ def _render(p, frame, mode):
 
 
 def test_column_lengths_are_multiples_of_four():
-    lengths = _lengths()
-    assert len(lengths) >= 50 and all(n % 4 == 0 for n in lengths)
+    assert len(_lengths("COLS")) >= 50 and all(n % 4 == 0 for n in _lengths("COLS"))
+    assert len(_lengths("ROWS")) >= 45
+
+
+# rows or columns of padding, until the grid's cost model takes the length
+SPARE = (0, 16, 36, 46, 54, 80, 104, 120, 160, 190)
+
+
+def _check(p, frame, out, grid):
+    generic, grid2 = _render(p, frame, -1)
+    assert grid2 == grid
+    m = O.gaussian_rgb_matrix(O.wavelengths(p), p.rgbGaussCenterNm, p.rgbGaussSigmaNm)
+    ref = O.render(frame, p, O.build_psf_bank(p), m, m)
+    scale = float(ref[..., :3].max())
+    assert np.abs(out - ref).max() / scale < OUT_TOL
+    assert np.abs(out - generic).max() / scale < 1e-5
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", [0, 1])
-@pytest.mark.parametrize("n", _lengths())
+@pytest.mark.parametrize("n", _lengths("COLS"))
 def test_column_length_matches_oracle(n, form):
     p = _lens().copy(fftForm=form)
-    for spare in (0, 46, 54, 104, 160, 190):  # rows of padding, until the grid's cost model takes this length
+    for spare in SPARE:
         frame = S.make_frame(64, n - 2 * R - spare, 200, 1.0, 50.0, seed=n)
         # the first and the last row carry highlights: both ends of the column
         frame[0, 3, :3] = 40.0
@@ -74,10 +87,22 @@ def test_column_length_matches_oracle(n, form):
         if grid[1] == n:
             break
     assert grid[1] == n
-    generic, grid2 = _render(p, frame, -1)
-    assert grid2 == grid
-    m = O.gaussian_rgb_matrix(O.wavelengths(p), p.rgbGaussCenterNm, p.rgbGaussSigmaNm)
-    ref = O.render(frame, p, O.build_psf_bank(p), m, m)
-    scale = float(ref[..., :3].max())
-    assert np.abs(out - ref).max() / scale < OUT_TOL
-    assert np.abs(out - generic).max() / scale < 1e-5
+    _check(p, frame, out, grid)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("n", _lengths("ROWS"))
+def test_row_length_matches_oracle(n, form):
+    p = _lens().copy(fftForm=form)
+    for spare in SPARE:
+        # an odd width: the last pixel pair is half outside; 66 rows: a last
+        # row tile that is partly padding
+        frame = S.make_frame(2 * (n - R - spare) - 1, 66, 200, 1.0, 50.0, seed=n)
+        frame[3, 0, :3] = 40.0
+        frame[65, -1, :3] = 30.0
+        out, grid = _render(p, frame, 0)
+        if grid[0] == 2 * n:
+            break
+    assert grid[0] == 2 * n
+    _check(p, frame, out, grid)
