@@ -21,7 +21,8 @@ OUT = os.path.join(HERE, "liblensdiff_b200.so")
 ROOT = os.path.dirname(HERE)
 SOURCES = ["ld_host.cu", "ld_psf.cu", "ld_frame.cu", "ld_frame_fx.cu", "ld_fx_cols0.cu", "ld_fx_cols1.cu",
            "ld_fx_cols2.cu", "ld_fx_cols3.cu", "ld_fx_cols4.cu", "ld_fx_cols5.cu", "ld_fx_rows0.cu",
-           "ld_fx_rows1.cu", "ld_fx_rows2.cu", "ld_fx_rows3.cu", "ld_fx_rows4.cu", "ld_fx_rows5.cu", "ld_noalloc.cu", "ld_cufft.cu",
+           "ld_fx_rows1.cu", "ld_fx_rows2.cu", "ld_fx_rows3.cu", "ld_fx_rows4.cu", "ld_fx_rows5.cu", "ld_fx_psf0.cu",
+           "ld_fx_psf1.cu", "ld_fx_psf2.cu", "ld_fx_psf3.cu", "ld_noalloc.cu", "ld_cufft.cu",
            "ld_server.cu", "ld_dftgemm.cu", "ld_debug.cu", "ld_selftest.cu"]
 # cuFFT backs only the comparator form (fft_form LD_FFT_CUFFT)
 LIBS = ["-L/usr/local/cuda/lib64", "-lcufft", "-Xlinker", "-rpath", "-Xlinker", "/usr/local/cuda/lib64"]

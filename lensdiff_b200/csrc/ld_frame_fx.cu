@@ -1,5 +1,5 @@
 // ld_frame_fx.cu — the launchers of the fixed plans of ld_fxplans.h (their
-// kernels are in ld_fx_rows*.cu and ld_fx_cols*.cu) and the FP64 generation of
+// kernels are in ld_fx_rows*.cu, ld_fx_cols*.cu and ld_fx_psf*.cu) and the FP64 generation of
 // the plans' stage twiddle tables.
 //
 // Each fx_launch_* returns false when no fixed instantiation covers the launch
@@ -73,6 +73,12 @@ bool fx_launch_kspec_rows(const KernelSpectraArgs& a, cudaStream_t s) {
 bool fx_launch_kspec_cols(const KernelSpectraArgs& a, cudaStream_t s) {
     if (a.n_ker != 3 || a.g.plan_py.fixed == 0) return false;
     return cols_dispatch(a.g.plan_py.fixed, nullptr, &a, s);
+}
+
+bool fx_launch_psf(const PsfBankArgs& a, bool rows, cudaStream_t s) {
+    const int id = a.plan_s.fixed;
+    if (id == 0 || a.want_energy) return false;
+    return fx_psf_0(id, a, rows, s) || fx_psf_1(id, a, rows, s) || fx_psf_2(id, a, rows, s) || fx_psf_3(id, a, rows, s);
 }
 
 // A row plan's inverse runs its radices in reverse: its tables follow.

@@ -10,16 +10,18 @@
 // the fastest (the first is the default).  Odd radices lead where the length
 // has them: their strided first-stage stores spread over the shared-memory
 // banks.  A row plan's last radix is also its inverse's first, and is taken in
-// pairs of mirrored butterflies: a small one.
+// pairs of mirrored butterflies: a small one.  PSF plans (length S:
+// ld_fx_psf*.cu) cover the common PSF sizes; their first radix is a multiple
+// of four, whose transforms drop the zero half of the embedded pupil.
 #pragma once
 
 namespace ld {
 
-enum { kFxRows = 1, kFxCols = 2 };
+enum { kFxRows = 1, kFxCols = 2, kFxPsf = 3 };
 
 struct FxPlanDesc {
     int id;         // 1 .. 255 (0 means "no fixed plan")
-    int role;       // kFxRows, kFxCols
+    int role;       // kFxRows, kFxCols, kFxPsf
     int radix[3];   // radix of each stage, first stage first
     constexpr int n() const { return radix[0] * radix[1] * radix[2]; }
 };
@@ -64,16 +66,33 @@ struct FxPlanDesc {
     X(105, 9, 12, 4) X(111, 5, 25, 5) X(117, 9, 12, 8) X(123, 15, 10, 8) X(129, 15, 10, 10) \
     X(135, 16, 16, 8) X(141, 15, 16, 12) X(147, 20, 16, 12)
 
+// PSF plans X(id, R1, R2, R3), in the groups of ld_fx_psf0.cu .. ld_fx_psf3.cu.
+#define LD_FX_PSF_0(X) \
+    X(160, 8, 8, 8) X(164, 8, 9, 9) X(168, 12, 9, 8) X(172, 16, 8, 8) X(176, 16, 10, 8) \
+    X(180, 16, 12, 8) X(184, 16, 12, 10) X(188, 16, 16, 9) X(192, 20, 15, 10) X(196, 16, 16, 15)
+#define LD_FX_PSF_1(X) \
+    X(161, 8, 9, 8) X(165, 16, 9, 5) X(169, 20, 9, 5) X(173, 12, 10, 9) X(177, 16, 9, 9) \
+    X(181, 16, 10, 10) X(185, 20, 10, 10) X(189, 16, 15, 10) X(193, 16, 16, 12) X(197, 20, 20, 10)
+#define LD_FX_PSF_2(X) \
+    X(162, 12, 10, 5) X(166, 12, 8, 8) X(170, 12, 10, 8) X(174, 16, 9, 8) X(178, 16, 10, 9) \
+    X(182, 16, 12, 9) X(186, 16, 16, 8) X(190, 16, 16, 10) X(194, 20, 16, 10) X(198, 16, 16, 16)
+#define LD_FX_PSF_3(X) \
+    X(163, 16, 8, 5) X(167, 16, 10, 5) X(171, 20, 10, 5) X(175, 12, 10, 10) X(179, 20, 15, 5) \
+    X(183, 20, 10, 9) X(187, 16, 15, 9) X(191, 16, 15, 12) X(195, 20, 15, 12)
+
 #define LD_FX_COL_DESC(ID, A, B, C) {ID, kFxCols, {A, B, C}},
 #define LD_FX_ROW_DESC(ID, A, B, C) {ID, kFxRows, {A, B, C}},
+#define LD_FX_PSF_DESC(ID, A, B, C) {ID, kFxPsf, {A, B, C}},
 constexpr FxPlanDesc kFxPlans[] = {
     LD_FX_COLS_0(LD_FX_COL_DESC) LD_FX_COLS_1(LD_FX_COL_DESC) LD_FX_COLS_2(LD_FX_COL_DESC)
     LD_FX_COLS_3(LD_FX_COL_DESC) LD_FX_COLS_4(LD_FX_COL_DESC) LD_FX_COLS_5(LD_FX_COL_DESC)
     LD_FX_ROWS_0(LD_FX_ROW_DESC) LD_FX_ROWS_1(LD_FX_ROW_DESC) LD_FX_ROWS_2(LD_FX_ROW_DESC)
     LD_FX_ROWS_3(LD_FX_ROW_DESC) LD_FX_ROWS_4(LD_FX_ROW_DESC) LD_FX_ROWS_5(LD_FX_ROW_DESC)
+    LD_FX_PSF_0(LD_FX_PSF_DESC) LD_FX_PSF_1(LD_FX_PSF_DESC) LD_FX_PSF_2(LD_FX_PSF_DESC) LD_FX_PSF_3(LD_FX_PSF_DESC)
 };
 #undef LD_FX_COL_DESC
 #undef LD_FX_ROW_DESC
+#undef LD_FX_PSF_DESC
 
 inline const FxPlanDesc* fx_plan(int id) {
     for (const FxPlanDesc& d : kFxPlans)

@@ -1356,7 +1356,7 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
     // 5 (the reference's Bluestein sizes) in every own form
     const bool dft = p.fft_form == LD_FFT_OWN_CHOSEN || (p.fft_form == LD_FFT_OWN_FP32 && !smooth(S));
     if (!pre && !dft && p.fft_form != LD_FFT_CUFFT) {
-        a.plan_s = make_plan(c, S, fft_family(S, 1) == kE25);
+        a.plan_s = make_plan(c, S, fft_family(S, 1) == kE25, kFxPsf);
         a.rows = static_cast<float2*>(ensure(c, c->rows, static_cast<size_t>(B) * a.row_n * win_stride * sizeof(float2)));
     }
     a.win = pre ? pre->win
@@ -1387,8 +1387,15 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
     } else if (dft) {
         dft_gemm_psf(c, a, infos, s);
     } else {
-        staged(c, LD_STAGE_PSF_ROWS, s, [&] { launch_psf_rows(a, s); });
-        staged(c, LD_STAGE_PSF_COLS, s, [&] { launch_psf_cols(a, s); });
+        bool fx = false;
+        staged(c, LD_STAGE_PSF_ROWS, s, [&] {
+            fx = fx_launch_psf(a, true, s);
+            if (!fx) launch_psf_rows(a, s);
+        });
+        staged(c, LD_STAGE_PSF_COLS, s, [&] {
+            if (fx) fx_launch_psf(a, false, s);
+            else launch_psf_cols(a, s);
+        });
     }
     bool filtered = false;
     float inv_max = 0.0f;

@@ -180,6 +180,15 @@ bool fx_rows_2(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* k
 bool fx_rows_3(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
 bool fx_rows_4(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
 bool fx_rows_5(int id, int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s);
+// The row (rows) or column pass of a PSF bank's windows on the fixed plan of
+// a.plan_s (ld_fx_psf*.cu); false when none covers it, and for passes that sum
+// the energy (want_energy).  Both passes of a bank go the same way: the row
+// pass's phases differ from psf_rows_kernel's.
+bool fx_launch_psf(const PsfBankArgs& a, bool rows, cudaStream_t s);
+bool fx_psf_0(int id, const PsfBankArgs& a, bool rows, cudaStream_t s);
+bool fx_psf_1(int id, const PsfBankArgs& a, bool rows, cudaStream_t s);
+bool fx_psf_2(int id, const PsfBankArgs& a, bool rows, cudaStream_t s);
+bool fx_psf_3(int id, const PsfBankArgs& a, bool rows, cudaStream_t s);
 // ld_selftest.cu: one bounded-wait self-test (LD_SELFTEST_*) on `err`.
 int launch_wait_selftest(int mode, long long budget, float4* scratch, int* err, cudaStream_t s);
 // FP64 stage twiddle tables of fixed plan `id` (ld_fxplans.h).
