@@ -51,27 +51,27 @@ void append_stages(const int (&radix)[3], std::vector<float2>* out) {
 }  // namespace
 
 bool fx_launch_frame_rows(const FrameArgs& a, cudaStream_t s) {
-    if (a.n_drv != 1 || a.drv_effect || a.g.plan_m.fixed == 0) return false;
+    if (a.g.plan_m.fixed == 0) return false;
     return rows_dispatch(a.g.plan_m.fixed, kFxPassRows, &a, nullptr, 0, s);
 }
 
 bool fx_launch_frame_cols(const FrameArgs& a, cudaStream_t s) {
-    if (a.n_drv != 1 || a.n_out != 3 || a.g.plan_py.fixed == 0) return false;
+    if (a.g.plan_py.fixed == 0) return false;
     return cols_dispatch(a.g.plan_py.fixed, &a, nullptr, s);
 }
 
 bool fx_launch_frame_inverse(const FrameArgs& a, int rows, cudaStream_t s) {
-    if (a.n_out != 3 || a.g.plan_m.fixed == 0) return false;
+    if (a.g.plan_m.fixed == 0) return false;
     return rows_dispatch(a.g.plan_m.fixed, kFxPassInverse, &a, nullptr, rows, s);
 }
 
 bool fx_launch_kspec_rows(const KernelSpectraArgs& a, cudaStream_t s) {
-    if (a.n_ker != 3 || a.g.plan_m.fixed == 0) return false;
+    if (a.g.plan_m.fixed == 0) return false;
     return rows_dispatch(a.g.plan_m.fixed, kFxPassKspecRows, nullptr, &a, 0, s);
 }
 
 bool fx_launch_kspec_cols(const KernelSpectraArgs& a, cudaStream_t s) {
-    if (a.n_ker != 3 || a.g.plan_py.fixed == 0) return false;
+    if (a.g.plan_py.fixed == 0) return false;
     return cols_dispatch(a.g.plan_py.fixed, nullptr, &a, s);
 }
 

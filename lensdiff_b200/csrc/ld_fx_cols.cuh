@@ -17,35 +17,36 @@ struct ColsHeader {
     float part[32];
 };
 
-constexpr size_t cols_bytes(int n) { return kColsHeader + static_cast<size_t>(n) * 4 * sizeof(float2); }
+// Shared memory of a column pass: C interleaved sequences and one more.
+constexpr size_t cols_bytes(int n, int C) { return kColsHeader + static_cast<size_t>(n) * (C + 1) * sizeof(float2); }
 
-// Threads of a column pass over three interleaved sequences: the multiple of
-// 32 with the most useful element slots in flight per SM.  A stage of radix
-// R keeps ceil(3 n / R / T) butterflies of R values per thread in registers
+// Threads of a column pass over C interleaved sequences: the multiple of 32
+// with the most useful element slots in flight per SM.  A stage of radix
+// R keeps ceil(C n / R / T) butterflies of R values per thread in registers
 // (at most 32 values); a thread needs 80 registers, and each CTA its share of
 // shared memory (cols_bytes).
 struct ColsShape {
     int threads, ctas;
 };
-template <class P>
+template <class P, int C>
 constexpr ColsShape cols_shape() {
     const int radix[3] = {P::R1, P::R2, P::R3};
     ColsShape best{0, 0};
     double score = -1.0;
-    for (int t = 96; t <= 800; t += 32) {
+    for (int t = 32; t <= 800; t += 32) {
         int steps = 0;
         bool fits = true;
         for (int r : radix) {
-            const int it = (3 * P::n / r + t - 1) / t;
+            const int it = (C * P::n / r + t - 1) / t;
             steps += it * r;
             if (it * r > 32) fits = false;
         }
-        const int by_smem = static_cast<int>((228 * 1024) / (cols_bytes(P::n) + 1024));
+        const int by_smem = static_cast<int>((228 * 1024) / (cols_bytes(P::n, C) + 1024));
         const int by_regs = 65536 / (80 * t);
         int ctas = by_smem < by_regs ? by_smem : by_regs;
         if (ctas > 8) ctas = 8;
         if (!fits || ctas < 1) continue;
-        const double s = 9.0 * P::n / steps * ctas;  // useful slots per SM
+        const double s = 3.0 * C * P::n / steps * ctas;  // useful slots per SM
         if (s > score) {
             score = s;
             best = ColsShape{t, ctas};
@@ -54,9 +55,10 @@ constexpr ColsShape cols_shape() {
     return best;
 }
 
-// Column k = blockIdx.x: its row spectra transformed, multiplied by its three
-// kernel spectra, the products transformed back, the first Hp rows stored to
-// B.  Shared memory: the header, F [n] (the column's spectrum), W [n][3].
+// Column k = blockIdx.x: its row spectra transformed, multiplied by its C (3 or,
+// with the luma lock, 4) kernel spectra, the products transformed back, the
+// first Hp rows stored to B.  Shared memory: the header, F [n] (the column's
+// spectrum), W [n][C].
 // H16: the half2 row spectra and their row exponents arrive at the start of W
 // (widened as the forward transform's first stage loads them), the half2
 // kernel spectra in W's upper half (multiplied with F as the inverse's first
@@ -75,7 +77,7 @@ constexpr ColsShape cols_shape() {
 //   1126 columns of 1800: 42 us (101)
 //   1251 columns of 1600: 37 us (50)
 //   1201 columns of 1152: 29 us FP32 (72)
-template <class P, int T, int MINB, bool H16>
+template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int N = P::n;
@@ -85,12 +87,12 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
     const int Hp = a.Hp, cols = a.g.cols;
     const int k = blockIdx.x;
     const uint32_t a_bytes = static_cast<uint32_t>(Hp * (H16 ? sizeof(__half2) : sizeof(float2)));
-    constexpr uint32_t k_bytes = static_cast<uint32_t>(N * 3 * (H16 ? sizeof(__half2) : sizeof(float2)));
+    constexpr uint32_t k_bytes = static_cast<uint32_t>(N * C * (H16 ? sizeof(__half2) : sizeof(float2)));
     const char* asrc = reinterpret_cast<const char*>(a.A) + static_cast<size_t>(k) * a_bytes;
     const char* ksrc = reinterpret_cast<const char*>(a.spectra) + static_cast<size_t>(k) * k_bytes;
     __half2* ah = reinterpret_cast<__half2*>(W);
     signed char* aex = reinterpret_cast<signed char*>(ah + Hp);
-    __half2* kh = reinterpret_cast<__half2*>(W) + 3 * N;
+    __half2* kh = reinterpret_cast<__half2*>(W) + C * N;
     if (threadIdx.x == 0) {
         mbar_init(&h->bar[0], 1);
         mbar_init(&h->bar[1], 1);
@@ -129,20 +131,20 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
         fp_stage<N, 1, T, false, P::R3, P::R1 * P::R2, true>(tw + P::tab3, ldF, stF);
     }
     if (__syncthreads_or(!mbar_wait(&h->bar[1], 0, a.err))) return;
-    fp_stage<N, 3, T, true, P::R1, 1, true>(
-        nullptr, [&](int e) { return cmul(H16 ? __half22float2(kh[e]) : W[e], F[e / 3]); }, stW);
+    fp_stage<N, C, T, true, P::R1, 1, true>(
+        nullptr, [&](int e) { return cmul(H16 ? __half22float2(kh[e]) : W[e], F[e / C]); }, stW);
     __syncthreads();
-    fp_stage<N, 3, T, true, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+    fp_stage<N, C, T, true, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
     __syncthreads();
-    LastStage<N, 3, T, true, P::R3> last;
+    LastStage<N, C, T, true, P::R3> last;
     last.run(tw + P::tab3, ldW);
-    // element e = row * 3 + c of column k goes to B's group of four columns
-    const int64_t base = (static_cast<int64_t>(k / kBGroup) * Hp * kBGroup + k % kBGroup) * 3;
-    constexpr int step = kBGroup * 3;
+    // element e = row * C + c of column k goes to B's group of four columns
+    const int64_t base = (static_cast<int64_t>(k / kBGroup) * Hp * kBGroup + k % kBGroup) * C;
+    constexpr int step = kBGroup * C;
     if constexpr (H16) {
         float m = 0.0f;
         last.each([&](int e, float2 v) {
-            if (e < Hp * 3) m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+            if (e < Hp * C) m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
         });
         m = cta_max<T>(m, h->part);
         const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
@@ -150,39 +152,93 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
         if (threadIdx.x == 0) a.bscale[k] = (m > 0.0f ? m / kHalfTop : 1.0f) * a.kscale[k];
         __half2* out = reinterpret_cast<__half2*>(a.Bout) + base;
         last.each([&](int e, float2 v) {
-            const int row = e / 3;
-            if (row < Hp) out[row * step + (e - row * 3)] = to_half2(v, sc);
+            const int row = e / C;
+            if (row < Hp) out[row * step + (e - row * C)] = to_half2(v, sc);
         });
     } else {
         float2* out = a.Bout + base;
         last.each([&](int e, float2 v) {
-            const int row = e / 3;
-            if (row < Hp) out[row * step + (e - row * 3)] = v;
+            const int row = e / C;
+            if (row < Hp) out[row * step + (e - row * C)] = v;
         });
     }
 }
 
-// Column k of the kernel spectra: the row spectra of the canvas rows (Kp x 3)
+// The Mono column pass (FP32): the three colours' row spectra (X [n][3], arriving
+// in its first Hp rows) transformed, multiplied by the one kernel spectrum
+// (Kc [n]), transformed back.  321 columns of 400 take 7.8 us (16.8 with the
+// runtime-planned transforms), the scatter's 1001 of 1200 35 us (60).
+template <class P, int T, int MINB>
+__global__ void __launch_bounds__(T, MINB) fx_frame_cols_mono_kernel(FrameArgs a) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    constexpr int N = P::n, C = 3;
+    ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
+    float2* X = reinterpret_cast<float2*>(smraw + kColsHeader);
+    float2* Kc = X + C * N;
+    const int Hp = a.Hp, cols = a.g.cols;
+    const int k = blockIdx.x;
+    const uint32_t a_bytes = static_cast<uint32_t>(Hp * C * sizeof(float2));
+    constexpr uint32_t k_bytes = N * sizeof(float2);
+    const float2* asrc = a.A + static_cast<size_t>(k) * Hp * C;
+    const float2* ksrc = a.spectra + static_cast<size_t>(k) * N;
+    if (threadIdx.x == 0) {
+        mbar_init(&h->bar[0], 1);
+        mbar_init(&h->bar[1], 1);
+        mbar_init_fence();
+        bulk_load_checked(X, asrc, a_bytes, &h->bar[0], smraw, a.err);
+        bulk_load_checked(Kc, ksrc, k_bytes, &h->bar[1], smraw, a.err);
+        const int later = k + a.ahead;
+        if (later < cols) {
+            bulk_prefetch_l2(a.A + static_cast<size_t>(later) * Hp * C, a_bytes);
+            bulk_prefetch_l2(a.spectra + static_cast<size_t>(later) * N, k_bytes);
+        }
+    }
+    __syncthreads();  // barriers initialised before anyone waits on them
+    const float2* tw = a.g.plan_py.stw;
+    if (__syncthreads_or(!mbar_wait(&h->bar[0], 0, a.err))) return;
+    auto ld = [&](int e) { return X[e]; };
+    auto st = [&](int e, float2 v) { X[e] = v; };
+    fp_stage<N, C, T, false, P::R1, 1, true>(
+        nullptr, [&](int e) { return e < Hp * C ? X[e] : make_float2(0.0f, 0.0f); }, st);
+    __syncthreads();
+    fp_stage<N, C, T, false, P::R2, P::R1, true>(tw + P::tab2, ld, st);
+    __syncthreads();
+    fp_stage<N, C, T, false, P::R3, P::R1 * P::R2, true>(tw + P::tab3, ld, st);
+    if (__syncthreads_or(!mbar_wait(&h->bar[1], 0, a.err))) return;
+    fp_stage<N, C, T, true, P::R1, 1, true>(nullptr, [&](int e) { return cmul(X[e], Kc[e / C]); }, st);
+    __syncthreads();
+    fp_stage<N, C, T, true, P::R2, P::R1, true>(tw + P::tab2, ld, st);
+    __syncthreads();
+    LastStage<N, C, T, true, P::R3> last;
+    last.run(tw + P::tab3, ld);
+    float2* out = a.Bout + (static_cast<int64_t>(k / kBGroup) * Hp * kBGroup + k % kBGroup) * C;
+    last.each([&](int e, float2 v) {
+        const int row = e / C;
+        if (row < Hp) out[row * (kBGroup * C) + (e - row * C)] = v;
+    });
+}
+
+// Column k of the C kernel spectra: the row spectra of the canvas rows (Kp x C)
 // arrive by bulk copy behind W, take their wrapped grid rows as the first
 // stage loads them, and the last stage's registers go out to KS[k] (H16: in
 // FP16 with the column's scale).  2501 columns of 3200 take 97 us (128 before,
 // see above), 4097 of 5120 284 us (517), 1126 of 1800 28 us (66).
-template <class P, int T, int MINB, bool H16>
+template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArgs a) {
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int N = P::n;
     ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
     float2* W = reinterpret_cast<float2*>(smraw + kColsHeader);
-    float2* Rb = W + 3 * N;
+    float2* Rb = W + C * N;
     const int cols = a.g.cols, Kp = a.Kp, R = a.R;
     const int k = blockIdx.x;
-    const uint32_t r_bytes = static_cast<uint32_t>(Kp * 3 * sizeof(float2));
+    const uint32_t r_bytes = static_cast<uint32_t>(Kp * C * sizeof(float2));
     if (threadIdx.x == 0) {
         mbar_init(&h->bar[0], 1);
         mbar_init_fence();
-        bulk_load_checked(Rb, a.rows + static_cast<size_t>(k) * Kp * 3, r_bytes, &h->bar[0], smraw, a.err);
+        bulk_load_checked(Rb, a.rows + static_cast<size_t>(k) * Kp * C, r_bytes, &h->bar[0], smraw, a.err);
         const int later = k + a.ahead;
-        if (later < cols) bulk_prefetch_l2(a.rows + static_cast<size_t>(later) * Kp * 3, r_bytes);
+        if (later < cols) bulk_prefetch_l2(a.rows + static_cast<size_t>(later) * Kp * C, r_bytes);
     }
     __syncthreads();  // barrier initialised before anyone waits on it
     const float2* tw = a.g.plan_py.stw;
@@ -190,19 +246,19 @@ __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArg
     auto ldW = [&](int e) { return W[e]; };
     auto stW = [&](int e, float2 v) { W[e] = v; };
     // grid row v holds canvas row v + R (v <= R) or v - N + R (v >= N - R)
-    fp_stage<N, 3, T, false, P::R1, 1, false>(
+    fp_stage<N, C, T, false, P::R1, 1, false>(
         nullptr,
         [&](int e) {
-            const int lo = e + 3 * R, hi = e - 3 * (N - R);
-            if (e < 3 * (R + 1)) return Rb[lo];
+            const int lo = e + C * R, hi = e - C * (N - R);
+            if (e < C * (R + 1)) return Rb[lo];
             if (hi >= 0) return Rb[hi];
             return make_float2(0.0f, 0.0f);
         },
         stW);
     __syncthreads();
-    fp_stage<N, 3, T, false, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+    fp_stage<N, C, T, false, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
     __syncthreads();
-    LastStage<N, 3, T, false, P::R3> last;
+    LastStage<N, C, T, false, P::R3> last;
     last.run(tw + P::tab3, ldW);
     if constexpr (H16) {
         float m = 0.0f;
@@ -210,47 +266,74 @@ __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArg
         m = cta_max<T>(m, h->part);
         const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
         if (threadIdx.x == 0) a.kscale[k] = m > 0.0f ? m / kHalfTop * a.scale : 1.0f;
-        __half2* out = reinterpret_cast<__half2*>(a.spectra) + static_cast<size_t>(k) * N * 3;
+        __half2* out = reinterpret_cast<__half2*>(a.spectra) + static_cast<size_t>(k) * N * C;
         last.each([&](int e, float2 v) { out[e] = to_half2(v, sc); });
     } else {
-        float2* out = a.spectra + static_cast<size_t>(k) * N * 3;
+        float2* out = a.spectra + static_cast<size_t>(k) * N * C;
         const float sc = a.scale;
         last.each([&](int e, float2 v) { out[e] = cscale(v, sc); });
     }
 }
 
-template <class P, bool H16>
+template <class P, int C, bool H16>
 void frame_cols_fx(FrameArgs a, cudaStream_t s) {
-    constexpr ColsShape sh = cols_shape<P>();
+    constexpr ColsShape sh = cols_shape<P, C>();
+    static_assert(sh.threads > 0);
     static KernelState state;
-    auto f = fx_frame_cols_kernel<P, sh.threads, sh.ctas, H16>;
-    const size_t sm = cols_bytes(P::n);
+    auto f = fx_frame_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
+    constexpr size_t sm = cols_bytes(P::n, C);
     a.ahead = state.get(f, sh.threads, sm);
     f<<<a.g.cols, sh.threads, sm, s>>>(a);
 }
 
-template <class P, bool H16>
-bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
-    constexpr ColsShape sh = cols_shape<P>();
+template <class P>
+void frame_cols_mono_fx(FrameArgs a, cudaStream_t s) {
+    constexpr ColsShape sh = cols_shape<P, 3>();
     static KernelState state;
-    auto f = fx_kspec_cols_kernel<P, sh.threads, sh.ctas, H16>;
-    const size_t sm = kColsHeader + (static_cast<size_t>(P::n) + a.Kp) * 3 * sizeof(float2);
+    auto f = fx_frame_cols_mono_kernel<P, sh.threads, sh.ctas>;
+    constexpr size_t sm = cols_bytes(P::n, 3);
+    a.ahead = state.get(f, sh.threads, sm);
+    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+}
+
+template <class P, int C, bool H16>
+bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
+    constexpr ColsShape sh = cols_shape<P, C>();
+    static_assert(sh.threads > 0);
+    static KernelState state;
+    auto f = fx_kspec_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
+    const size_t sm = kColsHeader + (static_cast<size_t>(P::n) + a.Kp) * C * sizeof(float2);
     if (sm > kSmemOptIn) return false;
-    a.ahead = state.get(f, sh.threads, cols_bytes(P::n));
+    a.ahead = state.get(f, sh.threads, cols_bytes(P::n, C));
     f<<<a.g.cols, sh.threads, sm, s>>>(a);
     return true;
 }
 
 // The launch of plan P: the frame's column pass (fa) or the kernel spectra's
-// (ka); false when it does not fit.
+// (ka); false when it does not fit, and for the Mono and luma-lock chains at
+// lengths above kFxOtherMax, which stay on the runtime-planned transforms.
 template <class P>
 bool cols_launch(const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
-    if (fa) {
-        if (fa->h16) frame_cols_fx<P, true>(*fa, s);
-        else frame_cols_fx<P, false>(*fa, s);
+    if (fa && fa->n_drv == 1 && fa->n_out == 3) {
+        if (fa->h16) frame_cols_fx<P, 3, true>(*fa, s);
+        else frame_cols_fx<P, 3, false>(*fa, s);
         return true;
     }
-    return ka->h16 ? kspec_cols_fx<P, true>(*ka, s) : kspec_cols_fx<P, false>(*ka, s);
+    if (ka && ka->n_ker == 3) return ka->h16 ? kspec_cols_fx<P, 3, true>(*ka, s) : kspec_cols_fx<P, 3, false>(*ka, s);
+    if constexpr (P::n <= kFxOtherMax) {
+        if (fa && fa->n_drv == 3) {
+            frame_cols_mono_fx<P>(*fa, s);
+            return true;
+        }
+        if (fa) {
+            if (fa->h16) frame_cols_fx<P, 4, true>(*fa, s);
+            else frame_cols_fx<P, 4, false>(*fa, s);
+            return true;
+        }
+        if (ka->n_ker == 1) return kspec_cols_fx<P, 1, false>(*ka, s);
+        return ka->h16 ? kspec_cols_fx<P, 4, true>(*ka, s) : kspec_cols_fx<P, 4, false>(*ka, s);
+    }
+    return false;
 }
 
 }  // namespace

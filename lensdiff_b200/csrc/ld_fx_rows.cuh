@@ -333,24 +333,44 @@ void kspec_rows_fx(const KernelSpectraArgs& a, cudaStream_t s) {
     f<<<a.Kp, sh.threads, sm, s>>>(a);
 }
 
-// The launch of plan P named by `pass`.
+// The launch of plan P named by `pass`; false for the Mono and luma-lock chains
+// at lengths above kFxOtherMax.
 template <class P>
 bool rows_launch(int pass, const FrameArgs* fa, const KernelSpectraArgs* ka, int rows, cudaStream_t s) {
-    switch (pass) {
-        case kFxPassRows:
-            if (fa->n_drv != 1) return false;
+    constexpr bool other = P::n <= kFxOtherMax;
+    if (pass == kFxPassRows) {
+        if (fa->n_drv == 1) {
             frame_rows_fx<P, rows_per_cta(P::n), 1, false>(*fa, s);
             return true;
-        case kFxPassInverse:
-            if (fa->n_out != 3) return false;
+        }
+        if constexpr (other) {
+            if (fa->drv_effect) frame_rows_fx<P, 3, 3, true>(*fa, s);
+            else frame_rows_fx<P, 3, 3, false>(*fa, s);
+            return true;
+        }
+    } else if (pass == kFxPassInverse) {
+        if (fa->n_out == 3) {
             if (fa->h16) frame_inverse_fx<P, 3, true>(*fa, rows, s);
             else frame_inverse_fx<P, 3, false>(*fa, rows, s);
             return true;
-        default:
-            if (ka->n_ker != 3) return false;
+        }
+        if constexpr (other) {
+            if (fa->h16) frame_inverse_fx<P, 4, true>(*fa, rows, s);
+            else frame_inverse_fx<P, 4, false>(*fa, rows, s);
+            return true;
+        }
+    } else {
+        if (ka->n_ker == 3) {
             kspec_rows_fx<P, 3>(*ka, s);
             return true;
+        }
+        if constexpr (other) {
+            if (ka->n_ker == 1) kspec_rows_fx<P, 1>(*ka, s);
+            else kspec_rows_fx<P, 4>(*ka, s);
+            return true;
+        }
     }
+    return false;
 }
 
 }  // namespace

@@ -249,6 +249,10 @@ __device__ __forceinline__ float cta_max(float m, float* part) {
     return m;
 }
 
+// The Mono (three drivers, one kernel) and luma-lock (four kernels) chains are
+// compiled for lengths up to this one: every HD and most UHD grids.
+constexpr int kFxOtherMax = 3200;
+
 // Largest dynamic shared memory of a kernel without static shared memory.
 constexpr size_t kSmemOptIn = 227 * 1024;
 

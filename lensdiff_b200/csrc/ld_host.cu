@@ -1550,11 +1550,9 @@ int choose_length(int n, int mult, int C) {
     return best;
 }
 
-// Whether the compiled plans serve a chain: one driver and three
-// kernels and outputs (the spectral modes without the luma lock).
-bool fx_chain(const Combination& cb, const ld_params& p) {
-    return cb.n_drv == 1 && cb.n_ker == 3 && cb.n_out == 3 && p.fft_form != LD_FFT_CUFFT;
-}
+// Whether the compiled plans serve a chain: every own form's (the cuFFT
+// comparator's transforms are cuFFT's).
+bool fx_chain(const ld_params& p) { return p.fft_form != LD_FFT_CUFFT; }
 
 // 5-smooth grid covering the linear convolution: Px = 2M with M the row
 // transform length, Py even (16-byte bulk-copy sizes).  The reference pads to
@@ -1993,7 +1991,7 @@ SpectraGeometry spectra_geometry(ld_ctx* c, const ld_params& p, int W, int H) {
     const int c_rows = std::max(std::max(sg.cb.n_drv == 1 ? 4 : 3, sg.cb.n_out), sg.cb.n_ker);
     const int c_cols = std::max(std::max(sg.cb.n_out, sg.cb.n_ker), sg.cb.n_drv);
     int rw = 0, rh = 0;
-    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_chain(sg.cb, p), &rw, &rh);
+    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_chain(p), &rw, &rh);
     sg.key = spectra_key_for(bank_key(p, wl), sg.cb, sg.g);
     const bool h16 = chosen_h16(p);
     sg.bytes = sg.cb.parts * (ks_part_bytes(sg.cb.n_ker, sg.g, h16) + static_cast<size_t>(sg.g.cols) * sizeof(float));
@@ -2682,7 +2680,7 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         const ZoneTiles zt = zones && p.fft_form != LD_FFT_CUFFT ? zone_tiles(Ww, Hw, zn) : ZoneTiles{};
         const bool tiled = zt.n > 0 && static_cast<double>(zt.wo + Kmax - 1) * (zt.ho + Kmax - 1) <=
                                            0.5 * static_cast<double>(Ww + Kmax - 1) * (Hw + Kmax - 1);
-        const bool fx = fx_chain(cb, p);
+        const bool fx = fx_chain(p);
         const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx, &rw, &rh)
                                  : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx, &rw, &rh);
         // Spectra already cached (a warm frame)?  If not, the bank and kernel
@@ -2764,7 +2762,7 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         if (post.scatter) {
             const int Ks = 2 * std::max(1, static_cast<int>(std::ceil(std::max(0.5f, post.scatter_radius)))) + 1;
             int srw = 0, srh = 0;
-            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, false, &srw, &srh);
+            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, fx_chain(p), &srw, &srh);
         }
         // rows of the row spectra: the frame's, or a tile's input rows
         const int Hp = tiled ? ((zt.ho + Kmax - 1 + 3) & ~3) : ((Hw + 3) & ~3);
