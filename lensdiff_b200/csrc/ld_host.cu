@@ -63,7 +63,7 @@ struct BankEntry {
     bool h16 = false;    // chosen form: kernel spectra in FP16 with per-column scales
     bool split_sums = false;  // s_core / s_struct computed (first Split render of the bank)
     bool ring_means = false;  // ring means computed (built unfused, or on first Split use)
-    DevBuf canvas, ring_round, ring_ceil, ring_peak, ring_mean, scalars, wl;
+    DevBuf canvas, stats, wl;  // stats: ring sums, peaks and scalars (one memset), then the ring means
     PsfBankArgs args{};
 };
 
@@ -1363,21 +1363,22 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
                 : static_cast<float*>(ensure(c, c->win, static_cast<size_t>(B) * win_stride * win_stride * sizeof(float)));
     a.canvas = static_cast<float*>(ensure(c, b.canvas, static_cast<size_t>(B) * K * K * sizeof(float)));
     const size_t ringn = static_cast<size_t>(B) * (R + 1);
-    a.ring_round = static_cast<double*>(ensure(c, b.ring_round, ringn * sizeof(double)));
-    a.ring_ceil = static_cast<double*>(ensure(c, b.ring_ceil, ringn * sizeof(double)));
-    a.ring_peak = static_cast<unsigned int*>(ensure(c, b.ring_peak, ringn * sizeof(unsigned int)));
-    a.ring_mean = static_cast<float*>(ensure(c, b.ring_mean, ringn * sizeof(float)));
-    a.scalars = static_cast<PsfScalars*>(ensure(c, b.scalars, static_cast<size_t>(B) * sizeof(PsfScalars)));
+    // the statistics that start at zero lie together, for one memset
+    const size_t zeroed = static_cast<size_t>(B) * sizeof(PsfScalars) + ringn * (2 * sizeof(double) + sizeof(unsigned int));
+    static_assert(sizeof(PsfScalars) % sizeof(double) == 0, "the ring sums follow the scalars");
+    char* stats = static_cast<char*>(ensure(c, b.stats, zeroed + ringn * sizeof(float)));
+    a.scalars = reinterpret_cast<PsfScalars*>(stats);
+    a.ring_round = reinterpret_cast<double*>(a.scalars + B);
+    a.ring_ceil = a.ring_round + ringn;
+    a.ring_peak = reinterpret_cast<unsigned int*>(a.ring_ceil + ringn);
+    a.ring_mean = reinterpret_cast<float*>(a.ring_peak + ringn);
     WavelengthInfo* dwl =
         pre ? pre->wl : static_cast<WavelengthInfo*>(ensure(c, b.wl, static_cast<size_t>(B) * sizeof(WavelengthInfo)));
     a.wl = dwl;
     a.count_round = ring_counts(c, R);
     a.want_energy = 0;
     if (!pre) upload_async(c, dwl, infos.data(), infos.size() * sizeof(WavelengthInfo), s, "bank-upload");
-    check_cuda(cudaMemsetAsync(a.ring_round, 0, ringn * sizeof(double), s), "bank-memset");
-    check_cuda(cudaMemsetAsync(a.ring_ceil, 0, ringn * sizeof(double), s), "bank-memset");
-    check_cuda(cudaMemsetAsync(a.ring_peak, 0, ringn * sizeof(unsigned int), s), "bank-memset");
-    check_cuda(cudaMemsetAsync(a.scalars, 0, static_cast<size_t>(B) * sizeof(PsfScalars), s), "bank-memset");
+    check_cuda(cudaMemsetAsync(stats, 0, zeroed, s), "bank-memset");
     if (pre) {
         // windows already synthesised
     } else if (p.fft_form == LD_FFT_CUFFT) {
@@ -1809,7 +1810,7 @@ constexpr size_t kSetChunkBytes = size_t(32) << 30;
 void build_lens_set(ld_ctx* c, const ld_params* ps, size_t n, cudaStream_t s, int* rebuilt_count) {
     for (size_t i = n; i < c->set_banks.size(); ++i) {
         BankEntry& e = c->set_banks[i];
-        for (DevBuf* b : {&e.canvas, &e.ring_round, &e.ring_ceil, &e.ring_peak, &e.ring_mean, &e.scalars, &e.wl})
+        for (DevBuf* b : {&e.canvas, &e.stats, &e.wl})
             free_buf(c, *b);
     }
     c->set_banks.resize(n);
@@ -2081,15 +2082,14 @@ void ld_destroy(ld_ctx* c) {
         if (b.host) cudaFreeHost(b.host);
         if (b.ev) cudaEventDestroy(b.ev);
     }
-    DevBuf* bb[] = {&c->bank.canvas, &c->bank.ring_round, &c->bank.ring_ceil, &c->bank.ring_peak, &c->bank.ring_mean,
-                    &c->bank.scalars, &c->bank.wl,        &c->spectra.spectra};
+    DevBuf* bb[] = {&c->bank.canvas, &c->bank.stats, &c->bank.wl, &c->spectra.spectra};
     for (DevBuf* b : bb) free_buf(c, *b);
     for (auto& z : c->zone_spectra) free_buf(c, z.spectra);
     for (auto& z : c->spectra_lru) free_buf(c, z.spectra);
     for (auto* v : {&c->zone_pupil, &c->zone_wl, &c->zone_win, &c->set_pupil, &c->set_win})
         for (auto& z : *v) free_buf(c, z);
     for (BankEntry& e : c->set_banks)
-        for (DevBuf* b : {&e.canvas, &e.ring_round, &e.ring_ceil, &e.ring_peak, &e.ring_mean, &e.scalars, &e.wl})
+        for (DevBuf* b : {&e.canvas, &e.stats, &e.wl})
             free_buf(c, *b);
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
     delete c;

@@ -816,18 +816,34 @@ __global__ void __launch_bounds__(256) support_kernel(PsfBankArgs a) {
     chunk_sum[tid] = lsum;
     if (tid == 0) first_hit = 1 << 30;
     __syncthreads();
-    if (tid == 0) {  // exclusive prefix sums / suffix maxima over the 256 chunks
-        double run = 0.0;
-        for (int t = 0; t < 256; ++t) {
-            const double s = chunk_sum[t];
-            chunk_sum[t] = run;
-            run += s;
-        }
-        float m = 0.0f;
-        for (int t = 255; t >= 0; --t) {
-            const float v = chunk_max[t];
-            chunk_max[t] = m;  // maximum over the chunks after t
-            m = fmaxf(m, v);
+    {  // exclusive prefix sums / suffix maxima over the 256 chunks: one warp, eight chunks a lane
+        if (tid < 32) {
+            double run = 0.0, sums[8];
+            float m = 0.0f, maxs[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                sums[i] = run;
+                run += chunk_sum[tid * 8 + i];
+                maxs[7 - i] = m;  // maximum over this lane's chunks after 7 - i
+                m = fmaxf(m, chunk_max[tid * 8 + 7 - i]);
+            }
+            double before = run;
+            float after = m;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double t = __shfl_up_sync(0xffffffffu, before, o);
+                const float u = __shfl_down_sync(0xffffffffu, after, o);
+                if (tid >= o) before += t;
+                if (tid + o < 32) after = fmaxf(after, u);
+            }
+            before -= run;
+            after = __shfl_down_sync(0xffffffffu, after, 1);
+            if (tid == 31) after = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                chunk_sum[tid * 8 + i] = before + sums[i];
+                chunk_max[tid * 8 + i] = fmaxf(after, maxs[i]);
+            }
         }
     }
     __syncthreads();
@@ -868,7 +884,7 @@ __global__ void __launch_bounds__(256) support_kernel(PsfBankArgs a) {
     sc.start = fmaxf(0.0f, extent - fade);
 }
 
-// grid (ceil(K/8), B), block 256: s4 = sum over the crop box of taper *
+// grid (ceil((R+1)/32), B), block 256: s4 = sum over the crop box of taper *
 // normalised shaped kernel, the normaliser of cropKernelToRadius and
 // applySupportBoundaryTaper (LensDiffCpuReference.cpp:1038-1058, :957-982).
 // The canvas keeps the shaped kernel; the crop and the taper are applied
@@ -877,10 +893,13 @@ __global__ void __launch_bounds__(256) support_kernel(PsfBankArgs a) {
 // with r < extent lies in the crop box, so s4 = (the ceil(r) ring energies of
 // rings 0 .. S0 = floor(start)) / s3 + the annulus S0 < r < extent pixel by
 // pixel.  A pixel's ring is ceil(sqrtf(dx^2 + dy^2)) <= S0 exactly when
-// dx^2 + dy^2 <= S0^2 (integers; exact below 2^24), so each crop row reads
-// only its |dx| > isqrt(S0^2 - dy^2) part.  One warp per crop row, eight
-// reads in flight per thread.
-constexpr int kCropRows = 8;
+// dx^2 + dy^2 <= S0^2 (integers; exact below 2^24), and its taper is 0 from
+// dx^2 + dy^2 = rho^2 on (extent = rho), so each row of the quadrant dx, dy >=
+// 0 reads only the dx between, with the mirror images, which share the
+// pixel's taper.  A warp takes two quadrant rows, a CTA's reductions serve 16
+// (a row a warp of the whole crop box, out to its corners: 33 us for 31
+// wavelengths at K = 1025, 14 us now).
+constexpr int kCropRows = 16;
 
 __device__ __forceinline__ int isqrt_floor(int v) {  // floor(sqrt(v)), v >= 0
     int r = static_cast<int>(sqrtf(static_cast<float>(v)));
@@ -894,41 +913,32 @@ __global__ void __launch_bounds__(256) crop_sum_kernel(PsfBankArgs a) {
     const PsfScalars& sc = a.scalars[b];
     const int rho = sc.radius;
     const int K = a.K, R = a.R;
-    const int y0 = R - rho + static_cast<int>(blockIdx.x) * kCropRows;
-    if (y0 > R + rho) return;  // uniform
+    const int d0 = static_cast<int>(blockIdx.x) * kCropRows;
+    if (d0 > rho) return;  // uniform
     const float inv_s3 = static_cast<float>(1.0 / sc.s3);
     const float extent = sc.extent, fade = sc.fade, start = sc.start;
     const int s0 = static_cast<int>(floorf(start));
     const int lane = threadIdx.x & 31;
-    const int y = y0 + static_cast<int>(threadIdx.x >> 5);  // one warp per crop row
+    const float* centre = a.canvas + static_cast<size_t>(b) * K * K + static_cast<size_t>(R) * K + R;
     float lsum = 0.0f;
-    if (y <= R + rho) {
-        const float* row = a.canvas + static_cast<size_t>(b) * K * K + static_cast<size_t>(y) * K + R;  // dx = 0
-        const int dyi = y - R;
-        const int in2 = s0 * s0 - dyi * dyi;
-        // |dx| <= xin lies inside ring s0; a row that misses that disc reads
-        // all of [-rho, rho] (left part [-rho, 0], right part [1, rho])
-        const int xin = in2 >= 0 ? isqrt_floor(in2) : -1;
-        const int nl = xin >= 0 ? rho - xin : rho + 1;  // left part: dx = -rho .. -rho + nl - 1
-        const int r0 = xin >= 0 ? xin + 1 : 1;          // right part: dx = r0 .. rho
-        const int n = nl + (rho - r0 + 1);
-        const float dy2 = static_cast<float>(dyi) * static_cast<float>(dyi);
-        constexpr int kU = 8;
-        for (int t0 = lane; t0 < n; t0 += kU * 32) {
-            float v[kU];
-            int dxs[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int t = t0 + u * 32;
-                dxs[u] = t < nl ? t - rho : r0 + (t - nl);
-                v[u] = t < n ? __ldg(row + dxs[u]) : 0.0f;
+    for (int i = 0; i < kCropRows / 8; ++i) {
+        const int dy = d0 + static_cast<int>(threadIdx.x >> 5) + 8 * i;
+        if (dy > rho) break;  // uniform: a warp walks rows
+        const int in2 = s0 * s0 - dy * dy;
+        const int first = in2 >= 0 ? isqrt_floor(in2) + 1 : 0;
+        const int last = isqrt_floor(rho * rho - dy * dy);
+        const float* up = centre + static_cast<ptrdiff_t>(dy) * K;
+        const float* down = centre - static_cast<ptrdiff_t>(dy) * K;
+        const float dy2 = static_cast<float>(dy) * static_cast<float>(dy);
+        for (int dx = first + lane; dx <= last; dx += 32) {
+            float v = __ldg(up + dx);
+            if (dx > 0) v += __ldg(up - dx);
+            if (dy > 0) {
+                v += __ldg(down + dx);
+                if (dx > 0) v += __ldg(down - dx);
             }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                if (t0 + u * 32 >= n) break;
-                const float dx = static_cast<float>(dxs[u]);
-                lsum += (v[u] * inv_s3) * taper_weight(sqrtf(dx * dx + dy2), extent, fade, start);
-            }
+            const float x = static_cast<float>(dx);
+            lsum += (v * inv_s3) * taper_weight(sqrtf(x * x + dy2), extent, fade, start);
         }
     }
     double tot = block_sum(static_cast<double>(lsum));
@@ -978,141 +988,128 @@ __global__ void __launch_bounds__(256) split_sums_kernel(PsfBankArgs a) {
     if (threadIdx.x == 0 && threadIdx.y == 0) atomicAdd(&a.scalars[b].s_struct, ts);
 }
 
-// grid (ceil(K/32), ceil(K/32)), block (32, 8): out[k] = sum_b coef[k][b] *
-// final_b with final_b = crop_b(canvas_b * taper_b) / (s3_b * s4_b): the crop
-// box and boundary taper of each wavelength (cropKernelToRadius,
-// applySupportBoundaryTaper, LensDiffCpuReference.cpp:1038-1058, :957-982)
-// are applied here as the shaped kernels are read.  Eight wavelengths'
-// reads are issued before any is used.  SPLIT: the core and structure
-// kernels of the Split look instead.
+// grid (ceil((R+1)/32), ceil((R+1)/8)), block (32, 8): out[k] = sum_b
+// coef[k][b] * final_b with final_b = crop_b(canvas_b * taper_b) / (s3_b *
+// s4_b): the crop box and boundary taper of each wavelength
+// (cropKernelToRadius, applySupportBoundaryTaper,
+// LensDiffCpuReference.cpp:1038-1058, :957-982) are applied here as the shaped
+// kernels are read.  A thread takes a pixel of the quadrant dx, dy >= 0 and its
+// mirror images, which share the radius, the crop test and the taper of every
+// wavelength; kL wavelengths' reads are issued before any is used; per pixel
+// the wavelengths are summed in order.  31 wavelengths at K = 1025 take 38 us
+// (reading the canvases takes 20 of HBM time; 67 us with four unrelated
+// pixels a thread).  SPLIT: the core and structure kernels of the Split look
+// instead: core = mean * taper / s_core, structure = max(0, shaped * taper /
+// s3 - mean * taper) / s_struct.
 struct CombineBin {
-    float w[4];                // coef[k][b] / (s3 s4)
-    float ext, fade, start;    // taper
-    int rho;                   // crop radius
+    float w[4];                     // coef[k][b] / (s3 s4), Split: coef[k][b]
+    float ext, fade, start;         // taper
+    int rho;                        // crop radius
+    float inv_s3, inv_core, inv_struct;
 };
 
-// NK: kernel sets of the Physical look (1 Mono, 3 spectral; 4 covers any n_ker <= 4).
+// NK: output kernels (1 Mono, 3 spectral, 4 with the luma lock; Split: 4).
 template <bool SPLIT, int NK>
 __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
-    __shared__ float inv[kMaxBins], inv_s3[kMaxBins], inv_core[kMaxBins], inv_struct[kMaxBins];
-    __shared__ float ext[kMaxBins], fade[kMaxBins], start[kMaxBins];
-    __shared__ int rho[kMaxBins];
     __shared__ CombineBin bin[kMaxBins];
     const int tid = threadIdx.x + threadIdx.y * 32;
     const int B = a.bank.B;
     for (int b = tid; b < B; b += 256) {
         const PsfScalars& sc = a.bank.scalars[b];
-        const float ib = static_cast<float>(1.0 / (sc.s3 * sc.s4));
-        for (int k = 0; k < 4; ++k) bin[b].w[k] = a.coef[k][b] * ib;
-        bin[b].ext = sc.extent;
-        bin[b].fade = sc.fade;
-        bin[b].start = sc.start;
-        bin[b].rho = sc.radius;
-        inv[b] = ib;
-        inv_s3[b] = static_cast<float>(1.0 / sc.s3);
-        inv_core[b] = sc.s_core > 0.0 ? static_cast<float>(1.0 / sc.s_core) : 0.0f;
-        inv_struct[b] = sc.s_struct > 0.0 ? static_cast<float>(1.0 / sc.s_struct) : 0.0f;
-        ext[b] = sc.extent;
-        fade[b] = sc.fade;
-        start[b] = sc.start;
-        rho[b] = sc.radius;
+        CombineBin& t = bin[b];
+        const float ib = SPLIT ? 1.0f : static_cast<float>(1.0 / (sc.s3 * sc.s4));
+        for (int k = 0; k < 4; ++k) t.w[k] = a.coef[k][b] * ib;
+        t.ext = sc.extent;
+        t.fade = sc.fade;
+        t.start = sc.start;
+        t.rho = sc.radius;
+        t.inv_s3 = static_cast<float>(1.0 / sc.s3);
+        t.inv_core = sc.s_core > 0.0 ? static_cast<float>(1.0 / sc.s_core) : 0.0f;
+        t.inv_struct = sc.s_struct > 0.0 ? static_cast<float>(1.0 / sc.s_struct) : 0.0f;
     }
     __syncthreads();
-    const int x = blockIdx.x * kTile + threadIdx.x;
     const int K = a.bank.K, R = a.bank.R;
+    const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y;
+    if (ix > R || iy > R) return;
     const size_t plane = static_cast<size_t>(K) * K;
+    constexpr int kP = 4;  // the mirror images (on an axis some coincide: the same value, written twice)
+    const int up = (R + iy) * K + R, down = (R - iy) * K + R;
+    const int idx[kP] = {up + ix, up - ix, down + ix, down - ix};
+    const int aix = max(ix, iy);  // inside the crop box of b iff aix <= rho[b]
+    const float dx = static_cast<float>(ix), dy = static_cast<float>(iy);
+    const float rad = sqrtf(dx * dx + dy * dy);
+    constexpr int kL = 4;
     if constexpr (!SPLIT) {
-        // four pixels per thread (rows 8 apart) share each wavelength's bin
-        // constants; per pixel the wavelengths are summed in order, as below
-        constexpr int kP = kTile / 8;
-        float acc[kP][NK], rad[kP];
-        int aix[kP];
-        size_t idx[kP];
-#pragma unroll
-        for (int p = 0; p < kP; ++p) {
-            const int y = blockIdx.y * kTile + threadIdx.y + 8 * p;
-            const bool in = x < K && y < K;
-            const int ix = x - R, iy = y - R;
-            aix[p] = in ? max(abs(ix), abs(iy)) : INT_MAX;  // inside the crop box of b iff aix <= rho[b]
-            const float dx = static_cast<float>(ix), dy = static_cast<float>(iy);
-            rad[p] = sqrtf(dx * dx + dy * dy);
-            idx[p] = in ? static_cast<size_t>(y) * K + x : 0;
-#pragma unroll
-            for (int k = 0; k < NK; ++k) acc[p][k] = 0.0f;
-        }
-        // kL wavelengths' reads are issued before any of them is used, so
-        // kL * kP reads per thread are in flight over the canvases
-        constexpr int kL = 4;
+        float acc[kP][NK] = {};
         for (int b0 = 0; b0 < B; b0 += kL) {
             float v[kL][kP];
 #pragma unroll
             for (int l = 0; l < kL; ++l) {
-                const int b = b0 + l;
-                const int rho_b = b < B ? bin[b].rho : -1;
-                const float* cv = a.bank.canvas + static_cast<size_t>(b < B ? b : 0) * plane;
+                const int b = min(b0 + l, B - 1);
+                const bool in = b0 + l < B && aix <= bin[b].rho;
+                const float* cv = a.bank.canvas + b * plane;
 #pragma unroll
-                for (int p = 0; p < kP; ++p) v[l][p] = aix[p] <= rho_b ? __ldg(cv + idx[p]) : 0.0f;
+                for (int p = 0; p < kP; ++p) v[l][p] = in ? __ldg(cv + idx[p]) : 0.0f;
             }
 #pragma unroll
-            for (int l = 0; l < kL; ++l) {  // per pixel the wavelengths are summed in order
-                const int b = b0 + l;
-                if (b >= B) break;
-                const CombineBin& cb = bin[b];
-                const float ext_b = cb.ext, fade_b = cb.fade, start_b = cb.start;
-                float w[NK];
-#pragma unroll
-                for (int k = 0; k < NK; ++k) w[k] = cb.w[k];
+            for (int l = 0; l < kL; ++l) {
+                if (b0 + l >= B) break;
+                const CombineBin& cb = bin[b0 + l];
+                if (aix > cb.rho) continue;
+                const float wgt = taper_weight(rad, cb.ext, cb.fade, cb.start);
 #pragma unroll
                 for (int p = 0; p < kP; ++p) {
-                    if (v[l][p] != 0.0f) {  // else outside the crop box, or a zero kernel value
-                        const float f = v[l][p] * taper_weight(rad[p], ext_b, fade_b, start_b);
+                    const float f = v[l][p] * wgt;
 #pragma unroll
-                        for (int k = 0; k < NK; ++k) acc[p][k] += w[k] * f;
-                    }
+                    for (int k = 0; k < NK; ++k) acc[p][k] += cb.w[k] * f;
                 }
             }
         }
 #pragma unroll
         for (int p = 0; p < kP; ++p) {
-            if (aix[p] == INT_MAX) continue;
 #pragma unroll
-            for (int k = 0; k < NK; ++k)
-                if (k < a.n_ker) a.out[k * plane + idx[p]] = acc[p][k];
+            for (int k = 0; k < NK; ++k) a.out[k * plane + idx[p]] = acc[p][k];
         }
-        return;
-    }
-#pragma unroll 1
-    for (int i = 0; i < kTile / 8; ++i) {  // Split look
-        const int y = blockIdx.y * kTile + threadIdx.y + 8 * i;
-        if (x >= K || y >= K) continue;
-        const size_t idx = static_cast<size_t>(y) * K + x;
-        const int ix = x - R, iy = y - R;
-        const int aix = max(abs(ix), abs(iy));  // inside the crop box of b iff aix <= rho[b]
-        const float dx = static_cast<float>(ix), dy = static_cast<float>(iy);
-        const float rad = sqrtf(dx * dx + dy * dy);
-        {
-        // Split: core = mean * taper / s_core, structure = max(0, shaped *
-        // taper / s3 - mean * taper) / s_struct
+    } else {
         const int ring = min(R, static_cast<int>(roundf(rad)));
-        float core[4] = {0.0f, 0.0f, 0.0f, 0.0f}, strc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int b = 0; b < B; ++b) {
-            if (aix > rho[b]) continue;
-            const float wgt = taper_weight(rad, ext[b], fade[b], start[b]);
-            const float mt = a.bank.ring_mean[static_cast<size_t>(b) * (R + 1) + ring] * wgt;
-            const float c = mt * inv_core[b];
-            const float st = fmaxf(0.0f, (a.bank.canvas[b * plane + idx] * wgt) * inv_s3[b] - mt) * inv_struct[b];
+        float core[4] = {}, strc[kP][4] = {};
+        for (int b0 = 0; b0 < B; b0 += kL) {
+            float v[kL][kP], mean[kL];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                core[k] += a.coef[k][b] * c;
-                strc[k] += a.coef[k][b] * st;
+            for (int l = 0; l < kL; ++l) {
+                const int b = min(b0 + l, B - 1);
+                const bool in = b0 + l < B && aix <= bin[b].rho;
+                const float* cv = a.bank.canvas + b * plane;
+                mean[l] = in ? __ldg(a.bank.ring_mean + static_cast<size_t>(b) * (R + 1) + ring) : 0.0f;
+#pragma unroll
+                for (int p = 0; p < kP; ++p) v[l][p] = in ? __ldg(cv + idx[p]) : 0.0f;
+            }
+#pragma unroll
+            for (int l = 0; l < kL; ++l) {
+                if (b0 + l >= B) break;
+                const CombineBin& cb = bin[b0 + l];
+                if (aix > cb.rho) continue;
+                const float wgt = taper_weight(rad, cb.ext, cb.fade, cb.start);
+                const float mt = mean[l] * wgt;
+                const float c = mt * cb.inv_core;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) core[k] += cb.w[k] * c;
+#pragma unroll
+                for (int p = 0; p < kP; ++p) {
+                    const float st = fmaxf(0.0f, (v[l][p] * wgt) * cb.inv_s3 - mt) * cb.inv_struct;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) strc[p][k] += cb.w[k] * st;
+                }
             }
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (k >= a.n_ker) break;
-            a.out[k * plane + idx] = core[k];
-            a.out[(a.n_ker + k) * plane + idx] = strc[k];
-        }
+#pragma unroll
+            for (int p = 0; p < kP; ++p) {
+                a.out[k * plane + idx[p]] = core[k];
+                a.out[(a.n_ker + k) * plane + idx[p]] = strc[p][k];
+            }
         }
     }
 }
@@ -1371,7 +1368,7 @@ void launch_ring_means(const PsfBankArgs& a, cudaStream_t s) {
 void launch_support(const PsfBankArgs& a, cudaStream_t s) { support_kernel<<<a.B, 256, 0, s>>>(a); }
 
 void launch_crop_sum(const PsfBankArgs& a, cudaStream_t s) {
-    crop_sum_kernel<<<dim3((a.K + kCropRows - 1) / kCropRows, a.B), 256, 0, s>>>(a);
+    crop_sum_kernel<<<dim3((a.R + kCropRows) / kCropRows, a.B), 256, 0, s>>>(a);
 }
 
 void launch_split_sums(const PsfBankArgs& a, cudaStream_t s) {
@@ -1379,7 +1376,7 @@ void launch_split_sums(const PsfBankArgs& a, cudaStream_t s) {
 }
 
 void launch_combine(const CombineArgs& a, cudaStream_t s) {
-    const dim3 grid = canvas_grid(a.bank, 1), block(32, 8);
+    const dim3 grid((a.bank.R + 32) / 32, (a.bank.R + 8) / 8), block(32, 8);
     if (a.split) combine_kernel<true, 4><<<grid, block, 0, s>>>(a);
     else if (a.n_ker == 1) combine_kernel<false, 1><<<grid, block, 0, s>>>(a);
     else if (a.n_ker == 3) combine_kernel<false, 3><<<grid, block, 0, s>>>(a);
