@@ -101,8 +101,10 @@ struct ld_ctx {
     BankEntry bank;
     SpectraEntry spectra;
     std::vector<SpectraEntry> zone_spectra;  // field zones, zy * n + zx
-    // field zones' pupils, wavelength tables and windows of one batched transform
-    std::vector<DevBuf> zone_pupil, zone_wl, zone_win;
+    // field zones' pupils, wavelength tables and windows of one batched
+    // transform, and the canvases and statistics of a group of zones
+    std::vector<DevBuf> zone_pupil;
+    DevBuf zone_wl, zone_win, zone_canvas, zone_stats;
     // banks of unrelated lenses built together (ld_build_psf_banks), kept
     // until the next such build; the pupils, wavelength tables and windows of
     // one chunk of their batched transform
@@ -1314,6 +1316,53 @@ struct PreWindows {
     WavelengthInfo* wl;  // device, the matching wavelength table
 };
 
+// The canvas and statistics of a.B wavelengths (a.K, a.R set) in the given
+// buffers; the statistics that start at zero lie together, for one memset.
+size_t bank_zeroed(const PsfBankArgs& a) {
+    return static_cast<size_t>(a.B) *
+           (sizeof(PsfScalars) + (static_cast<size_t>(a.R) + 1) * (2 * sizeof(double) + sizeof(unsigned int)));
+}
+void bank_buffers(ld_ctx* c, PsfBankArgs& a, DevBuf& canvas, DevBuf& stats) {
+    static_assert(sizeof(PsfScalars) % sizeof(double) == 0, "the ring sums follow the scalars");
+    const size_t ringn = static_cast<size_t>(a.B) * (a.R + 1);
+    a.canvas = static_cast<float*>(ensure(c, canvas, static_cast<size_t>(a.B) * a.K * a.K * sizeof(float)));
+    char* p = static_cast<char*>(ensure(c, stats, bank_zeroed(a) + ringn * sizeof(float)));
+    a.scalars = reinterpret_cast<PsfScalars*>(p);
+    a.ring_round = reinterpret_cast<double*>(a.scalars + a.B);
+    a.ring_ceil = a.ring_round + ringn;
+    a.ring_peak = reinterpret_cast<unsigned int*>(a.ring_ceil + ringn);
+    a.ring_mean = reinterpret_cast<float*>(a.ring_peak + ringn);
+}
+
+// From the |F|^2 windows to the shaped canvases with their support and
+// normalisers; `infos`: the wavelengths' host table (or one zone's, when a.B
+// covers several zones of the same wavelengths).
+void shape_bank(ld_ctx* c, const PsfBankArgs& a, const std::vector<WavelengthInfo>& infos, cudaStream_t s) {
+    check_cuda(cudaMemsetAsync(a.scalars, 0, bank_zeroed(a), s), "bank-memset");
+    bool filtered = false;
+    float inv_max = 0.0f;
+    for (const WavelengthInfo& w : infos) {
+        if (w.taps != 0) filtered = true;
+        else inv_max = std::max(inv_max, w.inv_scale);
+    }
+    staged(c, LD_STAGE_RESAMPLE, s, [&] { launch_resample(a, filtered, inv_max, s); });
+    if (!fused_shaping(a)) staged(c, LD_STAGE_SHAPE_STATS, s, [&] { launch_shape_stats(a, s); });
+    staged(c, LD_STAGE_SUPPORT, s, [&] { launch_support(a, s); });
+    staged(c, LD_STAGE_CROP_SUM, s, [&] { launch_crop_sum(a, s); });
+}
+
+// What the canvas passes need of lens `p` beyond its windows and buffers.
+void bank_geometry(ld_ctx* c, PsfBankArgs& a, const ld_params& p, int S, int R) {
+    a.S = S;
+    a.half = S / 2;
+    a.off = std::max(0, (S - pupil_size(p)) / 2);
+    a.raw_center = (S % 2 == 0) ? static_cast<float>(S) * 0.5f : static_cast<float>(S - 1) * 0.5f;
+    a.R = R;
+    a.K = 2 * R + 1;
+    a.gain = 1.0f + std::max(0.0f, static_cast<float>(p.anisotropy_emphasis)) * 4.0f;  // :1127
+    a.count_round = ring_counts(c, R);
+}
+
 // The bank of `p`: the context's bank or a bank of the last lens set when
 // one matches, else built into the context's bank.  With `into`, built into
 // that entry unconditionally (lens sets).
@@ -1344,14 +1393,8 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
     a = PsfBankArgs{};
     if (!pre) setup_pupil(c, a, p, false, s);
     a.B = B;
-    a.S = S;
-    a.half = S / 2;
-    a.off = std::max(0, (S - np) / 2);
     a.win_stride = win_stride;
-    a.raw_center = (S % 2 == 0) ? static_cast<float>(S) * 0.5f : static_cast<float>(S - 1) * 0.5f;
-    a.R = R;
-    a.K = K;
-    a.gain = 1.0f + std::max(0.0f, static_cast<float>(p.anisotropy_emphasis)) * 4.0f;  // :1127
+    bank_geometry(c, a, p, S, R);
     // tensor-core DFT for the chosen form, and for S with a prime factor above
     // 5 (the reference's Bluestein sizes) in every own form
     const bool dft = p.fft_form == LD_FFT_OWN_CHOSEN || (p.fft_form == LD_FFT_OWN_FP32 && !smooth(S));
@@ -1361,24 +1404,12 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
     }
     a.win = pre ? pre->win
                 : static_cast<float*>(ensure(c, c->win, static_cast<size_t>(B) * win_stride * win_stride * sizeof(float)));
-    a.canvas = static_cast<float*>(ensure(c, b.canvas, static_cast<size_t>(B) * K * K * sizeof(float)));
-    const size_t ringn = static_cast<size_t>(B) * (R + 1);
-    // the statistics that start at zero lie together, for one memset
-    const size_t zeroed = static_cast<size_t>(B) * sizeof(PsfScalars) + ringn * (2 * sizeof(double) + sizeof(unsigned int));
-    static_assert(sizeof(PsfScalars) % sizeof(double) == 0, "the ring sums follow the scalars");
-    char* stats = static_cast<char*>(ensure(c, b.stats, zeroed + ringn * sizeof(float)));
-    a.scalars = reinterpret_cast<PsfScalars*>(stats);
-    a.ring_round = reinterpret_cast<double*>(a.scalars + B);
-    a.ring_ceil = a.ring_round + ringn;
-    a.ring_peak = reinterpret_cast<unsigned int*>(a.ring_ceil + ringn);
-    a.ring_mean = reinterpret_cast<float*>(a.ring_peak + ringn);
+    bank_buffers(c, a, b.canvas, b.stats);
     WavelengthInfo* dwl =
         pre ? pre->wl : static_cast<WavelengthInfo*>(ensure(c, b.wl, static_cast<size_t>(B) * sizeof(WavelengthInfo)));
     a.wl = dwl;
-    a.count_round = ring_counts(c, R);
     a.want_energy = 0;
     if (!pre) upload_async(c, dwl, infos.data(), infos.size() * sizeof(WavelengthInfo), s, "bank-upload");
-    check_cuda(cudaMemsetAsync(stats, 0, zeroed, s), "bank-memset");
     if (pre) {
         // windows already synthesised
     } else if (p.fft_form == LD_FFT_CUFFT) {
@@ -1398,17 +1429,7 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
             else launch_psf_cols(a, s);
         });
     }
-    bool filtered = false;
-    float inv_max = 0.0f;
-    for (const WavelengthInfo& w : infos) {
-        if (w.taps != 0) filtered = true;
-        else inv_max = std::max(inv_max, w.inv_scale);
-    }
-    staged(c, LD_STAGE_RESAMPLE, s, [&] { launch_resample(a, filtered, inv_max, s); });
-    const bool fused = fused_shaping(a);
-    if (!fused) staged(c, LD_STAGE_SHAPE_STATS, s, [&] { launch_shape_stats(a, s); });
-    staged(c, LD_STAGE_SUPPORT, s, [&] { launch_support(a, s); });
-    staged(c, LD_STAGE_CROP_SUM, s, [&] { launch_crop_sum(a, s); });
+    shape_bank(c, a, infos, s);
     check_launch("psf-bank");
     b.B = B;
     b.np = np;
@@ -1420,7 +1441,7 @@ BankEntry& ensure_bank(ld_ctx* c, const ld_params& p, cudaStream_t s, bool* rebu
     b.cufft = p.fft_form == LD_FFT_CUFFT;
     b.h16 = chosen_h16(p);
     b.split_sums = false;
-    b.ring_means = !fused;
+    b.ring_means = !fused_shaping(a);
     b.key = key;
     b.valid = true;
     if (!into) c->spectra.valid = false;
@@ -1740,57 +1761,94 @@ std::vector<const SpectraEntry*> ensure_zone_spectra(ld_ctx* c, const ld_params&
     // zone's windows come from one batched launch per pass.
     const int np = pupil_size(p), R = max_kernel_radius(p), S = raw_psf_size(np, R);
     const bool dft = p.fft_form == LD_FFT_OWN_CHOSEN || (p.fft_form == LD_FFT_OWN_FP32 && !smooth(S));
-    std::vector<PreWindows> pre(static_cast<size_t>(nz), PreWindows{nullptr, nullptr});
     if (dft && need.size() >= 2) {
-        c->zone_pupil.resize(static_cast<size_t>(nz));
-        c->zone_wl.resize(static_cast<size_t>(nz));
-        c->zone_win.resize(static_cast<size_t>(nz));
+        // every zone's wavelength table and windows lie one after another, so
+        // that the canvas passes take several zones as one bank of more
+        // wavelengths
+        const int B = static_cast<int>(wl.size());
+        if (B > kMaxBins) throw Fail{LD_ERR_ARG, "too-many-wavelengths"};
         const float r0 = first_zero(c, np, S, s);
         std::vector<PsfBankArgs> args(need.size());
         std::vector<std::vector<WavelengthInfo>> infos(need.size());
+        std::vector<WavelengthInfo> table;
+        int ws = 0;
+        for (size_t k = 0; k < need.size(); ++k) {
+            fill_wavelength_infos(zps[static_cast<size_t>(need[k])], wl, r0, S, R, &infos[k], &ws);
+            table.insert(table.end(), infos[k].begin(), infos[k].end());
+        }
+        c->zone_pupil.resize(static_cast<size_t>(nz));
+        WavelengthInfo* dwl =
+            static_cast<WavelengthInfo*>(ensure(c, c->zone_wl, table.size() * sizeof(WavelengthInfo)));
+        const size_t wsz = static_cast<size_t>(B) * ws * ws;
+        float* dwin = static_cast<float*>(ensure(c, c->zone_win, need.size() * wsz * sizeof(float)));
+        upload_async(c, dwl, table.data(), table.size() * sizeof(WavelengthInfo), s, "zone-upload");
         std::vector<const PsfBankArgs*> bp;
         std::vector<const std::vector<WavelengthInfo>*> ip;
         for (size_t k = 0; k < need.size(); ++k) {
-            const int z = need[k];
-            const ld_params& zp = zps[static_cast<size_t>(z)];
-            int ws = 0;
-            fill_wavelength_infos(zp, wl, r0, S, R, &infos[k], &ws);
             PsfBankArgs& a = args[k];
-            setup_pupil(c, a, zp, false, s, &c->zone_pupil[static_cast<size_t>(z)]);
-            a.B = static_cast<int>(wl.size());
-            a.S = S;
-            a.half = S / 2;
-            a.off = std::max(0, (S - np) / 2);
+            setup_pupil(c, a, zps[static_cast<size_t>(need[k])], false, s, &c->zone_pupil[static_cast<size_t>(need[k])]);
+            a.B = B;
             a.win_stride = ws;
-            a.wl = static_cast<WavelengthInfo*>(
-                ensure(c, c->zone_wl[static_cast<size_t>(z)], infos[k].size() * sizeof(WavelengthInfo)));
-            a.win = static_cast<float*>(
-                ensure(c, c->zone_win[static_cast<size_t>(z)], static_cast<size_t>(a.B) * ws * ws * sizeof(float)));
-            upload_async(c, const_cast<WavelengthInfo*>(a.wl), infos[k].data(),
-                         infos[k].size() * sizeof(WavelengthInfo), s, "zone-upload");
-            pre[static_cast<size_t>(z)] = PreWindows{a.win, const_cast<WavelengthInfo*>(a.wl)};
+            bank_geometry(c, a, p, S, R);
+            a.wl = dwl + k * B;
+            a.win = dwin + k * wsz;
             bp.push_back(&a);
             ip.push_back(&infos[k]);
         }
         dft_gemm_psf_batch(c, bp, ip, s);
-    }
-    std::vector<const SpectraEntry*> out;
-    for (int zy = 0; zy < n; ++zy) {
-        for (int zx = 0; zx < n; ++zx) {
-            const int z = zy * n + zx;
-            const ld_params& zp = zps[static_cast<size_t>(z)];
-            SpectraEntry& e = c->zone_spectra[static_cast<size_t>(z)];
-            const std::string& key = keys[static_cast<size_t>(z)];
-            if (!(e.valid && e.key == key)) {
-                bool rb = false, rs = false;
-                const PreWindows& pw = pre[static_cast<size_t>(z)];
-                BankEntry& b = ensure_bank(c, zp, s, &rb, pw.win ? &pw : nullptr);
-                ensure_spectra_in(c, e, b, cb, g, s, &rs);
-                *bank_rebuilt = *bank_rebuilt || rb;
+        // The canvas passes of `group` zones at a time: small kernels leave the
+        // GPU to a few CTAs per zone (3 x 3 zones of 9 wavelengths at K = 267:
+        // 20 + 5 + 7 us nine times), while canvases beyond kZoneCanvas would
+        // leave L2 before the combination reads them.  (A group's wavelengths
+        // are a launch dimension: at most 65535.)
+        constexpr size_t kZoneCanvas = size_t(96) << 20;
+        const size_t plane = static_cast<size_t>(2 * R + 1) * (2 * R + 1);
+        const size_t group = std::max<size_t>(
+            1, std::min({need.size(), kZoneCanvas / (plane * B * sizeof(float)), size_t(65535) / B}));
+        for (size_t k0 = 0; k0 < need.size(); k0 += group) {
+            const size_t m = std::min(group, need.size() - k0);
+            PsfBankArgs ga = args[k0];
+            ga.B = static_cast<int>(m) * B;
+            bank_buffers(c, ga, c->zone_canvas, c->zone_stats);
+            shape_bank(c, ga, infos[k0], s);
+            check_launch("psf-bank");
+            for (size_t k = k0; k < k0 + m; ++k) {
+                const size_t z = static_cast<size_t>(need[k]), first = (k - k0) * B, ring = first * (R + 1);
+                BankEntry b;  // zone z's part of the group
+                b.args = ga;
+                b.args.B = B;
+                b.args.wl = args[k].wl;
+                b.args.win = args[k].win;
+                b.args.canvas = ga.canvas + first * plane;
+                b.args.scalars = ga.scalars + first;
+                b.args.ring_round = ga.ring_round + ring;
+                b.args.ring_ceil = ga.ring_ceil + ring;
+                b.args.ring_peak = ga.ring_peak + ring;
+                b.args.ring_mean = ga.ring_mean + ring;
+                b.B = B;
+                b.R = R;
+                b.K = 2 * R + 1;
+                b.h16 = chosen_h16(p);
+                b.ring_means = !fused_shaping(ga);
+                b.key = bank_key(zps[z], wl);
+                bool rs = false;
+                ensure_spectra_in(c, c->zone_spectra[z], b, cb, g, s, &rs);
+                *bank_rebuilt = true;
                 *spectra_rebuilt = *spectra_rebuilt || rs;
             }
-            out.push_back(&e);
         }
+    }
+    std::vector<const SpectraEntry*> out;
+    for (size_t z = 0; z < static_cast<size_t>(nz); ++z) {
+        SpectraEntry& e = c->zone_spectra[z];
+        if (!(e.valid && e.key == keys[z])) {
+            bool rb = false, rs = false;
+            BankEntry& b = ensure_bank(c, zps[z], s, &rb);
+            ensure_spectra_in(c, e, b, cb, g, s, &rs);
+            *bank_rebuilt = *bank_rebuilt || rb;
+            *spectra_rebuilt = *spectra_rebuilt || rs;
+        }
+        out.push_back(&e);
     }
     return out;
 }
@@ -2061,7 +2119,8 @@ void ld_destroy(ld_ctx* c) {
     DevBuf* bufs[] = {&c->rows,   &c->win,     &c->combine_out, &c->kspec_rows, &c->frameA,    &c->frameB,
                       &c->calib,  &c->calib_psf, &c->err_word,  &c->pupil_pre,  &c->effect,    &c->cf_grid,
                       &c->cf_planes, &c->cf_sd,  &c->cf_prod,   &c->work,       &c->scatter_canvas,
-                      &c->scatter_ks, &c->dft,  &c->basis,    &c->debug,    &c->selftest, &c->custom.img};
+                      &c->scatter_ks, &c->dft,  &c->basis,    &c->debug,    &c->selftest, &c->custom.img,
+                      &c->zone_wl, &c->zone_win, &c->zone_canvas, &c->zone_stats};
     c->cufft.release();
     for (DevBuf* b : bufs) free_buf(c, *b);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
@@ -2086,7 +2145,7 @@ void ld_destroy(ld_ctx* c) {
     for (DevBuf* b : bb) free_buf(c, *b);
     for (auto& z : c->zone_spectra) free_buf(c, z.spectra);
     for (auto& z : c->spectra_lru) free_buf(c, z.spectra);
-    for (auto* v : {&c->zone_pupil, &c->zone_wl, &c->zone_win, &c->set_pupil, &c->set_win})
+    for (auto* v : {&c->zone_pupil, &c->set_pupil, &c->set_win})
         for (auto& z : *v) free_buf(c, z);
     for (BankEntry& e : c->set_banks)
         for (DevBuf* b : {&e.canvas, &e.stats, &e.wl})
