@@ -40,6 +40,7 @@
 
 #include "ld_async.cuh"
 #include "ld_internal.h"
+#include "ld_launch.cuh"
 
 namespace ld {
 namespace {
@@ -142,6 +143,7 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<ui
 // 2 pi ((x + koff) * u_n mod S) / S with u_n = (x0 + n + S/2) mod S, the
 // exponential evaluated in FP64.  Pairs with x >= k_valid are zero.
 __global__ void __launch_bounds__(256) dft_basis_kernel(DftBasisArgs a) {
+    stream_order();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t per_chunk = static_cast<int64_t>(a.rows) * 32;
     if (i >= per_chunk * a.kc) return;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(256) dft_basis_kernel(DftBasisArgs a) {
 // of K-chunk c (one 128-byte image row per warp), looping over the
 // wavelengths.
 __global__ void __launch_bounds__(256) pupil_field_kernel(PsfBankArgs a, DftPlan d) {
+    stream_order();
     const int c = blockIdx.y;
     const int m = blockIdx.x * 8 + threadIdx.y, q = threadIdx.x;
     const int np = a.pupil.size;
@@ -264,6 +267,7 @@ __device__ __forceinline__ TileSlot next_tile(const DftBatchArgs& g) {
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1) dft_gemm_kernel(DftBatchArgs g) {
+    stream_order();
     extern __shared__ __align__(1024) unsigned char smraw[];
     __shared__ uint64_t full[kStages], empty[kStages];
     __shared__ uint64_t acc_full[2], acc_empty[2];
@@ -464,13 +468,14 @@ size_t dft_gemm_smem() { return static_cast<size_t>(kStages) * kStageBytes + 102
 void launch_dft_basis(const DftBasisArgs& a, cudaStream_t s) {
     const int64_t total = static_cast<int64_t>(a.rows) * 32 * a.kc;
     if (total <= 0) return;
-    dft_basis_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(a);
+    launch_after(dft_basis_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, s, a);
 }
 
 void launch_pupil_field(const PsfBankArgs& a, const DftPlan& d, cudaStream_t s) {
     if (d.mt_rows <= 0 || d.kc_rows <= 0) return;
-    pupil_field_kernel<<<dim3(static_cast<unsigned>(d.mt_rows * kTileM / 8), static_cast<unsigned>(d.kc_rows), 1),
-                         dim3(32, 8), 0, s>>>(a, d);
+    launch_after(pupil_field_kernel,
+                 dim3(static_cast<unsigned>(d.mt_rows * kTileM / 8), static_cast<unsigned>(d.kc_rows), 1),
+                 dim3(32, 8), 0, s, a, d);
 }
 
 void launch_dft_gemm(const DftBatchArgs& g, cudaStream_t s) {
@@ -478,7 +483,7 @@ void launch_dft_gemm(const DftBatchArgs& g, cudaStream_t s) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    dft_gemm_kernel<<<static_cast<unsigned>(std::min(g.tiles, sms)), kGemmThreads, dft_gemm_smem(), s>>>(g);
+    launch_after(dft_gemm_kernel, static_cast<unsigned>(std::min(g.tiles, sms)), kGemmThreads, dft_gemm_smem(), s, g);
 }
 
 void configure_dft_kernels() {

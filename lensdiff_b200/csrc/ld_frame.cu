@@ -33,7 +33,7 @@ namespace {
 template <class Kern>
 void launch_ahead(Kern f, FrameArgs a, int grid, int T, size_t sm, cudaStream_t s) {
     a.ahead = resident_ctas(f, T, sm);
-    f<<<grid, T, sm, s>>>(a);
+    launch_after(f, grid, T, sm, s, a);
 }
 
 template <int E>
@@ -52,7 +52,8 @@ void rows_e(const FrameArgs& a, cudaStream_t s) {
     } else {
         const size_t sm = rows_smem(M, 3);
         if (a.drv_effect)
-            frame_rows_kernel<E, 3, 3, Fam<E>::max_threads, 1, true><<<a.Hp, fft_threads(M, 3, E), sm, s>>>(a);
+            launch_after(frame_rows_kernel<E, 3, 3, Fam<E>::max_threads, 1, true>, a.Hp, fft_threads(M, 3, E), sm, s,
+                         a);
         else
             launch_ahead(frame_rows_kernel<E, 3, 3>, a, a.Hp, fft_threads(M, 3, E), sm, s);
     }
@@ -62,7 +63,7 @@ template <int E, class Kern>
 void cols_launch(Kern f, FrameArgs a, int C, size_t sm, cudaStream_t s) {
     const int T = fft_threads(a.g.Py, C, E);
     a.ahead = resident_ctas(f, T, sm);
-    f<<<a.g.cols, T, sm, s>>>(a);
+    launch_after(f, a.g.cols, T, sm, s, a);
 }
 
 // Spectral column pass: two CTAs per SM (register cap 85) when the transform
@@ -116,8 +117,8 @@ void inverse_e(const FrameArgs& a, int rows, cudaStream_t s) {  // rows: grid si
 
 template <int E, int C>
 void kspec_rows_c(const KernelSpectraArgs& a, cudaStream_t s) {
-    kspec_rows_kernel<E, C><<<a.Kp, fft_threads(a.g.M, C, E), static_cast<size_t>(a.g.M) * C * sizeof(float2), s>>>(
-        a);
+    launch_after(kspec_rows_kernel<E, C>, a.Kp, fft_threads(a.g.M, C, E),
+                 static_cast<size_t>(a.g.M) * C * sizeof(float2), s, a);
 }
 
 template <int E, int C, bool H16>
@@ -128,11 +129,11 @@ void kspec_cols_h(KernelSpectraArgs a, cudaStream_t s) {
         // two CTAs per SM (register cap 80)
         auto f = kspec_cols_kernel<E, C, 384, 2, H16>;
         a.ahead = resident_ctas(f, T, sm);
-        f<<<a.g.cols, T, sm, s>>>(a);
+        launch_after(f, a.g.cols, T, sm, s, a);
     } else {
         auto f = kspec_cols_kernel<E, C, Fam<E>::max_threads, 1, H16>;
         a.ahead = resident_ctas(f, T, sm);
-        f<<<a.g.cols, T, sm, s>>>(a);
+        launch_after(f, a.g.cols, T, sm, s, a);
     }
 }
 
@@ -233,16 +234,16 @@ void launch_frame_inverse_rows(const FrameArgs& a, int rows, cudaStream_t s) {
     else inverse_e<kE16>(a, rows, s);
 }
 
-void launch_effect_sums(const FrameArgs& a, cudaStream_t s) { effect_sums_kernel<<<a.H, 256, 0, s>>>(a); }
+void launch_effect_sums(const FrameArgs& a, cudaStream_t s) { launch_after(effect_sums_kernel, a.H, 256, 0, s, a); }
 
 template <int MODE>
 void composite_launch(const FrameArgs& a, bool fringe, bool rs, int rows, cudaStream_t s) {
     if (rs) {
-        if (fringe) composite_kernel<MODE, true, true><<<rows, 256, 0, s>>>(a);
-        else composite_kernel<MODE, false, true><<<rows, 256, 0, s>>>(a);
+        if (fringe) launch_after(composite_kernel<MODE, true, true>, rows, 256, 0, s, a);
+        else launch_after(composite_kernel<MODE, false, true>, rows, 256, 0, s, a);
     } else {
-        if (fringe) composite_kernel<MODE, true, false><<<rows, 256, 0, s>>>(a);
-        else composite_kernel<MODE, false, false><<<rows, 256, 0, s>>>(a);
+        if (fringe) launch_after(composite_kernel<MODE, true, false>, rows, 256, 0, s, a);
+        else launch_after(composite_kernel<MODE, false, false>, rows, 256, 0, s, a);
     }
 }
 
@@ -255,16 +256,16 @@ void launch_composite(const FrameArgs& a, cudaStream_t s) {
             composite_launch<kOutEffect>(a, fringe, rs, rows, s);
             break;
         case kOutFringePreview:
-            if (rs) composite_kernel<kOutFringePreview, true, true><<<rows, 256, 0, s>>>(a);
-            else composite_kernel<kOutFringePreview, true, false><<<rows, 256, 0, s>>>(a);
+            if (rs) launch_after(composite_kernel<kOutFringePreview, true, true>, rows, 256, 0, s, a);
+            else launch_after(composite_kernel<kOutFringePreview, true, false>, rows, 256, 0, s, a);
             break;
         case kOutSelection:
             if (rs) {
-                selection_max_kernel<true><<<a.H, 256, 0, s>>>(a);
-                composite_kernel<kOutSelection, false, true><<<rows, 256, 0, s>>>(a);
+                launch_after(selection_max_kernel<true>, a.H, 256, 0, s, a);
+                launch_after(composite_kernel<kOutSelection, false, true>, rows, 256, 0, s, a);
             } else {
-                selection_max_kernel<false><<<a.H, 256, 0, s>>>(a);
-                composite_kernel<kOutSelection, false, false><<<rows, 256, 0, s>>>(a);
+                launch_after(selection_max_kernel<false>, a.H, 256, 0, s, a);
+                launch_after(composite_kernel<kOutSelection, false, false>, rows, 256, 0, s, a);
             }
             break;
         default:
@@ -274,7 +275,7 @@ void launch_composite(const FrameArgs& a, cudaStream_t s) {
 
 void launch_resample_source(const FrameArgs& a, cudaStream_t s) {
     if (a.Ww <= 0 || a.Hw <= 0) return;
-    resample_source_kernel<<<dim3((a.Ww + 255) / 256, a.Hw), 256, 0, s>>>(a);
+    launch_after(resample_source_kernel, dim3((a.Ww + 255) / 256, a.Hw), 256, 0, s, a);
 }
 
 void launch_kspec_rows(const KernelSpectraArgs& a, cudaStream_t s) {

@@ -34,6 +34,7 @@
 #include "ld_async.cuh"
 #include "ld_fft.cuh"
 #include "ld_internal.h"
+#include "ld_launch.cuh"
 #include "ld_pixel.cuh"
 
 namespace ld {
@@ -279,6 +280,7 @@ __device__ __forceinline__ void fill_rows(const FrameArgs& a, int y0, int M, flo
 // to A[k][y0 + col / NDRV][col % NDRV].
 template <int E, int C, int NDRV, int MAXT = Fam<E>::max_threads, int MINB = 1, bool FROM_EFFECT = false>
 __global__ void __launch_bounds__(MAXT, MINB) frame_rows_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ float2 smem[];
     const int y0 = blockIdx.x * (C / NDRV);
     const int M = a.g.M;
@@ -302,6 +304,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_rows_kernel(FrameArgs a) {
 // kernel spectra land in the upper half of Wk and are widened in the multiply.
 template <int E, int NOUT, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
 __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     const int Py = a.g.Py, Hp = a.Hp, cols = a.g.cols;
     const int k = blockIdx.x;
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_cols_kernel(FrameArgs a) {
 // multiply by Kc, inverse, bulk store of the first Hp rows.
 template <int E>
 __global__ void __launch_bounds__(Fam<E>::max_threads, 1) frame_cols_mono_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     const int Py = a.g.Py, Hp = a.Hp, cols = a.g.cols;
     const int k = blockIdx.x;
@@ -580,6 +584,7 @@ __device__ __forceinline__ void inverse_epilogue(const FrameArgs& a, const Inver
 // One row per CTA (inverse_row); smem M * C float2 (C = n_out interleaved channels).
 template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
 __global__ void __launch_bounds__(MAXT, MINB) frame_inverse_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ float2 smem[];
     const InverseRow w = inverse_row(a);
     const bool have = w.have;
@@ -637,6 +642,7 @@ __global__ void __launch_bounds__(MAXT, MINB) frame_inverse_kernel(FrameArgs a) 
 // Luma sums of the redistributed source and of the stored effect over the
 // whole source frame (field zones with Preserve energy); one source row per CTA.
 __global__ void __launch_bounds__(256) effect_sums_kernel(FrameArgs a) {
+    stream_order();
     const int sy = blockIdx.x;
     const bool aligned_s = ((reinterpret_cast<uintptr_t>(a.src) | static_cast<uintptr_t>(a.src_pitch)) & 15) == 0;
     const unsigned char* srow = a.src + static_cast<int64_t>(sy) * a.src_pitch;
@@ -733,6 +739,7 @@ __device__ __forceinline__ float3 tap_value(const FrameArgs& a, int x, int y) {
 // (makeDebugFromScalar, :1370-1389; *a.mask_max from selection_max_kernel).
 template <int MODE, bool FRINGE, bool RESAMPLE>
 __global__ void __launch_bounds__(256) composite_kernel(FrameArgs a) {
+    stream_order();
     const int yo = a.out_y1 + blockIdx.x;
     const int sy = yo - a.src_y1;
     const bool have = sy >= 0 && sy < a.H;
@@ -808,6 +815,7 @@ __global__ void __launch_bounds__(256) composite_kernel(FrameArgs a) {
 // *a.mask_max as float bits; one source row per CTA.
 template <bool RESAMPLE>
 __global__ void __launch_bounds__(256) selection_max_kernel(FrameArgs a) {
+    stream_order();
     const int sy = blockIdx.x;
     const bool aligned_s = ((reinterpret_cast<uintptr_t>(a.src) | static_cast<uintptr_t>(a.src_pitch)) & 15) == 0;
     const unsigned char* srow = a.src + static_cast<int64_t>(sy) * a.src_pitch;
@@ -846,6 +854,7 @@ __global__ void __launch_bounds__(256) selection_max_kernel(FrameArgs a) {
 // bilinearly, zero outside [0, W-1] x [0, H-1] (resampleRgbaImage
 // :414-434 with sampleRgbaBilinearImage :373-395).
 __global__ void __launch_bounds__(256) resample_source_kernel(FrameArgs a) {
+    stream_order();
     const int y = blockIdx.y;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.Ww) return;
@@ -888,6 +897,7 @@ __device__ __forceinline__ int canvas_index(int g, int P, int R) {
 // KR[k][i][c], k < M + 1.
 template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1>
 __global__ void __launch_bounds__(MAXT, MINB) kspec_rows_kernel(KernelSpectraArgs a) {
+    stream_order();
     extern __shared__ float2 smem[];
     const int i = blockIdx.x;
     const int Px = a.g.Px, R = a.R, K = a.K;
@@ -910,6 +920,7 @@ __global__ void __launch_bounds__(MAXT, MINB) kspec_rows_kernel(KernelSpectraArg
 // one bulk store.
 template <int E, int C, int MAXT = Fam<E>::max_threads, int MINB = 1, bool H16 = false>
 __global__ void __launch_bounds__(MAXT, MINB) kspec_cols_kernel(KernelSpectraArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     const int Py = a.g.Py, cols = a.g.cols, Kp = a.Kp, R = a.R;
     const int k = blockIdx.x;

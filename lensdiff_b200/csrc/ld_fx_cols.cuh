@@ -79,6 +79,7 @@ constexpr ColsShape cols_shape() {
 //   1201 columns of 1152: 29 us FP32 (72)
 template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int N = P::n;
     ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
 // runtime-planned transforms), the scatter's 1001 of 1200 35 us (60).
 template <class P, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_frame_cols_mono_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int N = P::n, C = 3;
     ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_mono_kernel(FrameArgs a
 // see above), 4097 of 5120 284 us (517), 1126 of 1800 28 us (66).
 template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int N = P::n;
     ColsHeader* h = reinterpret_cast<ColsHeader*>(smraw);
@@ -283,7 +286,7 @@ void frame_cols_fx(FrameArgs a, cudaStream_t s) {
     auto f = fx_frame_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
     constexpr size_t sm = cols_bytes(P::n, C);
     a.ahead = state.get(f, sh.threads, sm);
-    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+    launch_after(f, a.g.cols, sh.threads, sm, s, a);
 }
 
 template <class P>
@@ -293,7 +296,7 @@ void frame_cols_mono_fx(FrameArgs a, cudaStream_t s) {
     auto f = fx_frame_cols_mono_kernel<P, sh.threads, sh.ctas>;
     constexpr size_t sm = cols_bytes(P::n, 3);
     a.ahead = state.get(f, sh.threads, sm);
-    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+    launch_after(f, a.g.cols, sh.threads, sm, s, a);
 }
 
 template <class P, int C, bool H16>
@@ -305,7 +308,7 @@ bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
     const size_t sm = kColsHeader + (static_cast<size_t>(P::n) + a.Kp) * C * sizeof(float2);
     if (sm > kSmemOptIn) return false;
     a.ahead = state.get(f, sh.threads, cols_bytes(P::n, C));
-    f<<<a.g.cols, sh.threads, sm, s>>>(a);
+    launch_after(f, a.g.cols, sh.threads, sm, s, a);
     return true;
 }
 

@@ -143,6 +143,7 @@ __device__ __forceinline__ int window_index(int k, int x0, int half, int S) {
 // bound by issue: the fields' sine and cosine and the transform.
 template <class P, int C, int NZ, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_psf_rows_kernel(PsfBankArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int S = P::n;
     float2* s = reinterpret_cast<float2*>(smraw);
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(T, MINB) fx_psf_rows_kernel(PsfBankArgs a) {
 // Windows of 236-413 columns of 2048 for 31 wavelengths take 55 us (215).
 template <class P, int C, int NZ, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_psf_cols_kernel(PsfBankArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int S = P::n;
     float2* s = reinterpret_cast<float2*>(smraw);
@@ -226,12 +228,12 @@ void psf_launch(const PsfBankArgs& a, bool rows, cudaStream_t s) {
         static KernelState state;
         auto f = fx_psf_rows_kernel<P, C, NZ, sh.threads, sh.ctas>;
         state.get(f, sh.threads, sm);
-        f<<<dim3((a.row_n + C - 1) / C, a.B), sh.threads, sm, s>>>(a);
+        launch_after(f, dim3((a.row_n + C - 1) / C, a.B), sh.threads, sm, s, a);
     } else {
         static KernelState state;
         auto f = fx_psf_cols_kernel<P, C, NZ, sh.threads, sh.ctas>;
         state.get(f, sh.threads, sm);
-        f<<<dim3((a.win_stride + C - 1) / C, a.B), sh.threads, sm, s>>>(a);
+        launch_after(f, dim3((a.win_stride + C - 1) / C, a.B), sh.threads, sm, s, a);
     }
 }
 

@@ -192,6 +192,7 @@ struct Mirror {
 // instruction fetches (142 us for 2160 rows of 2500, against 88 before).
 template <class P, int C, int NDRV, bool FROM_EFFECT, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_frame_rows_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int M = P::n;
     float* part = reinterpret_cast<float*>(smraw);
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_rows_kernel(FrameArgs a) {
 // 361 us (475, runtime-planned), 620 of 1125 24 us (52).
 template <class P, int C, bool H16, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_frame_inverse_kernel(FrameArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int M = P::n;
     float2* s = reinterpret_cast<float2*>(smraw + kRowsHeader);
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_inverse_kernel(FrameArgs a) 
 // 2500 take 54 us (64 before), 1502 of 4096 158 us (214), 1026 of 1125 24 us (75).
 template <class P, int C, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_kspec_rows_kernel(KernelSpectraArgs a) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smraw[];
     constexpr int M = P::n;
     float2* s = reinterpret_cast<float2*>(smraw + kRowsHeader);
@@ -308,7 +311,7 @@ void frame_rows_fx(FrameArgs a, cudaStream_t s) {
     auto f = fx_frame_rows_kernel<P, C, NDRV, FROM_EFFECT, sh.threads, sh.ctas>;
     const size_t sm = kRowsHeader + static_cast<size_t>(P::n) * C * sizeof(float2);
     a.ahead = state.get(f, sh.threads, sm);
-    f<<<a.Hp / (C / NDRV), sh.threads, sm, s>>>(a);
+    launch_after(f, a.Hp / (C / NDRV), sh.threads, sm, s, a);
 }
 
 template <class P, int C, bool H16>
@@ -319,7 +322,7 @@ void frame_inverse_fx(FrameArgs a, int rows, cudaStream_t s) {
     auto f = fx_frame_inverse_kernel<P, C, H16, sh.threads, sh.ctas>;
     const size_t sm = kRowsHeader + static_cast<size_t>(P::n) * C * sizeof(float2);
     a.ahead = state.get(f, sh.threads, sm);
-    f<<<rows, sh.threads, sm, s>>>(a);
+    launch_after(f, rows, sh.threads, sm, s, a);
 }
 
 template <class P, int C>
@@ -330,7 +333,7 @@ void kspec_rows_fx(const KernelSpectraArgs& a, cudaStream_t s) {
     auto f = fx_kspec_rows_kernel<P, C, sh.threads, sh.ctas>;
     const size_t sm = kRowsHeader + static_cast<size_t>(P::n) * C * sizeof(float2);
     state.get(f, sh.threads, sm);
-    f<<<a.Kp, sh.threads, sm, s>>>(a);
+    launch_after(f, a.Kp, sh.threads, sm, s, a);
 }
 
 // The launch of plan P named by `pass`; false for the Mono and luma-lock chains

@@ -24,6 +24,7 @@
 #include "ld_async.cuh"
 #include "ld_fft.cuh"
 #include "ld_internal.h"
+#include "ld_launch.cuh"
 
 namespace ld {
 

@@ -23,6 +23,7 @@
 #include "../../include/lensdiff_b200.h"
 #include "ld_fxplans.h"
 #include "ld_internal.h"
+#include "ld_launch.cuh"
 
 using namespace ld;
 
@@ -259,6 +260,7 @@ constexpr int kBigStages = 8;
 // round trip.
 constexpr int kHostWordsThreads = 1024;
 __global__ void __launch_bounds__(kHostWordsThreads) host_words_kernel(uint32_t* dst, const uint32_t* src, int words) {
+    stream_order();
     int i0 = 0;
     if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
         const int q = words / 4;
@@ -315,8 +317,8 @@ void upload_async(ld_ctx* c, void* dst, const void* src, size_t bytes, cudaStrea
     std::memcpy(h, src, bytes);
     void* hd = nullptr;
     check_cuda(cudaHostGetDevicePointer(&hd, h, 0), what);
-    host_words_kernel<<<1, kHostWordsThreads, 0, s>>>(static_cast<uint32_t*>(dst), static_cast<const uint32_t*>(hd),
-                                                       static_cast<int>(bytes / 4));
+    launch_after(host_words_kernel, 1, kHostWordsThreads, 0, s, static_cast<uint32_t*>(dst),
+                 static_cast<const uint32_t*>(hd), static_cast<int>(bytes / 4));
     check_launch(what);
     ++c->launches;
     check_cuda(cudaEventRecord(c->stage_ev[static_cast<size_t>(i)], s), what);
@@ -2337,6 +2339,7 @@ void run_chain(ld_ctx* c, cudaStream_t s, const std::string& key, const std::fun
         return;
     }
     try {
+        LaunchScope scope(true);
         chain();
     } catch (...) {
         cudaGraph_t g = nullptr;
@@ -3233,6 +3236,7 @@ int run_guarded(ld_ctx* ctx, ld_status* st, const std::function<void()>& fn) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     DeviceGuard g(ctx->device);
     CustomScope custom(&ctx->custom);
+    LaunchScope launches(false);
     try {
         fn();
     } catch (const Fail& f) {

@@ -21,6 +21,7 @@
 #include <climits>
 
 #include "ld_internal.h"
+#include "ld_launch.cuh"
 
 namespace ld {
 namespace {
@@ -99,6 +100,7 @@ __device__ __forceinline__ void warp_runs_accumulate(int slot, float v, float to
 
 // ---- pupil, once per bank --------------------------------------------------------
 __global__ void __launch_bounds__(256) pupil_pre_kernel(PsfBankArgs a) {
+    stream_order();
     const int n = a.pupil.size;
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n * n) return;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) pupil_pre_kernel(PsfBankArgs a) {
 // window columns are written by the drain.
 template <int E>
 __global__ void __launch_bounds__(E >= kE25 ? kE25MaxThreads : kE16MaxThreads, 1) psf_rows_kernel(PsfBankArgs a) {
+    stream_order();
     extern __shared__ float2 smem[];
     const int yr = blockIdx.x;
     const int y = a.row_lo + yr;
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(E >= kE25 ? kE25MaxThreads : kE16MaxThreads, 1
 // that can be non-zero are read, |F|^2 of the window rows is written.
 template <int E, int C>
 __global__ void __launch_bounds__(E >= kE25 ? kE25MaxThreads : kE16MaxThreads, 1) psf_cols_kernel(PsfBankArgs a) {
+    stream_order();
     extern __shared__ float2 smem[];
     const int b = blockIdx.y;
     const WavelengthInfo* w = a.wl + b;
@@ -630,6 +634,7 @@ struct ResampleGrid {
 };
 template <bool FUSED>
 __global__ void __launch_bounds__(256) resample_kernel(PsfBankArgs a, ResampleGrid g) {
+    stream_order();
     extern __shared__ float2 smem[];
     int i = blockIdx.x;
     if (i < g.nq) {
@@ -667,6 +672,7 @@ __device__ double mean_kernel_sum(const double* ring, const int* count, int R, d
 // normalised azimuthal mean of every round(r) ring, once per wavelength, for
 // shape_stats_kernel to read.
 __global__ void __launch_bounds__(256) ring_mean_kernel(PsfBankArgs a) {
+    stream_order();
     const int b = blockIdx.x;
     const int R = a.R;
     const double s1 = a.scalars[b].s1;
@@ -682,6 +688,7 @@ __global__ void __launch_bounds__(256) ring_mean_kernel(PsfBankArgs a) {
 // of a canvas that resample_kernel<true> filled (the unnormalised resampled
 // kernel), for the ring means of the Split look.
 __global__ void __launch_bounds__(256) ring_sums_kernel(PsfBankArgs a) {
+    stream_order();
     __shared__ float ring[kRingSpanTall];
     const int b = blockIdx.z;
     const int K = a.K, R = a.R;
@@ -717,6 +724,7 @@ __global__ void __launch_bounds__(256) ring_sums_kernel(PsfBankArgs a) {
 // written in place, its sum, and its ring energy / peak by ceil(r)
 // (estimateAdaptiveSupportRadius, :984-1007).
 __global__ void __launch_bounds__(256) shape_stats_kernel(PsfBankArgs a) {
+    stream_order();
     __shared__ float ring_e[kRingSpanTall];
     __shared__ unsigned int ring_p[kRingSpanTall];
     __shared__ float mean_r[kRingSpanTall];
@@ -791,6 +799,7 @@ __global__ void __launch_bounds__(256) shape_stats_kernel(PsfBankArgs a) {
 // Suffix maxima of the ring peaks and prefix sums of the ring energies are
 // block scans over per-thread chunks of rings.
 __global__ void __launch_bounds__(256) support_kernel(PsfBankArgs a) {
+    stream_order();
     __shared__ float chunk_max[256];
     __shared__ double chunk_sum[256];
     __shared__ int first_hit;
@@ -909,6 +918,7 @@ __device__ __forceinline__ int isqrt_floor(int v) {  // floor(sqrt(v)), v >= 0
 }
 
 __global__ void __launch_bounds__(256) crop_sum_kernel(PsfBankArgs a) {
+    stream_order();
     const int b = blockIdx.y;
     const PsfScalars& sc = a.scalars[b];
     const int rho = sc.radius;
@@ -957,6 +967,7 @@ __global__ void __launch_bounds__(256) crop_sum_kernel(PsfBankArgs a) {
 // s_core = sum of mean * taper, s_struct = sum of max(0, shaped * taper / s3
 // - mean * taper) over the crop box.
 __global__ void __launch_bounds__(256) split_sums_kernel(PsfBankArgs a) {
+    stream_order();
     const int b = blockIdx.z;
     const PsfScalars& sc = a.scalars[b];
     const float inv_s3 = static_cast<float>(1.0 / sc.s3);
@@ -1011,6 +1022,7 @@ struct CombineBin {
 // NK: output kernels (1 Mono, 3 spectral, 4 with the luma lock; Split: 4).
 template <bool SPLIT, int NK>
 __global__ void __launch_bounds__(256) combine_kernel(CombineArgs a) {
+    stream_order();
     __shared__ CombineBin bin[kMaxBins];
     const int tid = threadIdx.x + threadIdx.y * 32;
     const int B = a.bank.B;
@@ -1275,13 +1287,14 @@ __global__ void normalize_psf_kernel(float* psf, int64_t n, const PsfScalars* sc
 template <int E>
 void rows_launch(const PsfBankArgs& a, cudaStream_t s) {
     dim3 grid(a.row_n, a.B);
-    psf_rows_kernel<E><<<grid, fft_threads(a.S, 1, E), a.S * sizeof(float2), s>>>(a);
+    launch_after(psf_rows_kernel<E>, grid, fft_threads(a.S, 1, E), a.S * sizeof(float2), s, a);
 }
 
 template <int E, int C>
 void cols_launch(const PsfBankArgs& a, cudaStream_t s) {
     dim3 grid((a.win_stride + C - 1) / C, a.B);
-    psf_cols_kernel<E, C><<<grid, fft_threads(a.S, C, E), static_cast<size_t>(a.S) * C * sizeof(float2), s>>>(a);
+    launch_after(psf_cols_kernel<E, C>, grid, fft_threads(a.S, C, E), static_cast<size_t>(a.S) * C * sizeof(float2), s,
+                 a);
 }
 
 dim3 tall_grid(const PsfBankArgs& a) {
@@ -1301,7 +1314,7 @@ void opt_in(Kern k, size_t bytes) {
 
 void launch_pupil_pre(const PsfBankArgs& a, cudaStream_t s) {
     const int n = a.pupil.size * a.pupil.size;
-    pupil_pre_kernel<<<(n + 255) / 256, 256, 0, s>>>(a);
+    launch_after(pupil_pre_kernel, (n + 255) / 256, 256, 0, s, a);
 }
 
 void launch_psf_rows(const PsfBankArgs& a, cudaStream_t s) {
@@ -1351,36 +1364,36 @@ void launch_resample(const PsfBankArgs& a, bool filtered, float inv_max, cudaStr
         sm = std::max(sm, sizeof(FilterSmem));
         grid += g.fx * g.fy * a.B;
     }
-    if (fused_shaping(a)) resample_kernel<true><<<grid, dim3(32, 8), sm, s>>>(a, g);
-    else resample_kernel<false><<<grid, dim3(32, 8), sm, s>>>(a, g);
+    if (fused_shaping(a)) launch_after(resample_kernel<true>, grid, dim3(32, 8), sm, s, a, g);
+    else launch_after(resample_kernel<false>, grid, dim3(32, 8), sm, s, a, g);
 }
 
 void launch_shape_stats(const PsfBankArgs& a, cudaStream_t s) {
-    ring_mean_kernel<<<a.B, 256, 0, s>>>(a);
-    shape_stats_kernel<<<tall_grid(a), dim3(32, 8), 0, s>>>(a);
+    launch_after(ring_mean_kernel, a.B, 256, 0, s, a);
+    launch_after(shape_stats_kernel, tall_grid(a), dim3(32, 8), 0, s, a);
 }
 
 void launch_ring_means(const PsfBankArgs& a, cudaStream_t s) {
-    ring_sums_kernel<<<tall_grid(a), dim3(32, 8), 0, s>>>(a);
-    ring_mean_kernel<<<a.B, 256, 0, s>>>(a);
+    launch_after(ring_sums_kernel, tall_grid(a), dim3(32, 8), 0, s, a);
+    launch_after(ring_mean_kernel, a.B, 256, 0, s, a);
 }
 
-void launch_support(const PsfBankArgs& a, cudaStream_t s) { support_kernel<<<a.B, 256, 0, s>>>(a); }
+void launch_support(const PsfBankArgs& a, cudaStream_t s) { launch_after(support_kernel, a.B, 256, 0, s, a); }
 
 void launch_crop_sum(const PsfBankArgs& a, cudaStream_t s) {
-    crop_sum_kernel<<<dim3((a.R + kCropRows) / kCropRows, a.B), 256, 0, s>>>(a);
+    launch_after(crop_sum_kernel, dim3((a.R + kCropRows) / kCropRows, a.B), 256, 0, s, a);
 }
 
 void launch_split_sums(const PsfBankArgs& a, cudaStream_t s) {
-    split_sums_kernel<<<canvas_grid(a, a.B), dim3(32, 8), 0, s>>>(a);
+    launch_after(split_sums_kernel, canvas_grid(a, a.B), dim3(32, 8), 0, s, a);
 }
 
 void launch_combine(const CombineArgs& a, cudaStream_t s) {
     const dim3 grid((a.bank.R + 32) / 32, (a.bank.R + 8) / 8), block(32, 8);
-    if (a.split) combine_kernel<true, 4><<<grid, block, 0, s>>>(a);
-    else if (a.n_ker == 1) combine_kernel<false, 1><<<grid, block, 0, s>>>(a);
-    else if (a.n_ker == 3) combine_kernel<false, 3><<<grid, block, 0, s>>>(a);
-    else combine_kernel<false, 4><<<grid, block, 0, s>>>(a);
+    if (a.split) launch_after(combine_kernel<true, 4>, grid, block, 0, s, a);
+    else if (a.n_ker == 1) launch_after(combine_kernel<false, 1>, grid, block, 0, s, a);
+    else if (a.n_ker == 3) launch_after(combine_kernel<false, 3>, grid, block, 0, s, a);
+    else launch_after(combine_kernel<false, 4>, grid, block, 0, s, a);
 }
 
 void launch_export(const PsfBankArgs& a, const int64_t* offsets_dev, float* out, cudaStream_t s) {
