@@ -345,11 +345,15 @@ def algorithmic_bytes(W, H, grid, n_drv, n_ker, n_out, out_pixels, B=0, K=0, h16
     out_spec = cplx * H * bins
     canvas = 4 * B * K * K
     Kp = K + (K & 1)
+    R = K // 2
+    fade = min(R, max(6.0, min(24.0, 0.04 * R)))
     return {
         # bank passes over the B canvases of K x K floats (written once by the
         # lambda-rescale, which also takes the shaping statistics; read by the
-        # crop sums and the combination)
-        "resample": canvas, "shape_stats": 2 * canvas, "crop_sum": canvas,
+        # combination); the crop sums read the annulus under the taper, at most
+        # that of the full radius
+        "resample": canvas, "shape_stats": 2 * canvas,
+        "crop_sum": int(4 * B * math.pi * (R * R - (R - fade) ** 2)),
         "combine": canvas + 4 * n_ker * K * K,
         "kspec_rows": 4 * n_ker * K * K + 8 * n_ker * Kp * bins,
         "kspec_cols": 8 * n_ker * Kp * bins + cplx * n_ker * Py * bins,

@@ -149,7 +149,8 @@ class LensDiffPsfBankCache:
         return int(w.value)
 
     def set_graphs(self, enable: bool) -> None:
-        """Replay per-frame chains as CUDA graphs (default on)."""
+        """Capture per-frame chains as CUDA graphs on their second use and
+        replay them (default on)."""
         self._lib.ld_set_graphs(self._h, 1 if enable else 0)
 
     def set_autotune(self, mode: int) -> None:
@@ -163,7 +164,7 @@ class LensDiffPsfBankCache:
 
     def autotune_choice(self, n: int):
         """(radix order, launch shape, ms) the autotuner chose for transform
-        length n, or None."""
+        length n, or None (launch shape: 0, every order has one)."""
         r = (abi.c_i32 * 4)()
         shape = abi.c_i32(0)
         ms = ctypes.c_double(0.0)
