@@ -281,26 +281,25 @@ class Clocks:
                 "samples": len(sms)}
 
 
-# DRAM read + write per launch (bytes, median over the run's launches; the
-# lambda-rescale's pair and single-wavelength launches of one bank summed) of the
+# DRAM read + write per launch (bytes, median over the run's launches) of the
 # UHD 31-wavelength cold workload's kernels, by transform form, from one
 # one-pass ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # kernel sources whose digest is TRAFFIC_SOURCES_SHA (sources_digest()).  Any
 # other revision of the kernels reports traffic null: a figure measured on
 # other code says nothing about this code.  Writes still resident in L2 when a
 # kernel ends are not counted.
-TRAFFIC_SOURCES_SHA = "d7f4cd7799c9133d"
+TRAFFIC_SOURCES_SHA = "4d4f7172ff0be248"
 MEASURED_TRAFFIC_UHD31 = {
     "chosen": {
-        "resample": 78053376,
-        "crop_sum": 40304640,
-        "combine": 132500224,
-        "kspec_rows": 19684864,
-        "kspec_cols": 105022976,
-        "frame_rows": 140078848,
-        "frame_cols": 146548480,
-        "frame_inverse": 291208192,
-        "dft_gemm": 56408320,
+        "resample": 82423936,
+        "crop_sum": 15454592,
+        "combine": 132561024,
+        "kspec_rows": 22846720,
+        "kspec_cols": 103238144,
+        "frame_rows": 138003072,
+        "frame_cols": 144797824,
+        "frame_inverse": 323565184,
+        "dft_gemm": 56079872,
     },
 }
 
