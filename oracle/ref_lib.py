@@ -22,7 +22,7 @@ def build(force: bool = False) -> bool:
     """Compiles the reference shim when the reference sources are present."""
     if os.path.exists(REF_LIB) and not force:
         return True
-    if not REF_ROOT or not os.path.isdir(REF_ROOT):
+    if not REF_ROOT or not os.path.isdir(os.path.join(REF_ROOT, "source", "src", "core")):
         return False
     subprocess.run(["make", "-C", HERE, f"REF={REF_ROOT}"], check=True,
                    stdout=subprocess.DEVNULL)
