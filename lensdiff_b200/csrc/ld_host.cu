@@ -1363,6 +1363,7 @@ void bank_geometry(ld_ctx* c, PsfBankArgs& a, const ld_params& p, int S, int R) 
     a.K = 2 * R + 1;
     a.gain = 1.0f + std::max(0.0f, static_cast<float>(p.anisotropy_emphasis)) * 4.0f;  // :1127
     a.count_round = ring_counts(c, R);
+    a.h16 = chosen_h16(p) ? 1 : 0;
 }
 
 // The bank of `p`: the context's bank or a bank of the last lens set when

@@ -67,6 +67,7 @@ struct PsfBankArgs {
     const int* count_round;      // [R+1] pixel counts by round(r)
     PsfScalars* scalars;         // [B]
     int want_energy;
+    int h16;                     // the FP16 form: a bank with a box filter is sampled tap by tap (ld_psf.cu)
 };
 
 void launch_pupil_pre(const PsfBankArgs& a, cudaStream_t s);

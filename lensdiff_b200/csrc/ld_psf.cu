@@ -651,6 +651,211 @@ __global__ void __launch_bounds__(256) resample_kernel(PsfBankArgs a, ResampleGr
     }
 }
 
+// ---- lambda-rescale of the FP16 form's banks with a box filter ------------------
+// The FP16 form rounds its kernel spectra to half, where a canvas that differs
+// in FP32's last bits moves stored values to their neighbours: with
+// resample_filtered's separable weights in place of the tap-by-tap mean, and
+// the statistics that scale the kernel summed in another order, a small
+// log-encoded frame moved by 7e-5 of its norm, at the same error against FP64.
+// A bank with a box filter is therefore sampled tap by tap, and summed, over
+// 32 x 128 tiles, one wavelength a tile: 186 us for 16 wavelengths at K = 513
+// with footprints 3.3-5.7 (71 us separably).  (A bank without one moves by
+// less than its own float atomics moved it here: resample_quad.)
+// sampleSquareBilinear (LensDiffCpuReference.cpp:316-336) reading the |F|^2
+// window; the window covers every pixel the kernel touches.
+__device__ __forceinline__ float sample_bilinear(const Window& w, float x, float y) {
+    const float lim = static_cast<float>(w.S - 1);
+    if (x < 0.0f || y < 0.0f || x > lim || y > lim) return 0.0f;
+    const int x0 = static_cast<int>(floorf(x));
+    const int y0 = static_cast<int>(floorf(y));
+    const int x1 = min(x0 + 1, w.S - 1);
+    const int y1 = min(y0 + 1, w.S - 1);
+    const float tx = x - static_cast<float>(x0);
+    const float ty = y - static_cast<float>(y0);
+    const int hi = w.n - 1;
+    const int ax0 = min(max(x0 - w.x0, 0), hi), ax1 = min(max(x1 - w.x0, 0), hi);
+    const int ay0 = min(max(y0 - w.x0, 0), hi), ay1 = min(max(y1 - w.x0, 0), hi);
+    const float v00 = w.p[static_cast<size_t>(ay0) * w.stride + ax0];
+    const float v10 = w.p[static_cast<size_t>(ay0) * w.stride + ax1];
+    const float v01 = w.p[static_cast<size_t>(ay1) * w.stride + ax0];
+    const float v11 = w.p[static_cast<size_t>(ay1) * w.stride + ax1];
+    const float vx0 = v00 + (v10 - v00) * tx;
+    const float vx1 = v01 + (v11 - v01) * tx;
+    return vx0 + (vx1 - vx0) * ty;
+}
+
+// sampleSquareFiltered (LensDiffCpuReference.cpp:338-353)
+__device__ __forceinline__ float sample_filtered(const Window& w, float x, float y, float footprint, int taps,
+                                                 float step) {
+    float sum = 0.0f;
+    for (int ty = 0; ty < taps; ++ty) {
+        const float oy = (static_cast<float>(ty) + 0.5f) * step - footprint * 0.5f;
+        for (int tx = 0; tx < taps; ++tx) {
+            const float ox = (static_cast<float>(tx) + 0.5f) * step - footprint * 0.5f;
+            sum += sample_bilinear(w, x + ox, y + oy);
+        }
+    }
+    return sum / static_cast<float>(taps * taps);
+}
+
+// sample_bilinear with the column half precomputed (identical arithmetic).
+__device__ __forceinline__ float sample_row(const Window& w, const ColTap& c, float y) {
+    if (!c.in || y < 0.0f || y > static_cast<float>(w.S - 1)) return 0.0f;
+    const int y0 = static_cast<int>(floorf(y));
+    const int y1 = min(y0 + 1, w.S - 1);
+    const float ty = y - static_cast<float>(y0);
+    const int hi = w.n - 1;
+    const float* r0 = w.p + min(max(y0 - w.x0, 0), hi) * w.stride;
+    const float* r1 = w.p + min(max(y1 - w.x0, 0), hi) * w.stride;
+    const float v00 = __ldg(r0 + c.ax0), v10 = __ldg(r0 + c.ax1);
+    const float v01 = __ldg(r1 + c.ax0), v11 = __ldg(r1 + c.ax1);
+    const float vx0 = v00 + (v10 - v00) * c.tx;
+    const float vx1 = v01 + (v11 - v01) * c.tx;
+    return vx0 + (vx1 - vx0) * ty;
+}
+
+// Window pixels staged per tile of unfiltered samples (at most one window pixel
+// apart), one more on each side so that the span holds whatever the rounding
+// of the sample positions.
+constexpr int kStageW = kTile + 4, kStageH = kTallH + 4;
+
+// Rows / columns of the window that canvas coordinates c0 .. c1 sample
+// (sample_bilinear's x0 .. x1 of the first and last sample, clamped to the
+// window as it clamps them): [lo, hi] in window indices.
+__device__ __forceinline__ void stage_span(const Window& w, float rc, float kc, float inv, int c0, int c1, int* lo,
+                                           int* hi) {
+    const float p0 = rc + (static_cast<float>(c0) - kc) * inv;
+    const float p1 = rc + (static_cast<float>(c1) - kc) * inv;
+    const int whi = w.n - 1;
+    const int a0 = static_cast<int>(floorf(fmaxf(p0, 0.0f)));
+    const int a1 = min(static_cast<int>(floorf(fminf(fmaxf(p1, 0.0f), static_cast<float>(w.S - 1)))) + 1, w.S - 1);
+    *lo = min(max(a0 - 1 - w.x0, 0), whi);
+    *hi = min(max(a1 + 1 - w.x0, 0), whi);
+}
+
+// Statistics of one tile, and the window pixels it samples.
+template <bool FUSED>
+struct TileSmem {
+    RingSmem<FUSED> rings;
+    float stage[kStageH][kStageW];
+};
+
+// The window pixels (rows cy0.., columns cx0..) a staged tile samples.
+struct StageBox {
+    int cx0, cy0, sw, sh;
+};
+
+// The staged box of wavelength `w`'s window for the tile at (tx0, ty0);
+// ok = false when the samples are box-filtered or the span is too wide.
+__device__ __forceinline__ bool stage_box(const Window& w, float rc, float kc, float inv, int taps, int tx0, int ty0,
+                                          int K, StageBox* b) {
+    if (taps != 0) return false;
+    int cx1 = -1, cy1 = -1;
+    stage_span(w, rc, kc, inv, tx0, min(tx0 + kTile, K) - 1, &b->cx0, &cx1);
+    stage_span(w, rc, kc, inv, ty0, min(ty0 + kTallH, K) - 1, &b->cy0, &cy1);
+    b->sw = cx1 - b->cx0 + 1;
+    b->sh = cy1 - b->cy0 + 1;
+    return b->sw <= kStageW && b->sh <= kStageH;
+}
+
+__device__ __forceinline__ void stage_load(const Window& w, const StageBox& b, float (*stage)[kStageW], int tid) {
+    for (int i = tid; i < b.sw * b.sh; i += 256) {
+        const int r = i / b.sw, c = i - r * b.sw;
+        stage[r][c] = __ldg(w.p + static_cast<size_t>(b.cy0 + r) * w.stride + b.cx0 + c);
+    }
+}
+
+// sample_row's arithmetic on staged pixels: the bilinear sample at window
+// row coordinate yy of the column tap ct (sx0, sx1: its columns in the box).
+__device__ __forceinline__ float staged_sample(const Window& w, const ColTap& ct, int sx0, int sx1, int cy0,
+                                              const float (*stage)[kStageW], bool in, float yy) {
+    const float lim = static_cast<float>(w.S - 1);
+    if (!(in && ct.in && !(yy < 0.0f || yy > lim))) return 0.0f;
+    const int hi = w.n - 1;
+    const int y0 = static_cast<int>(floorf(yy));
+    const int y1 = min(y0 + 1, w.S - 1);
+    const float ty = yy - static_cast<float>(y0);
+    const int sy0 = min(max(y0 - w.x0, 0), hi) - cy0;
+    const int sy1 = min(max(y1 - w.x0, 0), hi) - cy0;
+    const float v00 = stage[sy0][sx0], v10 = stage[sy0][sx1];
+    const float v01 = stage[sy1][sx0], v11 = stage[sy1][sx1];
+    const float vx0 = v00 + (v10 - v00) * ct.tx;
+    const float vx1 = v01 + (v11 - v01) * ct.tx;
+    return vx0 + (vx1 - vx0) * ty;
+}
+
+// One wavelength's 32 x 128 canvas tile; block (32, 8), 16 rows per thread.
+// Unfiltered wavelengths of the bank stage the window pixels the tile reads in
+// shared memory (stage_box); box-filtered samples, and any span too wide to
+// stage, read the window directly.
+template <bool FUSED>
+__device__ void resample_tile(const PsfBankArgs& a, int b, int rbase, TileSmem<FUSED>& sm, int tid) {
+    sm.rings.clear(tid);
+    const WavelengthInfo* wi = a.wl + b;
+    const int K = a.K, R = a.R;
+    const int tx0 = blockIdx.x * kTile, ty0 = blockIdx.y * kTallH;
+    const Window w{a.win + static_cast<size_t>(b) * a.win_stride * a.win_stride, a.win_stride, wi->win_x0,
+                   wi->win_n, a.S};
+    const float kc = static_cast<float>(K - 1) * 0.5f;
+    const float inv = wi->inv_scale;
+    const int taps = wi->taps;
+    const float step = wi->step;
+    const float rc = a.raw_center;
+    float* canvas = a.canvas + static_cast<size_t>(b) * K * K;
+    float lsum = 0.0f;  // this thread's pixels; one double add per thread at the flush
+    unsigned int lpeak = 0u;
+    const int x = tx0 + threadIdx.x;
+    const bool in = x < K;
+    const float dx = static_cast<float>(x) - kc;
+    StageBox bx;
+    if (stage_box(w, rc, kc, inv, taps, tx0, ty0, K, &bx)) {  // uniform per CTA
+        stage_load(w, bx, sm.stage, tid);
+        __syncthreads();
+        const ColTap ct = col_tap(w, rc + dx * inv);
+        const int sx0 = ct.ax0 - bx.cx0, sx1 = ct.ax1 - bx.cx0;
+#pragma unroll 4
+        for (int i = 0; i < kTallH / 8; ++i) {
+            const int y = ty0 + threadIdx.y + 8 * i;
+            if (y >= K) break;  // uniform: a warp is one canvas row
+            const float dy = static_cast<float>(y) - kc;
+            const float v = staged_sample(w, ct, sx0, sx1, bx.cy0, sm.stage, in, rc + dy * inv);
+            if (in) canvas[static_cast<size_t>(y) * K + x] = v;
+            lsum += v;
+            if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
+            warp_runs_accumulate<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v, v, sm.rings.ring, sm.rings.ring_p);
+        }
+    } else {
+        __syncthreads();
+        const ColTap ct = col_tap(w, rc + dx * inv);
+#pragma unroll 4
+        for (int i = 0; i < kTallH / 8; ++i) {
+            const int y = ty0 + threadIdx.y + 8 * i;
+            if (y >= K) break;  // uniform: a warp is one canvas row (the last tile row is mostly past K)
+            const float dy = static_cast<float>(y) - kc;
+            float v = 0.0f;
+            if (in) {
+                v = taps == 0 ? sample_row(w, ct, rc + dy * inv)
+                              : sample_filtered(w, rc + dx * inv, rc + dy * inv, inv, taps, step);
+                canvas[static_cast<size_t>(y) * K + x] = v;
+                lsum += v;
+                if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
+            }
+            warp_runs_accumulate<FUSED>(ring_slot<FUSED>(in, dx, dy, R, rbase), v, v, sm.rings.ring, sm.rings.ring_p);
+        }
+    }
+    resample_flush<FUSED>(a, b, rbase, sm.rings, lsum, lpeak, tid);
+}
+
+// grid (ceil(K/32), ceil(K/128), B), block (32, 8): wavelength blockIdx.z.
+template <bool FUSED>
+__global__ void __launch_bounds__(256) resample_tile_kernel(PsfBankArgs a) {
+    stream_order();
+    __shared__ TileSmem<FUSED> sm;
+    const int tid = threadIdx.x + threadIdx.y * 32;
+    const int rbase = tile_ring_base(blockIdx.x * kTile, blockIdx.y * kTallH, a.R, a.R, kTallH);
+    resample_tile<FUSED>(a, blockIdx.z, rbase, sm, tid);
+}
+
 // Sum over rings of the unnormalised azimuthal mean, i.e. the normaliser of
 // azimuthalMeanKernel: sum_r count[r] * (ring[r] / s1) / count[r].
 __device__ double mean_kernel_sum(const double* ring, const int* count, int R, double s1) {
@@ -1343,6 +1548,12 @@ bool fused_shaping(const PsfBankArgs& a) { return a.gain == 1.0f; }
 // would take over 25 KB and cost resident CTAs (inv_max > 0.5), 16 where 64
 // rows would not give every SM two CTAs.
 void launch_resample(const PsfBankArgs& a, bool filtered, float inv_max, cudaStream_t s) {
+    const dim3 tall = tall_grid(a);
+    if (filtered && a.h16) {
+        if (fused_shaping(a)) launch_after(resample_tile_kernel<true>, tall, dim3(32, 8), 0, s, a);
+        else launch_after(resample_tile_kernel<false>, tall, dim3(32, 8), 0, s, a);
+        return;
+    }
     ResampleGrid g{};
     size_t sm = 0;
     int grid = 0;
@@ -1357,7 +1568,6 @@ void launch_resample(const PsfBankArgs& a, bool filtered, float inv_max, cudaStr
         grid = g.nq;
     }
     if (filtered) {
-        const dim3 tall = tall_grid(a);
         g.fth = tall.x * tall.y * tall.z < 148 ? 16 : kTile;
         g.fx = tall.x;
         g.fy = (a.K + g.fth - 1) / g.fth;
