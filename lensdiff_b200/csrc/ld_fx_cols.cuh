@@ -24,29 +24,31 @@ constexpr size_t cols_bytes(int n, int C) { return kColsHeader + static_cast<siz
 // with the most useful element slots in flight per SM.  A stage of radix
 // R keeps ceil(C n / R / T) butterflies of R values per thread in registers
 // (at most 32 values); a thread needs 80 registers, and each CTA its share of
-// shared memory (cols_bytes).
+// shared memory (cols_bytes).  ORD: the FP16 form's passes.
 struct ColsShape {
     int threads, ctas;
 };
-template <class P, int C>
+template <class P, int C, bool ORD>
 constexpr ColsShape cols_shape() {
-    const int radix[3] = {P::R1, P::R2, P::R3};
+    const int radix[4] = {ORD ? P::ord.radix(0) : P::R1, ORD ? P::ord.radix(1) : P::R2,
+                          ORD ? P::ord.radix(2) : P::R3, ORD ? P::ord.radix(3) : 0};
+    const int count = ORD ? P::ord.count : 3;
     ColsShape best{0, 0};
     double score = -1.0;
     for (int t = 32; t <= 800; t += 32) {
         int steps = 0;
         bool fits = true;
-        for (int r : radix) {
-            const int it = (C * P::n / r + t - 1) / t;
-            steps += it * r;
-            if (it * r > 32) fits = false;
+        for (int i = 0; i < count; ++i) {
+            const int it = (C * P::n / radix[i] + t - 1) / t;
+            steps += it * radix[i];
+            if (it * radix[i] > 32) fits = false;
         }
         const int by_smem = static_cast<int>((228 * 1024) / (cols_bytes(P::n, C) + 1024));
         const int by_regs = 65536 / (80 * t);
         int ctas = by_smem < by_regs ? by_smem : by_regs;
         if (ctas > 8) ctas = 8;
         if (!fits || ctas < 1) continue;
-        const double s = 3.0 * C * P::n / steps * ctas;  // useful slots per SM
+        const double s = static_cast<double>(count) * C * P::n / steps * ctas;  // useful slots per SM
         if (s > score) {
             score = s;
             best = ColsShape{t, ctas};
@@ -54,6 +56,35 @@ constexpr ColsShape cols_shape() {
     }
     return best;
 }
+
+// The forward passes of the column's order from I on, over the column in F
+// (pass 1 on) and the free half of W in turn (one barrier a pass), ending in
+// F; an even number of passes takes the first of them in place.
+template <class P, int T, int I>
+__device__ __forceinline__ void ord_column(const float2* __restrict__ tw, float2* F, float2* W) {
+    if constexpr (I < P::ord.count) {
+        constexpr bool left_even = (P::ord.count - I) % 2 == 0;
+        constexpr bool in_place = !left_even && I == 1;
+        const float2* from = left_even || in_place ? F : W;
+        float2* to = left_even ? W : F;
+        ord_pass<P, 1, T, false, I, in_place>(
+            tw, [&](int e) { return from[e]; }, [&](int e, float2 v) { to[e] = v; });
+        if constexpr (I + 1 < P::ord.count) __syncthreads();
+        ord_column<P, T, I + 1>(tw, F, W);
+    }
+}
+
+// The last pass of a column transform (H16: of the FP16 form's order).
+template <class P, int C, int T, bool INV, bool H16>
+struct ColsLastOf {
+    using type = LastStage<P::n, C, T, INV, P::R3>;
+};
+template <class P, int C, int T, bool INV>
+struct ColsLastOf<P, C, T, INV, true> {
+    using type = OrdLast<P, C, T, INV>;
+};
+template <class P, int C, int T, bool INV, bool H16>
+using ColsLast = typename ColsLastOf<P, C, T, INV, H16>::type;
 
 // Column k = blockIdx.x: its row spectra transformed, multiplied by its C (3 or,
 // with the luma lock, 4) kernel spectra, the products transformed back, the
@@ -118,12 +149,11 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
     auto stW = [&](int e, float2 v) { W[e] = v; };
     const float2 zero = make_float2(0.0f, 0.0f);
     if constexpr (H16) {
-        fp_stage<N, 1, T, false, P::R1, 1, false>(
-            nullptr, [&](int e) { return e < Hp ? from_half2(ah[e], exp2_int(aex[e])) : zero; }, stF);
+        const float2* otw = ord_table<P, C == 3>(tw);
+        ord_pass<P, 1, T, false, 0, false>(
+            otw, [&](int e) { return e < Hp ? from_half2(ah[e], exp2_int(aex[e])) : zero; }, stF);
         __syncthreads();
-        fp_stage<N, 1, T, false, P::R2, P::R1, false>(tw + P::tab2, ldF, stW);
-        __syncthreads();
-        fp_stage<N, 1, T, false, P::R3, P::R1 * P::R2, false>(tw + P::tab3, ldW, stF);
+        ord_column<P, T, 1>(otw, F, W);
     } else {
         fp_stage<N, 1, T, false, P::R1, 1, true>(nullptr, [&](int e) { return e < Hp ? F[e] : zero; }, stF);
         __syncthreads();
@@ -132,13 +162,21 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
         fp_stage<N, 1, T, false, P::R3, P::R1 * P::R2, true>(tw + P::tab3, ldF, stF);
     }
     if (__syncthreads_or(!mbar_wait(&h->bar[1], 0, a.err))) return;
-    fp_stage<N, C, T, true, P::R1, 1, true>(
-        nullptr, [&](int e) { return cmul(H16 ? __half22float2(kh[e]) : W[e], F[e / C]); }, stW);
-    __syncthreads();
-    fp_stage<N, C, T, true, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
-    __syncthreads();
-    LastStage<N, C, T, true, P::R3> last;
-    last.run(tw + P::tab3, ldW);
+    ColsLast<P, C, T, true, H16> last;
+    if constexpr (H16) {
+        const float2* otw = ord_table<P, C == 3>(tw);
+        const float ks = a.kscale[k];
+        ord_pass<P, C, T, true, 0, true>(otw, [&](int e) { return cmul(from_half2(kh[e], ks), F[e / C]); }, stW);
+        __syncthreads();
+        ord_middle<P, C, T, true>(otw, W);
+        last.run(otw + P::ord.table(P::ord.count - 1), ldW);
+    } else {
+        fp_stage<N, C, T, true, P::R1, 1, true>(nullptr, [&](int e) { return cmul(W[e], F[e / C]); }, stW);
+        __syncthreads();
+        fp_stage<N, C, T, true, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+        __syncthreads();
+        last.run(tw + P::tab3, ldW);
+    }
     // element e = row * C + c of column k goes to B's group of four columns
     const int64_t base = (static_cast<int64_t>(k / kBGroup) * Hp * kBGroup + k % kBGroup) * C;
     constexpr int step = kBGroup * C;
@@ -149,8 +187,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
         });
         m = cta_max<T>(m, h->part);
         const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
-        // the kernel spectra's own scale joins the outputs' here
-        if (threadIdx.x == 0) a.bscale[k] = (m > 0.0f ? m / kHalfTop : 1.0f) * a.kscale[k];
+        if (threadIdx.x == 0) a.bscale[k] = m > 0.0f ? m / kHalfTop : 1.0f;
         __half2* out = reinterpret_cast<__half2*>(a.Bout) + base;
         last.each([&](int e, float2 v) {
             const int row = e / C;
@@ -249,26 +286,33 @@ __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArg
     auto ldW = [&](int e) { return W[e]; };
     auto stW = [&](int e, float2 v) { W[e] = v; };
     // grid row v holds canvas row v + R (v <= R) or v - N + R (v >= N - R)
-    fp_stage<N, C, T, false, P::R1, 1, false>(
-        nullptr,
-        [&](int e) {
-            const int lo = e + C * R, hi = e - C * (N - R);
-            if (e < C * (R + 1)) return Rb[lo];
-            if (hi >= 0) return Rb[hi];
-            return make_float2(0.0f, 0.0f);
-        },
-        stW);
-    __syncthreads();
-    fp_stage<N, C, T, false, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
-    __syncthreads();
-    LastStage<N, C, T, false, P::R3> last;
-    last.run(tw + P::tab3, ldW);
+    auto ldR = [&](int e) {
+        const int lo = e + C * R, hi = e - C * (N - R);
+        if (e < C * (R + 1)) return Rb[lo];
+        if (hi >= 0) return Rb[hi];
+        return make_float2(0.0f, 0.0f);
+    };
+    ColsLast<P, C, T, false, H16> last;
+    if constexpr (H16) {
+        const float2* otw = ord_table<P, C == 3>(tw);
+        const float scale = a.scale;
+        ord_pass<P, C, T, false, 0, false>(otw, [&](int e) { return cscale(ldR(e), scale); }, stW);
+        __syncthreads();
+        ord_middle<P, C, T, false>(otw, W);
+        last.run(otw + P::ord.table(P::ord.count - 1), ldW);
+    } else {
+        fp_stage<N, C, T, false, P::R1, 1, false>(nullptr, ldR, stW);
+        __syncthreads();
+        fp_stage<N, C, T, false, P::R2, P::R1, true>(tw + P::tab2, ldW, stW);
+        __syncthreads();
+        last.run(tw + P::tab3, ldW);
+    }
     if constexpr (H16) {
         float m = 0.0f;
         last.each([&](int, float2 v) { m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))); });
         m = cta_max<T>(m, h->part);
         const float sc = m > 0.0f ? kHalfTop / m : 1.0f;
-        if (threadIdx.x == 0) a.kscale[k] = m > 0.0f ? m / kHalfTop * a.scale : 1.0f;
+        if (threadIdx.x == 0) a.kscale[k] = m > 0.0f ? m / kHalfTop : 1.0f;
         __half2* out = reinterpret_cast<__half2*>(a.spectra) + static_cast<size_t>(k) * N * C;
         last.each([&](int e, float2 v) { out[e] = to_half2(v, sc); });
     } else {
@@ -280,7 +324,7 @@ __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArg
 
 template <class P, int C, bool H16>
 void frame_cols_fx(FrameArgs a, cudaStream_t s) {
-    constexpr ColsShape sh = cols_shape<P, C>();
+    constexpr ColsShape sh = cols_shape<P, C, H16>();
     static_assert(sh.threads > 0);
     static KernelState state;
     auto f = fx_frame_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
@@ -291,7 +335,7 @@ void frame_cols_fx(FrameArgs a, cudaStream_t s) {
 
 template <class P>
 void frame_cols_mono_fx(FrameArgs a, cudaStream_t s) {
-    constexpr ColsShape sh = cols_shape<P, 3>();
+    constexpr ColsShape sh = cols_shape<P, 3, false>();
     static KernelState state;
     auto f = fx_frame_cols_mono_kernel<P, sh.threads, sh.ctas>;
     constexpr size_t sm = cols_bytes(P::n, 3);
@@ -301,7 +345,7 @@ void frame_cols_mono_fx(FrameArgs a, cudaStream_t s) {
 
 template <class P, int C, bool H16>
 bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
-    constexpr ColsShape sh = cols_shape<P, C>();
+    constexpr ColsShape sh = cols_shape<P, C, H16>();
     static_assert(sh.threads > 0);
     static KernelState state;
     auto f = fx_kspec_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
@@ -312,29 +356,40 @@ bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
     return true;
 }
 
-// The launch of plan P: the frame's column pass (fa) or the kernel spectra's
-// (ka); false when it does not fit, and for the Mono and luma-lock chains at
-// lengths above kFxOtherMax, which stay on the runtime-planned transforms.
-template <class P>
-bool cols_launch(const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
-    if (fa && fa->n_drv == 1 && fa->n_out == 3) {
-        if (fa->h16) frame_cols_fx<P, 3, true>(*fa, s);
-        else frame_cols_fx<P, 3, false>(*fa, s);
+// The FP16 form's launch, where the plan has an order.
+template <class P, int C>
+bool cols_launch_h16(const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
+    if constexpr (P::ord.count > 0) {
+        if (ka) return kspec_cols_fx<P, C, true>(*ka, s);
+        frame_cols_fx<P, C, true>(*fa, s);
         return true;
     }
-    if (ka && ka->n_ker == 3) return ka->h16 ? kspec_cols_fx<P, 3, true>(*ka, s) : kspec_cols_fx<P, 3, false>(*ka, s);
+    return false;
+}
+
+// The launch of plan P: the frame's column pass (fa) or the kernel spectra's
+// (ka); false when it does not fit, for the Mono and luma-lock chains at
+// lengths above kFxOtherMax, and in the FP16 form where the plan has no order:
+// those stay on the runtime-planned transforms.
+template <class P>
+bool cols_launch(const FrameArgs* fa, const KernelSpectraArgs* ka, cudaStream_t s) {
+    const bool h16 = fa ? fa->h16 != 0 : ka->h16 != 0;
+    if (fa ? fa->n_drv == 1 && fa->n_out == 3 : ka->n_ker == 3) {
+        if (h16) return cols_launch_h16<P, 3>(fa, ka, s);
+        if (ka) return kspec_cols_fx<P, 3, false>(*ka, s);
+        frame_cols_fx<P, 3, false>(*fa, s);
+        return true;
+    }
     if constexpr (P::n <= kFxOtherMax) {
         if (fa && fa->n_drv == 3) {
             frame_cols_mono_fx<P>(*fa, s);
             return true;
         }
-        if (fa) {
-            if (fa->h16) frame_cols_fx<P, 4, true>(*fa, s);
-            else frame_cols_fx<P, 4, false>(*fa, s);
-            return true;
-        }
-        if (ka->n_ker == 1) return kspec_cols_fx<P, 1, false>(*ka, s);
-        return ka->h16 ? kspec_cols_fx<P, 4, true>(*ka, s) : kspec_cols_fx<P, 4, false>(*ka, s);
+        if (ka && ka->n_ker == 1) return kspec_cols_fx<P, 1, false>(*ka, s);
+        if (h16) return cols_launch_h16<P, 4>(fa, ka, s);
+        if (ka) return kspec_cols_fx<P, 4, false>(*ka, s);
+        frame_cols_fx<P, 4, false>(*fa, s);
+        return true;
     }
     return false;
 }

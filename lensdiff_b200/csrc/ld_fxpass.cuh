@@ -23,6 +23,7 @@
 
 #include "ld_async.cuh"
 #include "ld_fft.cuh"
+#include "ld_fxorder.h"
 #include "ld_internal.h"
 #include "ld_launch.cuh"
 
@@ -135,9 +136,9 @@ __device__ __forceinline__ void fdft(float2* v) {
 }
 
 // ---- stages ---------------------------------------------------------------------
-// Twiddles and transforms one butterfly of span offset k (NS = 1: no twiddles).
+// The twiddles of one butterfly of span offset k (NS = 1: none).
 template <bool INV, int R, int NS>
-__device__ __forceinline__ void fp_butterfly(float2* v, int k, const float2* __restrict__ stw) {
+__device__ __forceinline__ void fp_twiddle(float2* v, int k, const float2* __restrict__ stw) {
     if constexpr (NS > 1) {
         const float4* t = reinterpret_cast<const float4*>(stw) + k;
 #pragma unroll
@@ -150,12 +151,61 @@ __device__ __forceinline__ void fp_butterfly(float2* v, int k, const float2* __r
             }
         }
     }
-    fdft<R, INV>(v);
 }
+
+// How a stage takes a butterfly of span offset k.  FastStage: the radices of
+// ld_fxplans.h.
+struct FastStage {
+    template <bool INV, int R, int NS>
+    static __device__ __forceinline__ void run(float2* v, int k, const float2* __restrict__ stw) {
+        fp_twiddle<INV, R, NS>(v, k, stw);
+        fdft<R, INV>(v);
+    }
+};
+// A pass of ld_fxorder.h: the stage of radix A over span NS and (B > 1) the
+// stage of radix B over span NS * A after it, with the arithmetic of
+// ld_fft.cuh.  The B butterflies j, j + N / (A B), .. of the first (inputs r
+// = B r1 + r2) feed the A butterflies of span offsets k1 NS + k of the second.
+template <int A, int B>
+struct OrderStage {
+    template <bool INV, int R, int NS>
+    static __device__ __forceinline__ void run(float2* v, int k, const float2* __restrict__ stw) {
+        static_assert(R == A * B);
+        if constexpr (B == 1) {
+            fp_twiddle<INV, A, NS>(v, k, stw);
+            dft<A, INV>(v);
+        } else {
+#pragma unroll
+            for (int r2 = 0; r2 < B; ++r2) {
+                float2 t[A];
+#pragma unroll
+                for (int r1 = 0; r1 < A; ++r1) t[r1] = v[B * r1 + r2];
+                fp_twiddle<INV, A, NS>(t, k, stw);
+                dft<A, INV>(t);
+#pragma unroll
+                for (int k1 = 0; k1 < A; ++k1) v[B * k1 + r2] = t[k1];
+            }
+            const float2* second = stw + FxOrder::stage(NS, A);
+            float2 o[R];
+#pragma unroll
+            for (int k1 = 0; k1 < A; ++k1) {
+                float2 t[B];
+#pragma unroll
+                for (int r2 = 0; r2 < B; ++r2) t[r2] = v[B * k1 + r2];
+                fp_twiddle<INV, B, NS * A>(t, k1 * NS + k, second);
+                dft<B, INV>(t);
+#pragma unroll
+                for (int k2 = 0; k2 < B; ++k2) o[k1 + A * k2] = t[k2];
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = o[r];
+        }
+    }
+};
 
 // One stage: ld(e) gives element e, st(e, value) takes it; SYNC: a CTA barrier
 // between the last load and the first store (the two share a buffer).
-template <int N, int C, int T, bool INV, int R, int NS, bool SYNC, class Ld, class St>
+template <int N, int C, int T, bool INV, int R, int NS, bool SYNC, class Stage = FastStage, class Ld, class St>
 __device__ __forceinline__ void fp_stage(const float2* __restrict__ stw, Ld ld, St st) {
     constexpr int NB = N / R * C;
     constexpr int IT = (NB + T - 1) / T;
@@ -172,7 +222,7 @@ __device__ __forceinline__ void fp_stage(const float2* __restrict__ stw, Ld ld, 
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
         const int b = tid + it * T;
-        if ((it + 1) * T <= NB || b < NB) fp_butterfly<INV, R, NS>(v[it], (b / C) % NS, stw);
+        if ((it + 1) * T <= NB || b < NB) Stage::template run<INV, R, NS>(v[it], (b / C) % NS, stw);
     }
     if constexpr (SYNC) __syncthreads();
 #pragma unroll
@@ -190,7 +240,7 @@ __device__ __forceinline__ void fp_stage(const float2* __restrict__ stw, Ld ld, 
 
 // The last stage, kept in the thread's registers: v[it][r] is element
 // tid + it * T + r * NB where that butterfly exists.
-template <int N, int C, int T, bool INV, int R>
+template <int N, int C, int T, bool INV, int R, class Stage = FastStage>
 struct LastStage {
     static constexpr int NB = N / R * C;
     static constexpr int IT = (NB + T - 1) / T;
@@ -211,7 +261,7 @@ struct LastStage {
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int b = static_cast<int>(threadIdx.x) + it * T;
-            if (has(it)) fp_butterfly<INV, R, N / R>(v[it], b / C, stw);
+            if (has(it)) Stage::template run<INV, R, N / R>(v[it], b / C, stw);
         }
     }
     // f(e, value) for every element the thread holds
@@ -228,14 +278,45 @@ struct LastStage {
     }
 };
 
-// A three-stage transform length.
+// A three-stage transform length; ord: the FP16 form's order.
 template <int R1_, int R2_, int R3_>
 struct Fx3 {
     static constexpr int R1 = R1_, R2 = R2_, R3 = R3_;
     static constexpr int n = R1 * R2 * R3;
-    // stage tables follow one another: the second stage's, then the third's
+    // stage tables follow one another: the second stage's, then the third's,
+    // then the order's (fx_stage_table in ld_frame_fx.cu)
     static constexpr int tab2 = 0, tab3 = R1 * FxPad<R2>::value;
+    static constexpr int tab_ord = tab3 + R1 * R2 * FxPad<R3>::value;
+    static constexpr FxOrder ord = fx_col_order(R1, R2, R3);
+    static constexpr bool table_twiddles = fx_table_twiddles(false, n);
 };
+
+// Where the order's twiddles lie: by products, then (lengths that have them)
+// from the table, which the spectral chain takes.
+template <class P, bool SPECTRAL>
+__device__ __forceinline__ const float2* ord_table(const float2* stw) {
+    return stw + P::tab_ord + (SPECTRAL && P::table_twiddles ? P::ord.table() : 0);
+}
+
+// Pass I of P's order.
+template <class P, int I>
+using OrdStage = OrderStage<P::ord.a[I], P::ord.b[I]>;
+template <class P, int C, int T, bool INV, int I, bool SYNC, class Ld, class St>
+__device__ __forceinline__ void ord_pass(const float2* __restrict__ tw, Ld ld, St st) {
+    fp_stage<P::n, C, T, INV, P::ord.radix(I), P::ord.span(I), SYNC, OrdStage<P, I>>(tw + P::ord.table(I), ld, st);
+}
+// The passes from I to the one before the last, in place in s, a barrier after each.
+template <class P, int C, int T, bool INV, int I = 1>
+__device__ __forceinline__ void ord_middle(const float2* __restrict__ tw, float2* s) {
+    if constexpr (I < P::ord.count - 1) {
+        ord_pass<P, C, T, INV, I, true>(tw, [&](int e) { return s[e]; }, [&](int e, float2 v) { s[e] = v; });
+        __syncthreads();
+        ord_middle<P, C, T, INV, I + 1>(tw, s);
+    }
+}
+// The last pass, in registers.
+template <class P, int C, int T, bool INV>
+using OrdLast = LastStage<P::n, C, T, INV, P::ord.radix(P::ord.count - 1), OrdStage<P, P::ord.count - 1>>;
 
 // Largest m over the CTA of T threads (every thread gets it); `part`: a shared
 // array of at least T / 32 floats, nobody's until the next barrier.

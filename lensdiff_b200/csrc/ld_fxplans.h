@@ -30,7 +30,7 @@ struct FxPlanDesc {
 // ld_fx_cols0.cu .. ld_fx_cols5.cu compile.
 #define LD_FX_COLS_0(X) \
     X(20, 5, 5, 12) X(26, 5, 10, 10) X(32, 9, 8, 10) X(38, 25, 5, 8) X(44, 9, 9, 16) \
-    X(50, 15, 10, 12) X(56, 25, 10, 10) X(62, 25, 8, 16) X(68, 12, 16, 24)
+    X(50, 15, 10, 12) X(56, 25, 10, 10) X(62, 25, 16, 8) X(68, 12, 16, 24)
 #define LD_FX_COLS_1(X) \
     X(21, 5, 8, 8) X(27, 8, 8, 8) X(33, 3, 16, 16) X(39, 8, 8, 16) X(45, 9, 10, 16) \
     X(51, 15, 8, 16) X(57, 20, 8, 16) X(63, 9, 24, 16) X(69, 25, 12, 16)
@@ -45,7 +45,7 @@ struct FxPlanDesc {
     X(54, 15, 9, 16) X(60, 25, 8, 15) X(66, 16, 16, 16) X(72, 15, 15, 24)
 #define LD_FX_COLS_5(X) \
     X(25, 5, 8, 12) X(31, 9, 8, 9) X(37, 15, 8, 8) X(43, 5, 16, 16) X(49, 9, 12, 16) \
-    X(55, 9, 16, 16) X(61, 25, 16, 8) X(67, 15, 12, 24)
+    X(55, 9, 16, 16) X(61, 25, 8, 16) X(67, 15, 12, 24)
 // Row plans X(id, R1, R2, R3), in the groups of ld_fx_rows0.cu .. ld_fx_rows5.cu.
 #define LD_FX_ROWS_0(X) \
     X(100, 8, 8, 4) X(106, 5, 10, 9) X(112, 5, 16, 8) X(118, 9, 10, 10) X(124, 25, 10, 5) \
