@@ -984,7 +984,7 @@ def main():
         roofline = {"bound": "hbm", "kernel": dominant, "achieved": None, "peak": peak, "unit": "GB/s",
                     "frac": None, "peak_source": peak_src, "traffic": None}
     stage_ms = {k: round(v[0] / n_prof, 4) for k, v in stage.items() if v[1]}
-    # the radix orders and launch shapes the autotuner picked for the grid
+    # the radix orders that the grid's lengths run on
     autotune = {}
     for n in (grid[0] // 2, grid[1]):
         ch = cache.autotune_choice(n)

@@ -247,25 +247,25 @@ enum {
  * stream is being captured.  No counterpart in the reference. */
 int ld_set_graphs(ld_ctx* ctx, int enable);
 
-/* Autotuner of the frame chain's transforms.  The row length M and column
- * length Py of a frame grid can each run on one of several compiled radix
- * orders (ld_fxplans.h).  With autotuning on (the default), the first frame
- * rendered at a grid, when it composites directly (no field zones, Preserve
- * energy or scatter) and the caller's stream is not being captured, times
- * every order of both lengths on that frame's own buffers with CUDA events
- * (the timed kernels rewrite the same results) and keeps the fastest for
- * later frames of the context: that first frame synchronises its stream a
- * few times.  mode 1: tune (the default); 0: the first compiled order of each
- * length; 2 + k (k <= 7): the k-th compiled order of each length (its last
- * when it has fewer), for tests and offline tuning; -1: the
- * runtime-planned transforms only, no compiled orders.  No counterpart in
- * the reference. */
+/* The radix orders of the frame chain's transforms.  The row length M and
+ * column length Py of a frame grid each run on a compiled radix order
+ * (ld_fxplans.h); column lengths 1600 and 3200 have two.  mode 1 (the
+ * default): the frame chain's own order (frames that composite directly,
+ * without field zones, Split, Preserve energy or scatter, take the last,
+ * others the first); 0: the first compiled order of each length; 2 + k
+ * (k <= 7): the k-th compiled order of each length (its last when it has
+ * fewer), for tests; -1: the runtime-planned transforms only, no compiled
+ * orders.  Nothing is timed on the caller's frames, so no mode launches
+ * more or waits.  No counterpart in the reference. */
 int ld_set_autotune(ld_ctx* ctx, int mode);
-/* The radix order chosen for transform length n: writes up to 4 radices
+/* The radix order that transform length n runs on: writes up to 4 radices
  * (first stage first) and returns how many, 0 when n has no compiled order
- * or has not been tuned yet.  *shape_out (may be null): the launch shape, 0
- * (every order runs in the shape compiled for it).  *ms_out (may be null): the
- * winner's time per tuned launch group. */
+ * or no frame has composited directly on it in mode 1 yet (for a length that
+ * is a grid's row and column length: the column order where it has two, else
+ * the row order).  *shape_out (may be null): the launch shape, 0 (every order
+ * runs in the shape compiled for it).  *ms_out (may be null): the duration of
+ * the first such frame's column pass, or inverse row pass; reading it waits
+ * for that pass. */
 int ld_autotune_choice(ld_ctx* ctx, int32_t n, int32_t* radices_out, int32_t* shape_out, double* ms_out);
 
 /* The Custom aperture mode's image (LD_APERTURE_CUSTOM).  The reference

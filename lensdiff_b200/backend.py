@@ -154,17 +154,17 @@ class LensDiffPsfBankCache:
         self._lib.ld_set_graphs(self._h, 1 if enable else 0)
 
     def set_autotune(self, mode: int) -> None:
-        """1: time the compiled radix orders of a new grid's transform lengths
-        on its first composite frame and keep the fastest (the default); 0: the
-        first compiled order; 2 + k: the k-th compiled order of each length
+        """1: each frame chain's compiled radix order (the default); 0:
+        the first compiled order; 2 + k: the k-th compiled order of each length
         (its last when it has fewer); -1: runtime-planned transforms only."""
         rc = self._lib.ld_set_autotune(self._h, int(mode))
         if rc != abi.LD_OK:
             raise ValueError(f"autotune mode {mode!r} rejected ({rc})")
 
     def autotune_choice(self, n: int):
-        """(radix order, launch shape, ms) the autotuner chose for transform
-        length n, or None (launch shape: 0, every order has one)."""
+        """(radix order, launch shape, ms of its first pass) of transform length
+        n, or None before a frame composited directly on it (launch shape: 0,
+        every order has one)."""
         r = (abi.c_i32 * 4)()
         shape = abi.c_i32(0)
         ms = ctypes.c_double(0.0)

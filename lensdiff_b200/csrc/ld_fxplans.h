@@ -1,15 +1,16 @@
 // ld_fxplans.h — the transform lengths and radix orders compiled as fixed
-// plans, shared by the host (planning, twiddle tables, the autotuner's
-// candidate lists) and the kernels' translation units.
+// plans, shared by the host (planning, twiddle tables) and the kernels'
+// translation units.
 //
 // Row plans (length M, half the grid's width: ld_fx_rows*.cu) and column plans
 // (length Py: ld_fx_cols*.cu) run on ld_fxpass.cuh.  Every length that the
 // grid's cost model (choose_length in ld_host.cu) picks for the spectral
-// chains has one: columns from 300 to 5400, rows from 256 to 4096.  Where a
-// length has several orders the autotuner times them on first use and keeps
-// the fastest (the first is the default).  Odd radices lead where the length
-// has them: their strided first-stage stores spread over the shared-memory
-// banks.  A row plan's last radix is also its inverse's first, and is taken in
+// chains has one: columns from 300 to 5400, rows from 256 to 4096.  Column
+// lengths 1600 and 3200 have two orders: frames that composite directly run the
+// second, others the first.  (They are within 3 % of one another; an order that
+// changes moves the FP16 form's results by up to 2e-5, so each chain keeps the
+// one it has always had.)  Odd radices lead where the length has them: their
+// strided first-stage stores spread over the shared-memory banks.  A row plan's last radix is also its inverse's first, and is taken in
 // pairs of mirrored butterflies: a small one.  PSF plans (length S:
 // ld_fx_psf*.cu) cover the common PSF sizes; their first radix is a multiple
 // of four, whose transforms drop the zero half of the embedded pupil.

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/lensdiff_b200.h"
+#include "ld_fxorder.h"
 #include "ld_fxplans.h"
 #include "ld_internal.h"
 #include "ld_launch.cuh"
@@ -91,10 +92,15 @@ struct ld_ctx {
     std::mutex mu;
     std::map<int, DevBuf> twiddles;
     std::map<int, DevBuf> stage_twiddles;  // by fixed plan id
-    // (transform length, role) -> fixed plan id and the winner's timed ms (autotuner)
-    std::map<std::pair<int, int>, int> fixed_choice;
-    std::map<std::pair<int, int>, double> fixed_ms;
-    int autotune = 1;  // 1: tune, 0: first compiled order, -1: runtime-planned transforms only
+    // (transform length, role) -> the fixed plan of its first composite frame and
+    // the events around that frame's launch on it
+    struct PlanUse {
+        int id;
+        bool h16;
+        cudaEvent_t e0, e1;
+    };
+    std::map<std::pair<int, int>, PlanUse> plan_use;
+    int autotune = 1;  // 1: each chain's order, 0: first compiled order, -1: runtime-planned transforms only
     int fail_alloc_after = -1;  // fault injection: allocations until one fails (-1: off)
     CustomAperture custom;      // the Custom aperture mode's image
     std::map<std::pair<int, int>, float> r0_cache;
@@ -485,27 +491,25 @@ const float2* stage_twiddles(ld_ctx* c, int id) {
     return static_cast<const float2*>(b.p);
 }
 
-// The fixed plan a length runs on: the autotuner's choice when it has made
-// one, else the first compiled radix order of that length (0: none).
-// Mode 2 + k pins the k-th compiled order of every length (its last when it
-// has fewer).
-int fixed_plan_for(ld_ctx* c, int n, int role) {
+// The fixed plan a length runs on (0: none): the first compiled radix order,
+// or (mode 1, `composite`) the last: see LD_FX_COLS in ld_fxplans.h.  Mode 2 + k
+// pins the k-th compiled order of every length (its last when it has fewer).
+int fixed_plan_for(ld_ctx* c, int n, int role, bool composite) {
     if (role == 0 || c->autotune < 0) return 0;
     int ids[8];
     const int count = fx_candidates(n, role, ids, 8);
-    if (c->autotune >= 2) return count > 0 ? ids[std::min(c->autotune - 2, count - 1)] : 0;
-    auto it = c->fixed_choice.find({n, role});
-    if (it != c->fixed_choice.end()) return it->second;
-    return count > 0 ? ids[0] : 0;
+    if (count == 0) return 0;
+    const int k = c->autotune >= 2 ? c->autotune - 2 : (c->autotune == 1 && composite ? count - 1 : 0);
+    return ids[std::min(k, count - 1)];
 }
 
 // The plan of length n: runtime-planned stages, and the fixed plan of `role`
 // (0: none) when one is compiled.
-FftPlan make_plan(ld_ctx* c, int n, bool allow25, int role = 0) {
+FftPlan make_plan(ld_ctx* c, int n, bool allow25, int role = 0, bool composite = false) {
     FftPlan p{};
     if (!factor_plan(n, allow25, &p)) throw Fail{LD_ERR_UNSUPPORTED, "fft-length-not-5-smooth"};
     p.tw = twiddles(c, n);
-    p.fixed = fixed_plan_for(c, n, role);
+    p.fixed = fixed_plan_for(c, n, role, composite);
     p.stw = p.fixed ? stage_twiddles(c, p.fixed) : nullptr;
     return p;
 }
@@ -1585,8 +1589,9 @@ bool fx_chain(const ld_params& p) { return p.fft_form != LD_FFT_CUFFT; }
 // W+K-1 x H+K-1 gives the same linear convolution.  c_rows / c_cols: the
 // most interleaved sequences any row / column kernel of the chain transforms
 // (they pick the FFT family); fx: the compiled plans serve the chain
-// (fx_chain).
-GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, bool fx, int* req_w, int* req_h) {
+// (fx_chain); composite: a spectral chain that composites directly.
+GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, bool fx, bool composite, int* req_w,
+                       int* req_h) {
     GridGeom g{};
     *req_w = W + K - 1;
     *req_h = H + K - 1;
@@ -1600,8 +1605,8 @@ GridGeom make_geometry(ld_ctx* c, int W, int H, int K, int c_rows, int c_cols, b
     const int Kp = K + (K & 1);
     if (frame_cols_smem(g.Py, c_cols) > kSmemBudget || kspec_cols_smem(g.Py, Kp, c_cols) > kSmemBudget)
         throw Fail{LD_ERR_UNSUPPORTED, "frame-too-large-for-column-pass"};
-    g.plan_m = make_plan(c, g.M, g.fam_m == kE25, fx ? kFxRows : 0);
-    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25, fx ? kFxCols : 0);
+    g.plan_m = make_plan(c, g.M, g.fam_m == kE25, fx ? kFxRows : 0, composite);
+    g.plan_py = make_plan(c, g.Py, g.fam_py == kE25, fx ? kFxCols : 0, composite);
     g.tw_px = twiddles(c, g.Px);
     return g;
 }
@@ -2033,6 +2038,13 @@ SelectionParams selection_params(const ld_params& p) {  // CpuReference.cpp:1221
 
 int run_guarded(ld_ctx* ctx, ld_status* st, const std::function<void()>& fn);
 
+// Whether the inverse rows composite the frame themselves (kEffectComposite), from
+// three spectral kernels.
+bool composite_chain(const ld_params& p, const Combination& cb) {
+    return cb.parts == 1 && cb.n_drv == 1 && cb.n_out == 3 && !has_field_phase(p) &&
+           p.energy_mode != LD_ENERGY_PRESERVE && !post_effects(p).any() && p.debug_view == LD_DEBUG_FINAL;
+}
+
 // The combination and frame grid of the kernel spectra that ld_render uses
 // for a width x height source frame (the same resolution as the render's).
 struct SpectraGeometry {
@@ -2053,7 +2065,8 @@ SpectraGeometry spectra_geometry(ld_ctx* c, const ld_params& p, int W, int H) {
     const int c_rows = std::max(std::max(sg.cb.n_drv == 1 ? 4 : 3, sg.cb.n_out), sg.cb.n_ker);
     const int c_cols = std::max(std::max(sg.cb.n_out, sg.cb.n_ker), sg.cb.n_drv);
     int rw = 0, rh = 0;
-    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_chain(p), &rw, &rh);
+    sg.g = make_geometry(c, Ww, Hw, 2 * max_kernel_radius(p) + 1, c_rows, c_cols, fx_chain(p), composite_chain(p, sg.cb), &rw,
+                         &rh);
     sg.key = spectra_key_for(bank_key(p, wl), sg.cb, sg.g);
     const bool h16 = chosen_h16(p);
     sg.bytes = sg.cb.parts * (ks_part_bytes(sg.cb.n_ker, sg.g, h16) + static_cast<size_t>(sg.g.cols) * sizeof(float));
@@ -2126,6 +2139,8 @@ void ld_destroy(ld_ctx* c) {
                       &c->zone_wl, &c->zone_win, &c->zone_canvas, &c->zone_stats};
     c->cufft.release();
     for (DevBuf* b : bufs) free_buf(c, *b);
+    for (auto& u : c->plan_use)
+        for (cudaEvent_t e : {u.second.e0, u.second.e1}) cudaEventDestroy(e);
     for (cudaEvent_t e : c->event_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : c->stage_ev) cudaEventDestroy(e);
     if (c->fork_ev) cudaEventDestroy(c->fork_ev);
@@ -2234,68 +2249,64 @@ constexpr size_t kGraphCache = 4;
 constexpr size_t kGraphSeen = 4;  // covers the three spectra slots that a stream of new lenses rotates through
 
 // ---------------------------------------------------------------------------
-// Autotuner of the fixed transform plans (ld_fxplans.h)
+// The fixed transform plans in use (ld_fxplans.h)
 // ---------------------------------------------------------------------------
-// Times launch(id) for every compiled radix order of length n on stream s (one
-// untimed launch, then kTuneReps between two events; a single order one timed
-// launch) and records the fastest as c->fixed_choice[{n, role}].
-void tune_length(ld_ctx* c, int n, int role, cudaStream_t s, const std::function<void(int)>& launch) {
-    int ids[8];
-    const int k = fx_candidates(n, role, ids, 8);
-    if (k == 0 || c->fixed_choice.count({n, role})) return;
-    constexpr int kTuneReps = 3;
-    const int reps = k > 1 ? kTuneReps : 1;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    check_cuda(cudaEventCreate(&e0), "tune-event");
-    check_cuda(cudaEventCreate(&e1), "tune-event");
-    int best = ids[0];
-    float best_ms = 0.0f;
-    for (int i = 0; i < k; ++i) {
-        if (k > 1) launch(ids[i]);
-        check_cuda(cudaEventRecord(e0, s), "tune-record");
-        for (int r = 0; r < reps; ++r) launch(ids[i]);
-        check_cuda(cudaEventRecord(e1, s), "tune-record");
-        check_cuda(cudaEventSynchronize(e1), "tune-sync");
-        float ms = 0.0f;
-        check_cuda(cudaEventElapsedTime(&ms, e0, e1), "tune-elapsed");
-        ms /= static_cast<float>(reps);
-        if (i == 0 || ms < best_ms) {
-            best = ids[i];
-            best_ms = ms;
-        }
+// Brackets the column and inverse launches of a context's first composite frame
+// on each length's plan by events, for ld_autotune_choice: at(0) before the
+// column pass, at(1) between, at(2) after the inverse rows.  Nothing is
+// launched again and the host does not wait.
+class PlanNotes {
+public:
+    PlanNotes(ld_ctx* c, const GridGeom& g, bool composite, bool h16, cudaStream_t s) : c_(c), s_(s), h16_(h16) {
+        if (c->autotune != 1 || !composite) return;
+        note(g.Py, kFxCols, g.plan_py.fixed, &cols_);
+        note(g.M, kFxRows, g.plan_m.fixed, &rows_);
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    check_launch("autotune");
-    c->fixed_choice[{n, role}] = best;
-    c->fixed_ms[{n, role}] = best_ms;
-}
+    void at(int i) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if ((!cols_.id && !rows_.id) || cudaStreamIsCapturing(s_, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+            return;
+        if (i == 0) mark(&cols_.e0);
+        if (i == 1) mark(&cols_.e1);
+        if (i == 1) mark(&rows_.e0);
+        if (i == 2) mark(&rows_.e1);
+        if (i < 2) return;
+        keep(kFxCols, &cols_);
+        keep(kFxRows, &rows_);
+    }
+    ~PlanNotes() {
+        for (Note* n : {&cols_, &rows_})
+            for (cudaEvent_t e : {n->e0, n->e1})
+                if (e) cudaEventDestroy(e);
+    }
+    PlanNotes(const PlanNotes&) = delete;
+    PlanNotes& operator=(const PlanNotes&) = delete;
 
-// Tunes the row length (frame_rows + frame_inverse, which share its plan) and
-// the column length (frame_cols) of a composite frame's grid, re-running the
-// frame's own launches: each rewrites the results it wrote before.
-void autotune_frame(ld_ctx* c, const FrameArgs& fa, cudaStream_t s) {
-    if (c->autotune != 1 || fa.effect_mode != kEffectComposite || fa.n_drv != 1 || fa.n_out != 3) return;
-    if (c->fixed_choice.count({fa.g.M, kFxRows}) && c->fixed_choice.count({fa.g.Py, kFxCols})) return;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return;
+private:
+    struct Note {
+        int n = 0, id = 0;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+    };
+    void note(int n, int role, int id, Note* out) {
+        if (id == 0 || c_->plan_use.count({n, role})) return;
+        out->n = n;
+        out->id = id;
+        check_cuda(cudaEventCreate(&out->e0), "plan-event");
+        check_cuda(cudaEventCreate(&out->e1), "plan-event");
     }
-    tune_length(c, fa.g.M, kFxRows, s, [&](int id) {
-        FrameArgs a = fa;
-        a.g.plan_m.fixed = id;
-        a.g.plan_m.stw = stage_twiddles(c, id);
-        launch_frame_rows(a, s);
-        launch_frame_inverse(a, s);
-    });
-    tune_length(c, fa.g.Py, kFxCols, s, [&](int id) {
-        FrameArgs a = fa;
-        a.g.plan_py.fixed = id;
-        a.g.plan_py.stw = stage_twiddles(c, id);
-        launch_frame_cols(a, s);
-    });
-}
+    void mark(cudaEvent_t* e) {
+        if (*e) check_cuda(cudaEventRecord(*e, s_), "plan-event");
+    }
+    void keep(int role, Note* n) {
+        if (n->id == 0) return;
+        c_->plan_use[{n->n, role}] = {n->id, h16_, n->e0, n->e1};
+        *n = Note{};
+    }
+    ld_ctx* c_;
+    cudaStream_t s_;
+    bool h16_;
+    Note cols_, rows_;
+};
 
 // Issues a frame chain through a cached CUDA graph: the first call with a
 // given key launches the chain directly, the second within the last
@@ -2540,18 +2551,33 @@ int ld_set_autotune(ld_ctx* c, int enable) {
 int ld_autotune_choice(ld_ctx* c, int32_t n, int32_t* radices_out, int32_t* shape_out, double* ms_out) {
     if (!c || !radices_out) return 0;
     std::lock_guard<std::mutex> lock(c->mu);
-    auto it = c->fixed_choice.find({n, kFxRows});
-    if (it == c->fixed_choice.end()) it = c->fixed_choice.find({n, kFxCols});
-    if (it == c->fixed_choice.end()) return 0;
-    const FxPlanDesc* d = fx_plan(it->second);
+    // a length with several column orders answers for the columns (the rows have one)
+    int ids[8];
+    const bool cols = fx_candidates(n, kFxCols, ids, 8) > 1;
+    auto it = c->plan_use.find({n, cols ? kFxCols : kFxRows});
+    if (it == c->plan_use.end()) it = c->plan_use.find({n, cols ? kFxRows : kFxCols});
+    if (it == c->plan_use.end()) return 0;
+    const FxPlanDesc* d = fx_plan(it->second.id);
     if (d == nullptr) return 0;
-    for (int i = 0; i < 3; ++i) radices_out[i] = d->radix[i];
+    // the passes of the FP16 form's order where it has one, else the plan's radices
+    FxOrder o{3, {d->radix[0], d->radix[1], d->radix[2], 0}, {1, 1, 1, 0}};
+    if (it->second.h16) {
+        const FxOrder own = d->role == kFxRows ? fx_row_order(d->radix[0], d->radix[1], d->radix[2])
+                                               : fx_col_order(d->radix[0], d->radix[1], d->radix[2]);
+        if (own.count > 0) o = own;
+    }
+    for (int i = 0; i < o.count; ++i) radices_out[i] = o.radix(i);
     if (shape_out) *shape_out = 0;
     if (ms_out) {
-        auto m = c->fixed_ms.find(it->first);
-        *ms_out = m != c->fixed_ms.end() ? m->second : 0.0;
+        float ms = 0.0f;
+        if (cudaEventSynchronize(it->second.e1) != cudaSuccess ||
+            cudaEventElapsedTime(&ms, it->second.e0, it->second.e1) != cudaSuccess) {
+            cudaGetLastError();
+            ms = 0.0f;
+        }
+        *ms_out = ms;
     }
-    return 3;
+    return o.count;
 }
 
 size_t ld_estimate_device_bytes(const ld_params* params, int32_t width, int32_t height) {
@@ -2744,8 +2770,9 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         const bool tiled = zt.n > 0 && static_cast<double>(zt.wo + Kmax - 1) * (zt.ho + Kmax - 1) <=
                                            0.5 * static_cast<double>(Ww + Kmax - 1) * (Hw + Kmax - 1);
         const bool fx = fx_chain(p);
-        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx, &rw, &rh)
-                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx, &rw, &rh);
+        const bool direct = composite_chain(p, cb);
+        const GridGeom g = tiled ? make_geometry(ctx, zt.wo, zt.ho, Kmax, c_rows, c_cols, fx, direct, &rw, &rh)
+                                 : make_geometry(ctx, Ww, Hw, Kmax, c_rows, c_cols, fx, direct, &rw, &rh);
         // Spectra already cached (a warm frame)?  If not, the bank and kernel
         // spectra are built on s while the source's row transforms run on a
         // side stream: they do not depend on the lens.  (Tiles transform
@@ -2825,7 +2852,7 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         if (post.scatter) {
             const int Ks = 2 * std::max(1, static_cast<int>(std::ceil(std::max(0.5f, post.scatter_radius)))) + 1;
             int srw = 0, srh = 0;
-            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, fx_chain(p), &srw, &srh);
+            gs = make_geometry(ctx, Ww, Hw, Ks, 3, 3, fx_chain(p), false, &srw, &srh);
         }
         // rows of the row spectra: the frame's, or a tile's input rows
         const int Hp = tiled ? ((zt.ho + Kmax - 1 + 3) & ~3) : ((Hw + 3) & ~3);
@@ -3002,6 +3029,7 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
         gkey = append_bytes(gkey, &part_lo, sizeof(part_lo));
         gkey = append_bytes(gkey, &part_hi, sizeof(part_hi));
         gkey = append_bytes(gkey, &overlap_rows, sizeof(overlap_rows));
+        PlanNotes notes(ctx, g, direct, fa.h16 != 0, s);
         auto chain = [&, fa = fw]() mutable {  // the loops below edit this copy
             if (dv == LD_DEBUG_SELECTION) {  // the mask alone: no convolution
                 check_cuda(cudaMemsetAsync(fin.mask_max, 0, sizeof(unsigned int), s), "mask-memset");
@@ -3015,8 +3043,11 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
                 if (!tiled) staged(ctx, LD_STAGE_FRAME_ROWS, s, [&] { launch_frame_rows(fa, s); });
             }
             if (fa.effect_mode != kEffectAccumulate) {
+                notes.at(0);
                 staged(ctx, LD_STAGE_FRAME_COLS, s, [&] { launch_frame_cols(fa, s); });
+                notes.at(1);
                 staged(ctx, LD_STAGE_FRAME_INVERSE, s, [&] { launch_frame_inverse(fa, s); });
+                notes.at(2);
             } else {
                 const int nz = zones ? zn * zn : 1;
                 fa.zone_n = zones ? zn : 0;
@@ -3059,9 +3090,6 @@ int ld_render(ld_ctx* ctx, const ld_render_request* rq, const ld_params* params,
             if (fa.effect_mode != kEffectComposite) staged(ctx, LD_STAGE_COMPOSITE, s, [&] { launch_composite(fin, s); });
         };
         run_chain(ctx, s, gkey, chain);
-        // the first composite frame at this grid picks the transforms' radix orders
-        if (!run_scatter && !zones && fa.effect_mode == kEffectComposite && dv == LD_DEBUG_FINAL)
-            autotune_frame(ctx, fw, s);
         for (const SpectraEntry* e : spectra) mark_used(const_cast<SpectraEntry&>(*e), s);
         check_launch("frame-chain");
         if (st) {
