@@ -1561,12 +1561,15 @@ int fft_passes(int n, bool allow25) {
 
 // Cheapest 5-smooth length >= n (a multiple of `mult`) for up to C
 // interleaved sequences: cost ~ m * (stages + 1.5), the stage passes plus the
-// fill and drain, so a slightly longer length with fewer stages can win.
+// fill and drain, so a slightly longer length with fewer stages can win among
+// those up to a tenth (or 64) longer.  Where there is none (649-654 and
+// 1297-1309 rows: the next multiples of four are 720 and 1440) the next one
+// that has an FFT family; -1 above them all.
 int choose_length(int n, int mult, int C) {
     int best = -1;
     double best_cost = 0.0;
     const int hi = n + std::max(64, n / 10);
-    for (int m = std::max(n, 2); m <= hi; ++m) {
+    for (int m = std::max(n, 2); m <= hi || (best < 0 && fft_family(m, C) != 0); ++m) {
         if (m % mult != 0 || !smooth(m)) continue;
         const int fam = fft_family(m, C);
         if (fam == 0) continue;
@@ -2594,7 +2597,7 @@ size_t ld_estimate_device_bytes(const ld_params* params, int32_t width, int32_t 
         const PostEffects post = post_effects(p);
         working_size(post, width, height, &width, &height);  // the effect's frame
         const int M = choose_length((width + static_cast<int>(K) - 1 + 1) / 2, 1, c_rows);
-        const int Py = choose_length(height + static_cast<int>(K) - 1, 2, c_cols);
+        const int Py = choose_length(height + static_cast<int>(K) - 1, 4, c_cols);  // as make_geometry
         if (M < 0 || Py < 0) return 0;
         const size_t cols = static_cast<size_t>(M) + 1, Hp = (static_cast<size_t>(height) + 3) & ~size_t(3);
         const size_t zones = has_field_phase(p) ? static_cast<size_t>(p.field_grid > 0 ? p.field_grid : 3) *
@@ -2613,7 +2616,7 @@ size_t ld_estimate_device_bytes(const ld_params* params, int32_t width, int32_t 
             const size_t Rs = static_cast<size_t>(std::ceil(std::max(0.5f, post.scatter_radius)));
             const size_t Ks = 2 * Rs + 1;
             const int Ms = choose_length((width + static_cast<int>(Ks) - 1 + 1) / 2, 1, 3);
-            const int Pys = choose_length(height + static_cast<int>(Ks) - 1, 2, 3);
+            const int Pys = choose_length(height + static_cast<int>(Ks) - 1, 4, 3);
             if (Ms < 0 || Pys < 0) return 0;
             const size_t cs = static_cast<size_t>(Ms) + 1;
             frame_ab = std::max(frame_ab, 6 * cs * Hp * 8);
