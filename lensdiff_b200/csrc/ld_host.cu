@@ -1811,12 +1811,23 @@ std::vector<const SpectraEntry*> ensure_zone_spectra(ld_ctx* c, const ld_params&
         // GPU to a few CTAs per zone (3 x 3 zones of 9 wavelengths at K = 267:
         // 20 + 5 + 7 us nine times), while canvases beyond kZoneCanvas would
         // leave L2 before the combination reads them.  (A group's wavelengths
-        // are a launch dimension: at most 65535.)
+        // are a launch dimension: at most 65535.)  A context with a memory
+        // budget takes the zones one by one through its own bank's canvases
+        // (group 0), which a frame without zones needs too.
         constexpr size_t kZoneCanvas = size_t(96) << 20;
         const size_t plane = static_cast<size_t>(2 * R + 1) * (2 * R + 1);
-        const size_t group = std::max<size_t>(
+        const size_t group = c->budget ? 0 : std::max<size_t>(
             1, std::min({need.size(), kZoneCanvas / (plane * B * sizeof(float)), size_t(65535) / B}));
-        for (size_t k0 = 0; k0 < need.size(); k0 += group) {
+        for (size_t k = 0; group == 0 && k < need.size(); ++k) {
+            const size_t z = static_cast<size_t>(need[k]);
+            const PreWindows pre{const_cast<float*>(args[k].win), const_cast<WavelengthInfo*>(args[k].wl)};
+            bool rb = false, rs = false;
+            BankEntry& b = ensure_bank(c, zps[z], s, &rb, &pre);
+            ensure_spectra_in(c, c->zone_spectra[z], b, cb, g, s, &rs);
+            *bank_rebuilt = *bank_rebuilt || rb;
+            *spectra_rebuilt = *spectra_rebuilt || rs;
+        }
+        for (size_t k0 = 0; group > 0 && k0 < need.size(); k0 += group) {
             const size_t m = std::min(group, need.size() - k0);
             PsfBankArgs ga = args[k0];
             ga.B = static_cast<int>(m) * B;
