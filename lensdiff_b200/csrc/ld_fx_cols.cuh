@@ -90,23 +90,23 @@ using ColsLast = typename ColsLastOf<P, C, T, INV, H16>::type;
 // with the luma lock, 4) kernel spectra, the products transformed back, the
 // first Hp rows stored to B.  Shared memory: the header, F [n] (the column's
 // spectrum), W [n][C].
-// H16: the half2 row spectra and their row exponents arrive at the start of W
-// (widened as the forward transform's first stage loads them), the half2
-// kernel spectra in W's upper half (multiplied with F as the inverse's first
-// stage loads them); the forward stages alternate between F and W's lower
-// half, so they need one barrier each.  FP32: the row spectra arrive in F,
-// the kernel spectra fill W.  The inverse's last stage stays in registers:
-// its largest component (H16: the column's scale) and the store come from
-// there.
-// Bound by the latency of its stages: at n = 3200, 24 warps per SM of which the
-// forward stages (a third of the inverse's butterflies) use some, 50 % of the
+// H16 (the passes of P::ord): the half2 row spectra and their row exponents
+// arrive at the start of W (widened as the forward transform's first pass
+// loads them), the half2 kernel spectra in W's upper half (scaled and
+// multiplied with F as the inverse's first pass loads them); the forward
+// passes alternate between F and W's lower half, so they need one barrier
+// each.  FP32: the row spectra arrive in F, the kernel spectra fill W.  The
+// inverse's last pass stays in registers: its largest component (H16: the
+// column's scale) and the store come from there.
+// Bound by the latency of its passes: at n = 3200, 24 warps per SM of which the
+// forward passes (a third of the inverse's butterflies) use some, 51 % of the
 // issue slots.  H16 / FP32 launch times, against the passes before it
 // (compiled transforms in place between a fill, a product and a drain; at the
 // other lengths the runtime-planned transforms):
-//   2501 columns of 3200: 138 us (175) / 130 us (155)
-//   4097 columns of 5120: 402 us (757)
-//   1126 columns of 1800: 42 us (101)
-//   1251 columns of 1600: 37 us (50)
+//   2501 columns of 3200: 140 us (175) / 130 us (155)
+//   4097 columns of 5120: 479 us (757; four passes) / 391 us
+//   1126 columns of 1800: 43 us H16 (101)
+//   1251 columns of 1600: 37 us (50) / 39 us
 //   1201 columns of 1152: 29 us FP32 (72)
 template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_frame_cols_kernel(FrameArgs a) {
@@ -260,8 +260,9 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_cols_mono_kernel(FrameArgs a
 // Column k of the C kernel spectra: the row spectra of the canvas rows (Kp x C)
 // arrive by bulk copy behind W, take their wrapped grid rows as the first
 // stage loads them, and the last stage's registers go out to KS[k] (H16: in
-// FP16 with the column's scale).  2501 columns of 3200 take 97 us (128 before,
-// see above), 4097 of 5120 284 us (517), 1126 of 1800 28 us (66).
+// FP16 with the column's scale).  H16 / FP32: 2501 columns of 3200 take 89 / 90
+// us (128 before, see above), 4097 of 5120 331 / 289 us (517), 1126 of 1800 28
+// us H16 (66).
 template <class P, int C, int T, int MINB, bool H16>
 __global__ void __launch_bounds__(T, MINB) fx_kspec_cols_kernel(KernelSpectraArgs a) {
     stream_order();

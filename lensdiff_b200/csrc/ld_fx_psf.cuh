@@ -139,7 +139,7 @@ __device__ __forceinline__ int window_index(int k, int x0, int half, int S) {
 }
 
 // grid (ceil(row_n / C), B): C pupil rows of wavelength blockIdx.y.  440 rows of
-// 2048 for 31 wavelengths take 86 us (266 with the runtime-planned transforms),
+// 2048 for 31 wavelengths take 87 us (266 with the runtime-planned transforms),
 // bound by issue: the fields' sine and cosine and the transform.
 template <class P, int C, int NZ, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_psf_rows_kernel(PsfBankArgs a) {
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(T, MINB) fx_psf_rows_kernel(PsfBankArgs a) {
 }
 
 // grid (ceil(win_stride / C), B): C window columns of wavelength blockIdx.y.
-// Windows of 236-413 columns of 2048 for 31 wavelengths take 55 us (215).
+// Windows of 236-413 columns of 2048 for 31 wavelengths take 56 us (215).
 template <class P, int C, int NZ, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_psf_cols_kernel(PsfBankArgs a) {
     stream_order();

@@ -233,10 +233,10 @@ __device__ __forceinline__ void rows_forward(const FftPlan& plan, const float2* 
 // ---- forward rows ---------------------------------------------------------------
 // C / NDRV frame rows per CTA (see frame_rows_kernel, whose work it does): the
 // last stage gives the bins, scaled and stored from registers.  Bound by the
-// latency of the fill and of the scattered stores (35 % of the warp slots, the
-// source read once): 2160 rows of 2500 take 66 us (88 before: in-place stages
-// and bins through shared memory), 3160 of 4096 171 us (207, runtime-planned),
-// 1648 tile rows of 1125 24 us (46).  The pixels'
+// latency of the fill and of the scattered stores (29 % of the warp slots, 40 %
+// of the issue slots, the source read once): H16 / FP32, 2160 rows of 2500 take
+// 69 / 67 us (88 before: in-place stages and bins through shared memory), 3160
+// of 4096 162 / 168 us (207, runtime-planned).  The pixels'
 // drivers go through shared memory: forming them in the first stage's
 // unrolled loads repeats the highlight mask 50 times and stalls on
 // instruction fetches (142 us for 2160 rows of 2500, against 88 before).
@@ -268,10 +268,10 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_rows_kernel(FrameArgs a) {
 // ---- inverse rows ---------------------------------------------------------------
 // One row of C channels per CTA (see frame_inverse_kernel): the first stage
 // takes the row's bins from the column outputs, two bins per load pair.  Bound
-// by instruction issue and latency (55 % of the issue slots at 24 warps per SM;
-// half the instructions are the composite's): 2160 rows of 2500 take 105 us
-// (H16) / 118 (FP32) (143 / 128 with compiled in-place stages), 3160 of 4096
-// 361 us (475, runtime-planned), 620 of 1125 24 us (52).
+// by instruction issue and latency (54 % of the issue slots at 24 warps per SM;
+// half the instructions are the composite's): H16 / FP32, 2160 rows of 2500 take
+// 107 / 110 us (143 / 128 with compiled in-place stages), 3160 of 4096 355 / 439
+// us (475 H16, runtime-planned).
 template <class P, int C, bool H16, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_frame_inverse_kernel(FrameArgs a) {
     stream_order();
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(T, MINB) fx_frame_inverse_kernel(FrameArgs a) 
 
 // ---- kernel-spectrum rows ---------------------------------------------------------
 // One canvas row of the C kernels per CTA (see kspec_rows_kernel).  1026 rows of
-// 2500 take 54 us (64 before), 1502 of 4096 158 us (214), 1026 of 1125 24 us (75).
+// 2500 take 54 us (64 before), 1502 of 4096 160 us (214), 1026 of 1125 25 us (75).
 template <class P, int C, bool H16, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) fx_kspec_rows_kernel(KernelSpectraArgs a) {
     stream_order();
@@ -344,13 +344,13 @@ constexpr RowsShape forward_shape() {
 }
 
 template <class P, int C, int NDRV, bool FROM_EFFECT, bool H16 = false>
-void frame_rows_fx(FrameArgs a, cudaStream_t s) {
+void frame_rows_fx(const FrameArgs& a, cudaStream_t s) {
     constexpr RowsShape sh = forward_shape<P, C, H16>();
     static_assert(sh.threads > 0);
     static KernelState state;
     auto f = fx_frame_rows_kernel<P, C, NDRV, FROM_EFFECT, H16, sh.threads, sh.ctas>;
     const size_t sm = kRowsHeader + static_cast<size_t>(P::n) * C * sizeof(float2);
-    a.ahead = state.get(f, sh.threads, sm);
+    state.get(f, sh.threads, sm);
     launch_after(f, a.Hp / (C / NDRV), sh.threads, sm, s, a);
 }
 

@@ -5,9 +5,10 @@
 // visible.  Each wait follows the previous kernel's, so a kernel runs its body
 // after everything that was before it on the stream, as with a plain launch.
 //
-// What it saves is the launch between the short kernels of a pass: 1024x576
-// with 3 wavelengths, cold (14 kernels), 77 -> 68 us; 3 x 3 zones at 1917x803
-// (80 kernels) 935 -> 917 us; UHD with 31 wavelengths, cold, 706 -> 695 us.
+// What it saved when it came is the launch between the short kernels of a pass:
+// 1024x576 with 3 wavelengths, cold (14 kernels), 77 -> 70 us; 3 x 3 zones at
+// 1917x803 (80 kernels) 935 -> 917 us; UHD with 31 wavelengths, cold, 706 -> 696
+// us.
 // No kernel lets its successor start earlier (launch_dependents): the waiting
 // CTAs then hold shared memory and registers that the other stream's kernels
 // could use, and the successor's CTAs crowd the SMs that drain first.  With

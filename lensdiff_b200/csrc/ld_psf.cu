@@ -305,8 +305,8 @@ __device__ __forceinline__ void resample_flush(const PsfBankArgs& a, int b, int 
 // rows; the rows' sample positions are uniform in the warp, so the two
 // horizontally interpolated window rows a sample blends are kept in registers
 // until the position moves to the next window row (every 1 / inv_scale
-// canvas rows).  Bound by instruction issue (84 M warp instructions, 76 % of
-// the issue slots): 112 us for 31 wavelengths at K = 1025 (168 us for tiles
+// canvas rows).  Bound by instruction issue (80 M warp instructions, 68 % of
+// the issue slots): 113 us for 31 wavelengths at K = 1025 (168 us for tiles
 // without the mirror images, two wavelengths at a time, every sample from
 // four shared-memory reads).
 constexpr int kQuadH = 128;
@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(256) support_kernel(PsfBankArgs a) {
     sc.start = fmaxf(0.0f, extent - fade);
 }
 
-// grid (ceil((R+1)/32), B), block 256: s4 = sum over the crop box of taper *
+// grid (ceil((R+1)/16), B), block 256: s4 = sum over the crop box of taper *
 // normalised shaped kernel, the normaliser of cropKernelToRadius and
 // applySupportBoundaryTaper (LensDiffCpuReference.cpp:1038-1058, :957-982).
 // The canvas keeps the shaped kernel; the crop and the taper are applied
