@@ -288,18 +288,18 @@ class Clocks:
 # other revision of the kernels reports traffic null: a figure measured on
 # other code says nothing about this code.  Writes still resident in L2 when a
 # kernel ends are not counted.
-TRAFFIC_SOURCES_SHA = "4d4f7172ff0be248"
+TRAFFIC_SOURCES_SHA = "0392dac47a074d0f"
 MEASURED_TRAFFIC_UHD31 = {
     "chosen": {
-        "resample": 82423936,
+        "resample": 82644736,
         "crop_sum": 15454592,
-        "combine": 132561024,
-        "kspec_rows": 22846720,
-        "kspec_cols": 103238144,
-        "frame_rows": 138003072,
-        "frame_cols": 144797824,
-        "frame_inverse": 323565184,
-        "dft_gemm": 56079872,
+        "combine": 132705152,
+        "kspec_rows": 22555392,
+        "kspec_cols": 103335552,
+        "frame_rows": 137743744,
+        "frame_cols": 144488192,
+        "frame_inverse": 324373632,
+        "dft_gemm": 56653312,
     },
 }
 
