@@ -2280,10 +2280,10 @@ public:
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if ((!cols_.id && !rows_.id) || cudaStreamIsCapturing(s_, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
             return;
-        if (i == 0) mark(&cols_.e0);
-        if (i == 1) mark(&cols_.e1);
-        if (i == 1) mark(&rows_.e0);
-        if (i == 2) mark(&rows_.e1);
+        if (i == 0) mark(cols_, &cols_.e0);
+        if (i == 1) mark(cols_, &cols_.e1);
+        if (i == 1) mark(rows_, &rows_.e0);
+        if (i == 2) mark(rows_, &rows_.e1);
         if (i < 2) return;
         keep(kFxCols, &cols_);
         keep(kFxRows, &rows_);
@@ -2305,11 +2305,11 @@ private:
         if (id == 0 || c_->plan_use.count({n, role})) return;
         out->n = n;
         out->id = id;
-        check_cuda(cudaEventCreate(&out->e0), "plan-event");
-        check_cuda(cudaEventCreate(&out->e1), "plan-event");
     }
-    void mark(cudaEvent_t* e) {
-        if (*e) check_cuda(cudaEventRecord(*e, s_), "plan-event");
+    void mark(const Note& n, cudaEvent_t* e) {
+        if (n.id == 0) return;
+        check_cuda(cudaEventCreate(e), "plan-event");
+        check_cuda(cudaEventRecord(*e, s_), "plan-event");
     }
     void keep(int role, Note* n) {
         if (n->id == 0) return;

@@ -658,47 +658,49 @@ __global__ void __launch_bounds__(256) resample_kernel(PsfBankArgs a, ResampleGr
 // the statistics that scale the kernel summed in another order, a small
 // log-encoded frame moved by 7e-5 of its norm, at the same error against FP64.
 // A bank with a box filter is therefore sampled tap by tap, and summed, over
-// 32 x 128 tiles, one wavelength a tile: 186 us for 16 wavelengths at K = 513
-// with footprints 3.3-5.7 (71 us separably).  (A bank without one moves by
-// less than its own float atomics moved it here: resample_quad.)
-// sampleSquareBilinear (LensDiffCpuReference.cpp:316-336) reading the |F|^2
-// window; the window covers every pixel the kernel touches.
-__device__ __forceinline__ float sample_bilinear(const Window& w, float x, float y) {
-    const float lim = static_cast<float>(w.S - 1);
-    if (x < 0.0f || y < 0.0f || x > lim || y > lim) return 0.0f;
-    const int x0 = static_cast<int>(floorf(x));
-    const int y0 = static_cast<int>(floorf(y));
-    const int x1 = min(x0 + 1, w.S - 1);
-    const int y1 = min(y0 + 1, w.S - 1);
-    const float tx = x - static_cast<float>(x0);
-    const float ty = y - static_cast<float>(y0);
-    const int hi = w.n - 1;
-    const int ax0 = min(max(x0 - w.x0, 0), hi), ax1 = min(max(x1 - w.x0, 0), hi);
-    const int ay0 = min(max(y0 - w.x0, 0), hi), ay1 = min(max(y1 - w.x0, 0), hi);
-    const float v00 = w.p[static_cast<size_t>(ay0) * w.stride + ax0];
-    const float v10 = w.p[static_cast<size_t>(ay0) * w.stride + ax1];
-    const float v01 = w.p[static_cast<size_t>(ay1) * w.stride + ax0];
-    const float v11 = w.p[static_cast<size_t>(ay1) * w.stride + ax1];
-    const float vx0 = v00 + (v10 - v00) * tx;
-    const float vx1 = v01 + (v11 - v01) * tx;
-    return vx0 + (vx1 - vx0) * ty;
+// 32 x 128 tiles, one wavelength a tile: 125 us for 16 wavelengths at K = 513
+// with footprints 3.3-5.7 (76 us separably, 193 us with the columns of a tap
+// formed anew for every sample).  (In a bank without a box filter
+// resample_quad's tiles take the same samples, and their sums move the outputs
+// by up to 1.7e-5, most by under 5e-6.)
+
+// The columns of a pixel's taps (the x terms of sampleSquareBilinear,
+// LensDiffCpuReference.cpp:316-336): the same for every row a thread samples.
+constexpr int kTaps = 6;
+__device__ __forceinline__ void tap_columns(const Window& w, float px, float footprint, float step, ColTap (&ct)[kTaps]) {
+#pragma unroll
+    for (int t = 0; t < kTaps; ++t) ct[t] = col_tap(w, px + ((static_cast<float>(t) + 0.5f) * step - footprint * 0.5f));
 }
 
-// sampleSquareFiltered (LensDiffCpuReference.cpp:338-353)
-__device__ __forceinline__ float sample_filtered(const Window& w, float x, float y, float footprint, int taps,
-                                                 float step) {
+// The mean of taps x taps bilinear samples (sampleSquareFiltered,
+// LensDiffCpuReference.cpp:338-353), a row of taps at a time; a tap outside
+// [0, S - 1] adds zero.
+__device__ __forceinline__ float sample_taps(const Window& w, const ColTap (&ct)[kTaps], float py, float footprint,
+                                             int taps, float step) {
+    const float lim = static_cast<float>(w.S - 1);
+    const int hi = w.n - 1;
     float sum = 0.0f;
-    for (int ty = 0; ty < taps; ++ty) {
-        const float oy = (static_cast<float>(ty) + 0.5f) * step - footprint * 0.5f;
-        for (int tx = 0; tx < taps; ++tx) {
-            const float ox = (static_cast<float>(tx) + 0.5f) * step - footprint * 0.5f;
-            sum += sample_bilinear(w, x + ox, y + oy);
+    for (int t = 0; t < taps; ++t) {  // uniform: a warp is one canvas row
+        const float y = py + ((static_cast<float>(t) + 0.5f) * step - footprint * 0.5f);
+        if (y < 0.0f || y > lim) continue;
+        const int y0 = static_cast<int>(floorf(y));
+        const float ty = y - static_cast<float>(y0);
+        const float* r0 = w.p + static_cast<size_t>(min(max(y0 - w.x0, 0), hi)) * w.stride;
+        const float* r1 = w.p + static_cast<size_t>(min(max(min(y0 + 1, w.S - 1) - w.x0, 0), hi)) * w.stride;
+#pragma unroll
+        for (int u = 0; u < kTaps; ++u) {
+            if (u >= taps || !ct[u].in) continue;
+            const float v00 = __ldg(r0 + ct[u].ax0), v10 = __ldg(r0 + ct[u].ax1);
+            const float v01 = __ldg(r1 + ct[u].ax0), v11 = __ldg(r1 + ct[u].ax1);
+            const float vx0 = v00 + (v10 - v00) * ct[u].tx;
+            const float vx1 = v01 + (v11 - v01) * ct[u].tx;
+            sum += vx0 + (vx1 - vx0) * ty;
         }
     }
     return sum / static_cast<float>(taps * taps);
 }
 
-// sample_bilinear with the column half precomputed (identical arithmetic).
+// One bilinear sample with the column half precomputed (identical arithmetic).
 __device__ __forceinline__ float sample_row(const Window& w, const ColTap& c, float y) {
     if (!c.in || y < 0.0f || y > static_cast<float>(w.S - 1)) return 0.0f;
     const int y0 = static_cast<int>(floorf(y));
@@ -720,7 +722,7 @@ __device__ __forceinline__ float sample_row(const Window& w, const ColTap& c, fl
 constexpr int kStageW = kTile + 4, kStageH = kTallH + 4;
 
 // Rows / columns of the window that canvas coordinates c0 .. c1 sample
-// (sample_bilinear's x0 .. x1 of the first and last sample, clamped to the
+// (x0 .. x1 of the first and last sample, clamped to the
 // window as it clamps them): [lo, hi] in window indices.
 __device__ __forceinline__ void stage_span(const Window& w, float rc, float kc, float inv, int c0, int c1, int* lo,
                                            int* hi) {
@@ -827,15 +829,15 @@ __device__ void resample_tile(const PsfBankArgs& a, int b, int rbase, TileSmem<F
     } else {
         __syncthreads();
         const ColTap ct = col_tap(w, rc + dx * inv);
-#pragma unroll 4
+        ColTap cts[kTaps];
+        if (taps != 0) tap_columns(w, rc + dx * inv, inv, step, cts);
         for (int i = 0; i < kTallH / 8; ++i) {
             const int y = ty0 + threadIdx.y + 8 * i;
             if (y >= K) break;  // uniform: a warp is one canvas row (the last tile row is mostly past K)
             const float dy = static_cast<float>(y) - kc;
             float v = 0.0f;
             if (in) {
-                v = taps == 0 ? sample_row(w, ct, rc + dy * inv)
-                              : sample_filtered(w, rc + dx * inv, rc + dy * inv, inv, taps, step);
+                v = taps == 0 ? sample_row(w, ct, rc + dy * inv) : sample_taps(w, cts, rc + dy * inv, inv, taps, step);
                 canvas[static_cast<size_t>(y) * K + x] = v;
                 lsum += v;
                 if constexpr (FUSED) lpeak = max(lpeak, __float_as_uint(v));
