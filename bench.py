@@ -288,18 +288,18 @@ class Clocks:
 # other revision of the kernels reports traffic null: a figure measured on
 # other code says nothing about this code.  Writes still resident in L2 when a
 # kernel ends are not counted.
-TRAFFIC_SOURCES_SHA = "0392dac47a074d0f"
+TRAFFIC_SOURCES_SHA = "cd3e14f52e9a879b"
 MEASURED_TRAFFIC_UHD31 = {
     "chosen": {
-        "resample": 82644736,
-        "crop_sum": 15454592,
-        "combine": 132705152,
-        "kspec_rows": 22555392,
-        "kspec_cols": 103335552,
-        "frame_rows": 137743744,
-        "frame_cols": 144488192,
-        "frame_inverse": 324373632,
-        "dft_gemm": 56653312,
+        "resample": 82240000,
+        "crop_sum": 15454976,
+        "combine": 132725760,
+        "kspec_rows": 23156992,
+        "kspec_cols": 103624704,
+        "frame_rows": 137830272,
+        "frame_cols": 144735232,
+        "frame_inverse": 323651200,
+        "dft_gemm": 56312320,
     },
 }
 
