@@ -251,18 +251,18 @@ int ld_set_graphs(ld_ctx* ctx, int enable);
  * column length Py of a frame grid each run on a compiled radix order
  * (ld_fxplans.h); column lengths 1600 and 3200 have two.  mode 1 (the
  * default): the frame chain's own order (frames that composite directly,
- * without field zones, Split, Preserve energy or scatter, take the last,
- * others the first); 0: the first compiled order of each length; 2 + k
- * (k <= 7): the k-th compiled order of each length (its last when it has
- * fewer), for tests; -1: the runtime-planned transforms only, no compiled
- * orders.  Nothing is timed on the caller's frames, so no mode launches
+ * without field zones, Split, Preserve energy or scatter, take the last from a
+ * context's second such frame on the length on, others the first); 0: the first
+ * compiled order of each length; 2 + k (k <= 7): the k-th compiled order of each
+ * length (its last when it has fewer), for tests; -1: the runtime-planned
+ * transforms only, no compiled orders.  Nothing is timed on the caller's frames, so no mode launches
  * more or waits.  No counterpart in the reference. */
 int ld_set_autotune(ld_ctx* ctx, int mode);
-/* The radix order that transform length n runs on: writes up to 4 radices
- * (first stage first) and returns how many, 0 when n has no compiled order
- * or no frame has composited directly on it in mode 1 yet (for a length that
- * is a grid's row and column length: the column order where it has two, else
- * the row order).  *shape_out (may be null): the launch shape, 0 (every order
+/* The radix order that frames which composite directly run on at transform
+ * length n: writes up to 4 radices (first stage first) and returns how many, 0
+ * when n has no compiled order or no such frame was rendered in mode 1 yet
+ * (for a length that is a grid's row and column length: the column order where
+ * it has two, else the row order).  *shape_out (may be null): the launch shape, 0 (every order
  * runs in the shape compiled for it).  *ms_out (may be null): the duration of
  * the first such frame's column pass, or inverse row pass; reading it waits
  * for that pass. */

@@ -331,7 +331,7 @@ void frame_cols_fx(FrameArgs a, cudaStream_t s) {
     auto f = fx_frame_cols_kernel<P, C, sh.threads, sh.ctas, H16>;
     constexpr size_t sm = cols_bytes(P::n, C);
     a.ahead = state.get(f, sh.threads, sm);
-    launch_after(f, a.g.cols, sh.threads, sm, s, a);
+    if (a.g.cols > 0) launch_after(f, a.g.cols, sh.threads, sm, s, a);  // (none: to load the kernel)
 }
 
 template <class P>
@@ -353,7 +353,7 @@ bool kspec_cols_fx(KernelSpectraArgs a, cudaStream_t s) {
     const size_t sm = kColsHeader + (static_cast<size_t>(P::n) + a.Kp) * C * sizeof(float2);
     if (sm > kSmemOptIn) return false;
     a.ahead = state.get(f, sh.threads, cols_bytes(P::n, C));
-    launch_after(f, a.g.cols, sh.threads, sm, s, a);
+    if (a.g.cols > 0) launch_after(f, a.g.cols, sh.threads, sm, s, a);
     return true;
 }
 

@@ -7,9 +7,10 @@
 // grid's cost model (choose_length in ld_host.cu) picks for the spectral
 // chains has one: columns from 300 to 5400, rows from 256 to 4096.  Column
 // lengths 1600 and 3200 have two orders: frames that composite directly run the
-// second, others the first.  (They are within 3 % of one another; an order that
-// changes moves the FP16 form's results by up to 2e-5, so each chain keeps the
-// one it has always had.)  Odd radices lead where the length has them: their
+// second from a context's second such frame on (the kernel spectra that the
+// first one built stay as they are), others the first.  (They are within 3 % of
+// one another; an order that changes moves the FP16 form's results by up to
+// 2e-5, so each frame keeps the one it has always had.)  Odd radices lead where the length has them: their
 // strided first-stage stores spread over the shared-memory banks.  A row plan's last radix is also its inverse's first, and is taken in
 // pairs of mirrored butterflies: a small one.  PSF plans (length S:
 // ld_fx_psf*.cu) cover the common PSF sizes; their first radix is a multiple

@@ -92,8 +92,8 @@ struct ld_ctx {
     std::mutex mu;
     std::map<int, DevBuf> twiddles;
     std::map<int, DevBuf> stage_twiddles;  // by fixed plan id
-    // (transform length, role) -> the fixed plan of its first composite frame and
-    // the events around that frame's launch on it
+    // (transform length, role) of a composite frame -> the fixed plan that later
+    // ones run on, and the events around the first one's launch
     struct PlanUse {
         int id;
         bool h16;
@@ -492,14 +492,16 @@ const float2* stage_twiddles(ld_ctx* c, int id) {
 }
 
 // The fixed plan a length runs on (0: none): the first compiled radix order,
-// or (mode 1, `composite`) the last: see LD_FX_COLS in ld_fxplans.h.  Mode 2 + k
-// pins the k-th compiled order of every length (its last when it has fewer).
+// or (mode 1, `composite`) from a context's second such frame on the last: see
+// ld_fxplans.h.  Mode 2 + k pins the k-th compiled order of every length (its
+// last when it has fewer).
 int fixed_plan_for(ld_ctx* c, int n, int role, bool composite) {
     if (role == 0 || c->autotune < 0) return 0;
     int ids[8];
     const int count = fx_candidates(n, role, ids, 8);
     if (count == 0) return 0;
-    const int k = c->autotune >= 2 ? c->autotune - 2 : (c->autotune == 1 && composite ? count - 1 : 0);
+    const bool last = c->autotune == 1 && composite && c->plan_use.count({n, role}) != 0;
+    const int k = c->autotune >= 2 ? c->autotune - 2 : (last ? count - 1 : 0);
     return ids[std::min(k, count - 1)];
 }
 
@@ -2265,13 +2267,15 @@ constexpr size_t kGraphSeen = 4;  // covers the three spectra slots that a strea
 // ---------------------------------------------------------------------------
 // The fixed transform plans in use (ld_fxplans.h)
 // ---------------------------------------------------------------------------
-// Brackets the column and inverse launches of a context's first composite frame
-// on each length's plan by events, for ld_autotune_choice: at(0) before the
-// column pass, at(1) between, at(2) after the inverse rows.  Nothing is
+// Notes a context's first composite frame on each length: its column and inverse
+// launches are bracketed by events for ld_autotune_choice (at(0) before the
+// column pass, at(1) between, at(2) after the inverse rows), and the kernels
+// and tables of the order that later frames take are loaded.  Nothing is
 // launched again and the host does not wait.
 class PlanNotes {
 public:
-    PlanNotes(ld_ctx* c, const GridGeom& g, bool composite, bool h16, cudaStream_t s) : c_(c), s_(s), h16_(h16) {
+    PlanNotes(ld_ctx* c, const GridGeom& g, bool composite, bool h16, cudaStream_t s)
+        : c_(c), g_(g), s_(s), h16_(h16) {
         if (c->autotune != 1 || !composite) return;
         note(g.Py, kFxCols, g.plan_py.fixed, &cols_);
         note(g.M, kFxRows, g.plan_m.fixed, &rows_);
@@ -2285,8 +2289,23 @@ public:
         if (i == 1) mark(rows_, &rows_.e0);
         if (i == 2) mark(rows_, &rows_.e1);
         if (i < 2) return;
-        keep(kFxCols, &cols_);
+        const int later = keep(kFxCols, &cols_);
         keep(kFxRows, &rows_);
+        if (later == 0 || later == g_.plan_py.fixed) return;
+        FrameArgs fa{};  // no columns: the kernels are only loaded
+        fa.g = g_;
+        fa.g.cols = 0;
+        fa.g.plan_py.fixed = later;
+        fa.n_drv = 1;
+        fa.n_out = 3;
+        fa.h16 = h16_ ? 1 : 0;
+        fx_launch_frame_cols(fa, s_);
+        KernelSpectraArgs ka{};
+        ka.g = fa.g;
+        ka.n_ker = 3;
+        ka.h16 = fa.h16;
+        fx_launch_kspec_cols(ka, s_);
+        stage_twiddles(c_, later);
     }
     ~PlanNotes() {
         for (Note* n : {&cols_, &rows_})
@@ -2311,12 +2330,17 @@ private:
         check_cuda(cudaEventCreate(e), "plan-event");
         check_cuda(cudaEventRecord(*e, s_), "plan-event");
     }
-    void keep(int role, Note* n) {
-        if (n->id == 0) return;
-        c_->plan_use[{n->n, role}] = {n->id, h16_, n->e0, n->e1};
+    // the plan that later frames run on (0: nothing noted)
+    int keep(int role, Note* n) {
+        if (n->id == 0) return 0;
+        int ids[8];
+        const int id = ids[fx_candidates(n->n, role, ids, 8) - 1];
+        c_->plan_use[{n->n, role}] = {id, h16_, n->e0, n->e1};
         *n = Note{};
+        return id;
     }
     ld_ctx* c_;
+    const GridGeom& g_;
     cudaStream_t s_;
     bool h16_;
     Note cols_, rows_;

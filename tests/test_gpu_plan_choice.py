@@ -1,6 +1,6 @@
 """Which compiled radix order a frame runs on is settled without the GPU: the
-first composite frame of a grid does not wait for it, every context settles on
-the same one, and a length that is both a row and a column length of a grid
+first composite frame of a grid does not wait for it, every context takes the
+same ones, and a length that is both a row and a column length of a grid
 answers for the role that has several."""
 import pytest
 
@@ -74,3 +74,33 @@ def test_first_composite_frame_does_not_wait():
     assert st.ok, st
     assert not waited
     cache.close()
+
+
+@pytest.mark.parametrize("n", [1600, 3200])
+def test_orders_of_a_contexts_frames(n):
+    """A context's first directly composited frame runs the first column order and
+    its kernel spectra stay on it; later frames, and kernel spectra of new lenses,
+    run the last.  Shown to the bit against the orders pinned one by one (the
+    lens has no box filter, so two contexts build the same bank)."""
+    stream = torch.cuda.Stream()
+    rq = _request(64, n - 2 * R, stream)
+    new = _lens().copy(phaseDefocus=0.3)
+
+    def frames(steps):
+        cache, out = LensDiffPsfBankCache(0), []
+        for mode, lens in steps:
+            cache.set_autotune(mode)
+            st = cache.render(rq, lens)
+            stream.synchronize()
+            assert st.ok and st.grid_used[1] == n, st
+            out.append(rq.dst.data.cpu().numpy())
+        cache.close()
+        return out
+
+    first, warm, cold = frames([(1, _lens()), (1, _lens()), (1, new)])
+    want_first, want_warm = frames([(2, _lens()), (3, _lens())])
+    want_cold, = frames([(3, new)])
+    assert (first == want_first).all()
+    assert (warm == want_warm).all()
+    assert (cold == want_cold).all()
+    assert not (want_first == want_warm).all()  # the orders do differ
