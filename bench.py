@@ -288,18 +288,18 @@ class Clocks:
 # other revision of the kernels reports traffic null: a figure measured on
 # other code says nothing about this code.  Writes still resident in L2 when a
 # kernel ends are not counted.
-TRAFFIC_SOURCES_SHA = "cd3e14f52e9a879b"
+TRAFFIC_SOURCES_SHA = "96f697f2b3f29fce"
 MEASURED_TRAFFIC_UHD31 = {
     "chosen": {
-        "resample": 82240000,
-        "crop_sum": 15454976,
-        "combine": 132725760,
-        "kspec_rows": 23156992,
-        "kspec_cols": 103624704,
-        "frame_rows": 137830272,
-        "frame_cols": 144735232,
-        "frame_inverse": 323651200,
-        "dft_gemm": 56312320,
+        "resample": 82155776,
+        "crop_sum": 15455488,
+        "combine": 132508544,
+        "kspec_rows": 22916864,
+        "kspec_cols": 103165824,
+        "frame_rows": 137676032,
+        "frame_cols": 144475136,
+        "frame_inverse": 324559488,
+        "dft_gemm": 56096896,
     },
 }
 
